@@ -177,18 +177,28 @@ struct Engine {
     cudaGraphExec_t chunk_exec[2] = {nullptr, nullptr};
     int chunk_steps = 16;
     int sm_count = 0;
-    // adjoint records
+    // adjoint records (the buffers are kept from one forward to the next of the same sizes)
     struct Adj {
         int ckpt = 0, nsteps = 0;
         std::vector<double*> ck;     // FP64 checkpoints: x, x_old, normal (9N doubles) every ckpt steps
-        double* s64 = nullptr;       // FP64 state: [x0 | xo0 | x1 | xo1 | n] (15N doubles)
-        double* rec = nullptr;       // (ckpt + 1) recorded states of the segment being replayed
-        double* lam = nullptr;       // 4 x 3N: adjoints of x, x_old (in / out)
+        double* tmp = nullptr;       // two FP64 states (18N) between checkpoints of the forward pass
+        double* rec = nullptr;       // recorded states of one segment (rec_states x 9N)
+        size_t rec_states = 0;
+        int rec_seg = -1;            // segment whose states rec holds (all but its checkpoint), -1: none
+        double* vel = nullptr;       // 6N: velocities of a step's input and output state
+        double* lam = nullptr;       // 2 x 3N: adjoints of x, x_old
         double* G = nullptr;         // 3N
-        double* dk = nullptr;        // per merged entry
-        double* dsc = nullptr;       // 3
-        uint32_t* rev = nullptr;     // reverse entry of every merged entry
+        double* g = nullptr;         // 12 per merged entry: its and its reverse entry's contributions to x, x_old
+        double* dk = nullptr;        // per merged entry dL/dk, its part of dL/dkd; per component of dL/dgamma, dL/dc
+        float* out = nullptr;        // per merged entry: the gradient in the caller's order
+        double* dsc = nullptr;       // 3, then the count of gradients that are not finite
+        uint32_t* wild = nullptr;
+        uint32_t* rev = nullptr;     // per merged entry: its reverse entry, its vertex and its place in the
+        uint32_t* src = nullptr;     // caller's order
+        uint32_t* pos = nullptr;
+        double* rest64 = nullptr;    // per merged entry: rest length, then (per-spring stiffness) stiffness
         unsigned* contacts = nullptr;  // vertices projected in each forward step
+        int contacts_cap = 0;
         bool ready = false;
     } adj;
 
@@ -241,7 +251,8 @@ struct Engine {
     void free_adjoint() {
         for (auto* q : adj.ck) cudaFree(q);
         adj.ck.clear();
-        void* ps[] = {adj.s64, adj.rec, adj.lam, adj.G, adj.dk, adj.dsc, adj.rev, adj.contacts};
+        void* ps[] = {adj.tmp, adj.rec, adj.vel, adj.lam, adj.G,   adj.g,   adj.dk,
+                      adj.out, adj.dsc, adj.wild, adj.rev, adj.src, adj.pos, adj.rest64, adj.contacts};
         for (void* q : ps)
             if (q) cudaFree(q);
         adj = Adj();
@@ -730,6 +741,7 @@ struct Engine {
         // device arrays are read by the build itself, in stream order; host arrays are
         // staged first.  The build also voids the garment's query-cache margins (the
         // body moves)
+        adj.rec_seg = -1;  // a backward pass replays every segment over the body as it is then
         const bool dev = kind == cudaMemcpyDeviceToDevice;
         if (!dev) {
             CU(cudaMemcpyAsync(bvh[g].xyz_in, xyz, (size_t)bvh[g].nv * 12, kind, stream));
@@ -798,6 +810,7 @@ struct Engine {
         if (n < 0 || (n > 0 && !idx)) return fail(VISG_ERR_INVALID_ARG, "bad pin list");
         for (int k = 0; k < n; ++k)
             if (idx[k] >= (uint32_t)N) return fail(VISG_ERR_INVALID_ARG, "pinned index out of range");
+        adj.rec_seg = -1;  // a backward pass replays every segment with the pins as they are then
         for (int64_t i = 0; i < N; ++i) h_rowp[i] &= ROW_MASK;
         for (int k = 0; k < n; ++k) h_rowp[idx[k]] |= PIN_BIT;
         for (int64_t i = 0; i < N; ++i) h_vcount[i].y = (h_vcount[i].y & ROW_MASK) | (h_rowp[i] & PIN_BIT);
@@ -1272,9 +1285,12 @@ struct Engine {
     int forward(int nsteps, int ckpt);
     int backward(const float* dL_dx, const float* dL_dxo, float* dL_dk, float* dL_dscalar);
     int forward_contacts(int64_t* counts, int n);
-    cudaError_t step64(int c, unsigned* contacts = nullptr);
-    cudaError_t save64(int c, double* dst);
-    cudaError_t load64(const double* src);
+    cudaError_t step64(const double* from, double* to, int k, unsigned* contacts = nullptr);
+    bool damped_springs() const {
+        uint32_t b;
+        std::memcpy(&b, &p.spring_damping, 4);
+        return b != 0u;
+    }
 };
 
 struct VisgSim {

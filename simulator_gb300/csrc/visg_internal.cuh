@@ -251,9 +251,38 @@ cudaError_t launch_set_vertices(float4* state, const uint32_t* idx, const float*
 cudaError_t launch_check_tame(const float4* state, int64_t n, uint32_t* wild, cudaStream_t s);
 
 // ---- adjoint ----------------------------------------------------------------------------
-// Packed float3 arrays of one recorded step: x, x_old and the contact normal entering
-// the step (n_in), and the contact normals the step produced (n_out: non-zero = the
-// vertex was projected, with that plane normal).
+// The differentiable forward: one step in double between packed double3 arrays.
+struct Step64Args {
+    const double* x;
+    const double* xo;
+    const double* n_in;   // contact normals entering the step
+    const double* v;      // (x - xo) / dt of the input state; NULL: spring damping is exactly +0
+    double* xn;
+    double* xon;
+    double* n_out;
+    double* vn;           // written when v is given
+    const uint32_t* rowp;
+    const uint2* ent;
+    const uint32_t* src;  // vertex of every merged entry
+    const double* rest64; // rest length of every merged entry
+    const double* k64;    // per entry stiffness, or NULL (list stiffness)
+    double list_k[VISG_MAX_LISTS];
+    const BvhView* bodies;
+    const float4* body_verts;
+    const uint32_t* body_tris;
+    StepParams p;
+    int refv, collide, n;
+    int* err;
+    unsigned* contacts;   // vertices projected, or NULL
+    uint32_t* wild;       // sticky: some state had a component too large for the damping term to be left out
+};
+cudaError_t launch_step_f64(const Step64Args& a, cudaStream_t s);
+// v = (x - xo) / dt (v may be NULL) and the wild word, of n3 components
+cudaError_t launch_vel_f64(const double* x, const double* xo, double* v, float dt, uint32_t* wild, int64_t n3,
+                           cudaStream_t s);
+// One reverse step.  x, x_old and the contact normal entering the step (n_in), and the
+// contact normals the step produced (n_out: non-zero = the vertex was projected, with
+// that plane normal), as packed double3 arrays.
 struct AdjArgs {
     const double* x;
     const double* xo;
@@ -261,24 +290,37 @@ struct AdjArgs {
     const double* n_out;
     const uint32_t* rowp;
     const uint2* ent;
-    const float* kent;     // per entry stiffness, or NULL (list stiffness)
+    const uint32_t* src;   // vertex of every entry
     const uint32_t* rev;   // reverse entry of every directed spring
-    const double* lx_in;   // adjoint of the step's outputs x', x_old' (double3 per vertex)
-    const double* lxo_in;
-    double* lx_out;        // adjoint of the step's inputs x, x_old
-    double* lxo_out;
-    double* G;             // adjoint of the force on each vertex (double3)
+    const double* rest64;  // rest length of every entry
+    const double* k64;     // per entry stiffness, or NULL (list stiffness)
+    double list_k[VISG_MAX_LISTS];
+    double* lx;            // adjoint of x, x_old in place: of the step's outputs (without the springs of
+    double* lxo;           // the step after, with gather), then of its inputs (without its own springs)
+    double* G;             // adjoint of the force on each vertex
+    double* v;             // (x - xo) / dt
+    double* gx;            // per entry two double3: its contribution to x of its vertex, and its reverse entry's;
+    double* gxo;           // the same for x_old (only with spring damping)
     double* dk;            // per entry, accumulated over steps
-    double* dscalar;       // [3]: gamma, force damping, spring damping; accumulated
+    double* dkd;           // per entry: its part of dL/d spring damping, accumulated
+    double* dgc;           // per vertex component: its parts of dL/d gamma and force damping, accumulated
+    const uint32_t* wild;
+    int gather;            // gx, gxo hold the springs of the step after this one
     int n;
+    int64_t E;
+    double inv_dt, dt2_mass, damp_dt, kd;  // 1 / dt, dt^2 / mass, force damping / dt, spring damping
     StepParams p;
 };
 cudaError_t launch_adjoint_step(const AdjArgs& a, cudaStream_t s);
-// the differentiable forward: one step in double (packed double3 arrays)
-cudaError_t launch_step_f64(const double* x, const double* xo, double* xn, double* xon, double* nrm,
-                            const uint32_t* rowp, const uint2* ent, const float* kent, const BvhView* bodies,
-                            const float4* body_verts, const uint32_t* body_tris, const StepParams& p, int refv,
-                            int collide, int n, int* err, unsigned* contacts, cudaStream_t s);
+// rest[e] and, with kent, k64[e] of n merged entries
+cudaError_t launch_entries_f64(const uint2* ent, const float* kent, double* rest, double* k64, int64_t n,
+                               cudaStream_t s);
+// dscalar[3] += the sums of the dgc and dkd parts
+cudaError_t launch_adj_scalars(const double* dgc, int64_t n3, const double* dkd, int64_t E, double* dscalar,
+                               cudaStream_t s);
+// out[pos[k]] = (float)dk[k]; *bad += those that are not finite
+cudaError_t launch_adj_result(const double* dk, const uint32_t* pos, float* out, unsigned* bad, int64_t n,
+                              cudaStream_t s);
 cudaError_t launch_widen(const float* src, double* dst, int64_t n, cudaStream_t s);
 cudaError_t launch_narrow(const double* src, float* dst, int64_t n, cudaStream_t s);
 
