@@ -66,7 +66,7 @@ constexpr int ERR_INDEX = 8;     // an index read on the device was out of range
 
 // LBVH internal node: children's boxes and links.  Links: >= 0 internal node,
 // < 0 leaf ~link.  Each child writes its own two float4 during the build.
-struct __align__(16) Node {
+struct __align__(32) Node {
     float4 a_lo;  // child A min xyz, w = link A
     float4 a_hi;  // child A max xyz
     float4 b_lo;  // child B min xyz, w = link B
@@ -122,28 +122,26 @@ struct BvhBuffers {
     Node* nodes = nullptr;       // nt-1
     float4* leaves = nullptr;    // 2*nt
     int2* range = nullptr;       // nt-1 leaf range of each internal node
-    // Summaries of the 512-leaf chunks for the nodes whose leaf range spans chunks
-    // (levels: per chunk, per 32 chunks, per 1024, per 32768, at lev_off[0..3])
-    int* cmin = nullptr;         // min delta over the boundaries of the entry's chunks
-    float4* cbox = nullptr;      // 2 per entry: union of the entry's leaf boxes
+    // Summaries of the chunks (512 sorted positions each) for the nodes whose leaf range spans chunks
+    int* cmin = nullptr;         // min delta over the boundaries that end the chunk's unjoined subtrees
+    float4* cbox = nullptr;      // 2 per chunk: union of its leaf boxes
     int2* srec = nullptr;        // 32 per chunk: suffix-minimum boundaries {position, delta}, right to left
     float4* sbox = nullptr;      // 2 per record: union of the chunk's leaves after the boundary
     int2* prec = nullptr;        // 32 per chunk: prefix-minimum boundaries, left to right
     float4* pbox = nullptr;      // 2 per record: union of the chunk's leaves up to the boundary
-    int* rcnt = nullptr;         // 3 per chunk: suffix and prefix record counts, nodes in `top`
+    uint32_t* rcnt = nullptr;    // 2 per chunk: prefix record count | nodes in `top` << 16; suffix record count
     int2* top = nullptr;         // 64 per chunk: {boundary, delta} of the nodes that span chunks
-    int chunks = 0;              // chunks of nt leaves
-    int lev_off[4] = {0, 0, 0, 0};
+    int chunks = 0;
     BvhRoot* root = nullptr;
     uint32_t* scratch = nullptr; // radix histograms, look-back status words, tile counters (the build clears them)
     size_t scratch_words = 0;
-    int max_ctas = 0;            // CTAs a build launches at most (one per 512 triangles)
+    int max_ctas = 0;            // CTAs a build launches at most
+    uint32_t* bcnt = nullptr;    // bucket counts of the bucket sort
+    unsigned long long* bkey = nullptr;  // its sampled keys
     float* part = nullptr;       // 8 per CTA: the CTA's box union
-    uint32_t* ucnt = nullptr;    // per CTA: distinct codes in its slice
+    uint32_t* ucnt = nullptr;    // per chunk: its leaves
     uint32_t* chg = nullptr;     // count + the triangles whose code changed since the last build
     uint32_t* sync = nullptr;    // grid-barrier counters, zero between builds
-    uint32_t* gdone = nullptr;   // per summary entry above level 0: members finished
-    int n_entries = 0;           // summary entries of all levels
 
     void plan(Arena& a, int nv_, int nt_, bool normals);
     BvhView view() const { return BvhView{nodes, leaves, root}; }

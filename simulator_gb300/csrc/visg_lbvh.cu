@@ -8,7 +8,8 @@
 // once, walk its phases, and a grid barrier (every CTA arrives on a counter, then
 // waits for the others, bounded) separates phases that read what others wrote:
 //   verts   vertex_extend (Mesh.cpp:101-117) v += thickness * n, stored as float4
-//           (the same launch voids the query-cache margins of the body's cloth)
+//           (the same launch voids the query-cache margins of the body's cloth); a small
+//           body's triangles gather the caller's vertices themselves and do not wait for it
 //   boxes   expanded triangle boxes (primitive.cu:79-91) and leaf records, three
 //           corners gathered as aligned float4; per CTA the union of its boxes
 //           with the identity box
@@ -16,27 +17,35 @@
 //           unions itself); the Morton code of each box centroid in the frame
 //           (bvh.cu:20-41,71-79; bbox.h:97-127); codes that differ from the last
 //           build's are listed
-//   sort    the stable order by (code, triangle).  When the last build's sorted
-//           list is at hand and at most CHG_CAP codes changed (a body that moves
-//           rigidly flips a few codes at cell edges), it is merged: the unchanged
+//   sort    the order by (code, triangle), one of three ways.  The last build's sorted list
+//           is at hand and at most CHG_CAP codes changed (a body that moves
+//           rigidly flips a few codes at cell edges): it is merged; the unchanged
 //           entries keep their order, every CTA sorts the changed ones in shared
 //           memory, and each entry's new position follows from binary searches
-//           (phase_merge).  Otherwise four stable LSD radix passes over 8-bit
+//           (phase_merge).  More changed (a body that turns or deforms), or there is no
+//           last list and the body is small: splitters cut the keys into buckets that
+//           single CTAs sort in shared memory (phase_scatter, phase_bucket_sort).
+//           Otherwise, or if a bucket overflows: four stable LSD radix passes over 8-bit
 //           digits, tiles claimed in order, decoupled look-back.
-//   unique  keep the first triangle of every distinct code (remove_redundant,
-//           Utilities.h:35-55): per-CTA counts, a barrier, then each CTA's offset
-//   build   bottom-up radix-tree build fused with the refit, per chunk of 512
-//           sorted leaves: each leaf thread climbs with handshakes in shared
-//           memory while both children lie in the chunk; the parent of range
+//   build   per chunk of 512 sorted positions: de-duplication (keep the first triangle
+//           of every distinct code, remove_redundant, Utilities.h:35-55) and a bottom-up
+//           radix-tree build fused with the refit: each leaf thread climbs with handshakes
+//           in shared memory while both children lie in the chunk; the parent of range
 //           [l, r] is the boundary with the longer common prefix (delta(l-1,l)
 //           vs delta(r,r+1), delta = clz(a ^ b) as cudaBRT.cu:9-19), the second
 //           child to arrive merges both boxes into the identity box
 //           (calculateBoudingBox, cudaBRT.cu:166-206) and continues.  Each chunk
-//           then publishes a summary for the nodes that span chunks; the CTA that
-//           finishes the last chunk of a group of 32 sums the group up a level
+//           then publishes a summary for the nodes that span chunks
 //   top     one warp per node that spans chunks: its range ends are the nearest
 //           boundaries with a smaller delta, its box the union of its leaves'
 //           boxes, both read off the chunk summaries
+// What bounds it is latency: a body is a few MB, a barrier about 1.3 us and a dependent
+// load through L2 about 0.5, so phases are merged where a grid-wide value is not needed
+// between them (de-duplication in the build, centroids kept in registers from the boxes to
+// the codes, small bodies without the vertex phase), 32-byte records move as one access,
+// and the sorts spread over all CTAs.  Kernel time, before and now: 19,584 triangles with
+// few changed codes 32 -> 23 us, with most changed (radix passes before) 69 -> 31, without a
+// last order 68 -> 34; 327,680 triangles with few changed 107 -> 75.
 // Nodes are numbered by their split position; the tree is the same binary radix
 // tree processInternalNode (cudaBRT.cu:120-161) builds, and visg_export_lbvh
 // renumbers it into the reference's layout.  Data one CTA reads after another wrote
@@ -62,15 +71,22 @@ constexpr int SORT_ITEMS = 4;
 constexpr int SORT_TILE = RB * SORT_ITEMS;  // 2048 keys per radix tile
 constexpr int RADIX = 256;
 constexpr int PASSES = 4;
-constexpr int UNIQ_ITEMS = 4;
-constexpr int CHG_CAP = 2048;  // changed codes the incremental sort merges
+constexpr int SPREAD_CTAS = 152;    // CTAs a small body is spread over (one per SM)
+constexpr int DIRECT_MAX = 65536;   // triangles up to which boxes gather the caller's vertices themselves
+constexpr int CHG_CAP = 256;   // changed codes the incremental sort merges (each CTA ranks them all)
+constexpr int BK_TARGET = 128; // triangles a bucket of the bucket sort should hold at least
+constexpr int BK_CAP = 512;    // and can hold: one key per thread of the sorting CTA
+constexpr int BK_MAX = 2048;   // buckets at most
+constexpr int OVERSAMPLE = 8;  // keys sampled per bucket for the splitters when there is no last order
+constexpr int SAMPLES = 2048;  // and in all
+constexpr int SAMPLED_MAX = SAMPLES / OVERSAMPLE * BK_TARGET;  // triangles up to which that is enough
 constexpr uint32_t ST_AGG = 1u << 30;
 constexpr uint32_t ST_PREFIX = 2u << 30;
 constexpr uint32_t ST_VALUE = (1u << 30) - 1u;
+constexpr uint32_t CNT_READY = 1u << 31;  // a chunk's leaf count has been published
 constexpr int SPIN_LIMIT = 1 << 22;
 constexpr uint64_t kGridWaitNs = 1000000000ull;  // a grid barrier gives up after 1 s
-constexpr int BUILD_LEAVES = RB;                 // leaves per chunk
-constexpr int NLEV = 4;
+constexpr int TOP_STAGED = 1024;  // chunks whose summaries the spanning-node phase stages in shared memory
 constexpr int BIG_DELTA = 64;  // above every delta: a boundary that does not exist
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {
@@ -146,24 +162,17 @@ __device__ __forceinline__ uint32_t block_scan_incl(uint32_t v, uint32_t* s_warp
     __syncthreads();
     return r;
 }
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_warp) {
-    (void)block_scan_incl(v, s_warp);
-    const uint32_t t = s_warp[RW - 1];
-    __syncthreads();  // every thread has read it before the next scan writes s_warp
-    return t;
-}
 
 // ---- arguments and shared memory ------------------------------------------------------------
-struct ChunkView {
+struct ChunkView {  // summaries of the chunks (build_chunk)
     int* cmin;
     float4* cbox;
     int2* srec;
     float4* sbox;
     int2* prec;
     float4* pbox;
-    int* rcnt;
+    uint32_t* rcnt;  // 2 per chunk
     int2* top;
-    int lev_off[NLEV];
 };
 
 struct RebuildArgs {
@@ -173,6 +182,7 @@ struct RebuildArgs {
     int nv, nt;
     float thickness, depth;
     int coherent;  // the last build's sorted list and codes may be reused
+    int direct;    // triangles gather the caller's vertices (else the pushed float4 copies)
     int tiles_sort;
     float4* verts;
     float4* tri_box;
@@ -190,29 +200,44 @@ struct RebuildArgs {
     uint32_t* ghist;   // PASSES x RADIX digit counts
     uint32_t* sstat;   // PASSES x tiles_sort x RADIX look-back status words
     uint32_t* scount;  // PASSES tile counters
+    uint32_t* bcnt;    // BK_MAX bucket counts
+    unsigned long long* bkey;  // SAMPLES sampled keys in order
     float* part;       // 8 per CTA: its box union (min xyz, max xyz)
-    uint32_t* ucnt;    // per CTA: distinct codes in its slice of the sorted list
+    uint32_t* ucnt;    // per chunk: its leaves, with CNT_READY once known
     uint32_t* chg;     // [0] changed codes, then {triangle, new code, old code} x CHG_CAP
     uint32_t* sync;    // [0] barrier arrivals, [1] CTAs finished (both 0 between launches)
-    uint32_t* gdone;   // per summary entry of levels 1..3: its member entries finished
-    int n_entries;     // summary entries of all levels
+    int chunks;
     int* err;
     float4* margin_state;  // cloth records whose query-cache margins the moved body voids
     int64_t m0, m1;        // (vertices [m0, m1): their margin words are cleared)
 };
 
+constexpr int MAX_PIECES = 64;  // subtrees a chunk leaves unjoined: at most 31 + 31 + 1 (30-bit codes)
 struct BuildSmem {
-    uint32_t flag[BUILD_LEAVES];  // bit 0: child A arrived, bit 1: child B
-    // per node and side (A, B): lo (w = link), hi (w = far range end)
-    float4 lo[BUILD_LEAVES][2], hi[BUILD_LEAVES][2];
-    int delta[BUILD_LEAVES + 4];  // delta of boundary j at j - c0 + 1
-    int wmin[RW], wsr[RW], wpr[RW], wtop[RW];  // per warp
-    float4 wlo[RW], whi[RW];
-    // per warp, over the warps before (x*p) / after (x*s) it
-    int xpm[RW], xsm[RW], xos[RW], xop[RW], xot[RW];
-    float4 xplo[RW], xphi[RW], xslo[RW], xshi[RW];
-    int nrec[4];
+    // per node and side (A, B): lo (w = link), hi (w = far_end)
+    float4 lo[RB][2], hi[RB][2];
+    uint32_t flag[RB];      // bit 0: child A arrived, bit 1: child B
+    uint32_t code[RB + 2];  // code of position p at p - p0 + 1
+    uint32_t lcode[RB], ltri[RB];  // the chunk's leaves, when some position is none
+    int delta[RB + 4];      // delta of local boundary j at j + 1
+    uint32_t next[32];      // codes after the chunk
+    uint32_t wcnt[RW], wsum[RW], pbits[RW];
+    float plo[MAX_PIECES][3], phi[MAX_PIECES][3];
+    int pend[MAX_PIECES];   // last leaf of each piece
 };
+static_assert(TOP_STAGED == 2 * RB, "a thread stages the counts of two chunks");
+struct TopSmem {
+    alignas(8) uint32_t rcnt[2 * TOP_STAGED];
+    float lo[TOP_STAGED][3], hi[TOP_STAGED][3];
+    int cmin[TOP_STAGED];
+    uint32_t pre[TOP_STAGED + 1];
+};
+struct BucketSmem {
+    unsigned long long key[BK_MAX];  // samples, splitters, then the keys of the bucket being sorted
+    uint32_t cnt[BK_MAX], base[BK_MAX];
+    uint32_t rank[BK_CAP];
+};
+static_assert(SAMPLES <= BK_MAX, "the samples share the splitters' array");
 struct SortSmem {
     uint32_t whist[RW][RADIX + 1];
     uint32_t tstart[RADIX];
@@ -223,33 +248,40 @@ struct SortSmem {
 struct MergeSmem {
     unsigned long long knew[CHG_CAP];  // changed entries by (new code, triangle)
     unsigned long long kold[CHG_CAP];  // the same entries by (old code, triangle)
+    unsigned long long in[2][CHG_CAP];  // both, as they were listed
+    uint32_t rank[2][CHG_CAP];
 };
 constexpr size_t smax(size_t a, size_t b) { return a > b ? a : b; }
-constexpr size_t kSmemBytes = smax(sizeof(BuildSmem), smax(sizeof(SortSmem), sizeof(MergeSmem)));
+constexpr size_t kSmemBytes =
+    smax(smax(sizeof(BuildSmem), sizeof(TopSmem)), smax(smax(sizeof(SortSmem), sizeof(MergeSmem)), sizeof(BucketSmem)));
 
 // ---- grid barrier ---------------------------------------------------------------------------
 // Every CTA arrives on sync[0] and waits until it holds `target` (gridDim.x per
 // barrier so far).  A CTA whose earlier wait gave up (ok false) still arrives, so
 // the others are not held, but does not wait.  Returns whether this CTA may go on.
+// One thread arrives with a release (cumulative over what the CTA barrier before it
+// ordered) and polls with acquires, without sleeping between them.  A barrier of 152 CTAs
+// takes 1.2-1.5 us (1.6 with fences around an atomic and 64 ns sleeps).
 __device__ bool grid_barrier(uint32_t* ctr, uint32_t& target, bool ok, int* err, int* s_ok) {
     __syncthreads();
     target += gridDim.x;
     if (threadIdx.x == 0) {
-        __threadfence();  // this CTA's writes before its arrival
-        atomicAdd(ctr, 1u);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
         int good = ok ? 1 : 0;
-        if (good && ld_volatile(ctr) < target) {
-            const uint64_t t0 = now_ns();
-            while (ld_volatile(ctr) < target) {
-                if (now_ns() - t0 > kGridWaitNs) {
+        uint64_t t0 = 0;
+        for (int polls = 0; good; ++polls) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+            if (v >= target) break;
+            if ((polls & 63) == 63) {
+                const uint64_t t = now_ns();
+                if (t0 == 0) t0 = t;
+                if (t - t0 > kGridWaitNs) {
                     atomicOr(err, ERR_TIMEOUT);
                     good = 0;
-                    break;
                 }
-                __nanosleep(64);
             }
         }
-        __threadfence();  // the others' writes before this CTA's reads
         *s_ok = good;
     }
     __syncthreads();
@@ -285,11 +317,14 @@ __device__ __forceinline__ void block_box_reduce(float r[6], float* s_red /* 6 *
     if (lane == 0)
         for (int k = 0; k < 6; ++k) s_red[k * RW + warp] = r[k];
     __syncthreads();
-    if (threadIdx.x < 6) {
-        const int k = threadIdx.x;
-        float v = s_red[k * RW];
-        for (int w = 1; w < RW; ++w) v = k < 3 ? fminf(v, s_red[k * RW + w]) : fmaxf(v, s_red[k * RW + w]);
-        s_red[k * RW] = v;
+    if (warp < 6) {  // warp k: component k of all warps
+        float v = s_red[warp * RW + (lane & (RW - 1))];
+#pragma unroll
+        for (int o = RW / 2; o > 0; o >>= 1) {
+            const float w = __shfl_xor_sync(0xffffffffu, v, o);
+            v = warp < 3 ? fminf(v, w) : fmaxf(v, w);
+        }
+        if (lane == 0) s_red[warp * RW] = v;
     }
     __syncthreads();
 }
@@ -310,11 +345,14 @@ constexpr int BOX_BATCH = 3;  // triangles a thread loads before it computes any
 
 // each triangle's expanded box (BBox(v0).expand(v1).expand(v2) and the three
 // corners pushed inward by depth * n) and leaf record; the CTA's union of its boxes
-// with the identity box in part[8 * cta]
-__device__ void phase_boxes(const RebuildArgs& A, float* s_red) {
+// with the identity box in part[8 * cta].  The centroids of a thread's first BOX_BATCH
+// triangles stay in its registers: phase_codes takes the same triangles.
+template <bool DIRECT>
+__device__ void phase_boxes(const RebuildArgs& A, float* s_red, f3 (&cen)[BOX_BATCH]) {
     const int stride = gridDim.x * RB;
+    const int first = blockIdx.x * RB + threadIdx.x;
     f3 lo = mk3(100.0f, 100.0f, 100.0f), hi = mk3(-100.0f, -100.0f, -100.0f);
-    for (int base = blockIdx.x * RB + threadIdx.x; base < A.nt; base += BOX_BATCH * stride) {
+    for (int base = first; base < A.nt; base += BOX_BATCH * stride) {
         uint32_t idx[BOX_BATCH][3];
 #pragma unroll
         for (int q = 0; q < BOX_BATCH; ++q) {
@@ -322,7 +360,7 @@ __device__ void phase_boxes(const RebuildArgs& A, float* s_red) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) idx[q][c] = t < A.nt ? __ldg(A.tris + 3 * t + c) : 0u;
         }
-        float4 w[BOX_BATCH][3];
+        f3 w[BOX_BATCH][3];
 #pragma unroll
         for (int q = 0; q < BOX_BATCH; ++q)
 #pragma unroll
@@ -335,13 +373,13 @@ __device__ void phase_boxes(const RebuildArgs& A, float* s_red) {
                     if (base + q * stride < A.nt) atomicOr(A.err, ERR_INDEX);
                     v = 0u;
                 }
-                w[q][c] = __ldcg(A.verts + v);
+                w[q][c] = DIRECT ? pushed(A, v) : xyz(__ldcg(A.verts + v));
             }
 #pragma unroll
         for (int q = 0; q < BOX_BATCH; ++q) {
             const int t = base + q * stride;
             if (t >= A.nt) break;
-            const f3 v0 = xyz(w[q][0]), v1 = xyz(w[q][1]), v2 = xyz(w[q][2]);
+            const f3 v0 = w[q][0], v1 = w[q][1], v2 = w[q][2];
             const f3 n = normalize(cross(sub(v1, v0), sub(v2, v0)));  // Primitive::d_get_normal
             f3 blo = v0, bhi = v0;
             box_add(blo, bhi, v1);
@@ -350,12 +388,12 @@ __device__ void phase_boxes(const RebuildArgs& A, float* s_red) {
             box_add(blo, bhi, sub(v0, dn));
             box_add(blo, bhi, sub(v1, dn));
             box_add(blo, bhi, sub(v2, dn));
-            A.tri_box[2 * t] = make_float4(blo.x, blo.y, blo.z, 0.0f);
-            A.tri_box[2 * t + 1] = make_float4(bhi.x, bhi.y, bhi.z, 0.0f);
-            A.tri_leaf[2 * t] = make_float4(v0.x, v0.y, v0.z, n.x);
-            A.tri_leaf[2 * t + 1] = make_float4(n.y, n.z, __int_as_float(t), 0.0f);
+            st8(A.tri_box + 2 * t, make_float4(blo.x, blo.y, blo.z, 0.0f), make_float4(bhi.x, bhi.y, bhi.z, 0.0f));
+            st8(A.tri_leaf + 2 * t, make_float4(v0.x, v0.y, v0.z, n.x),
+                make_float4(n.y, n.z, __int_as_float(t), 0.0f));
             box_add(lo, hi, blo);
             box_add(lo, hi, bhi);
+            if (base == first) cen[q] = divs(add(blo, bhi), 2.0f);  // BBox::centroid
         }
     }
     float r[6] = {lo.x, lo.y, lo.z, hi.x, hi.y, hi.z};
@@ -374,7 +412,8 @@ __device__ __forceinline__ uint32_t expand_bits(uint32_t v) {  // bvh.cu:20-27
 
 // the frame from the CTA unions; each triangle's code; with `listing`, the triangles
 // whose code changed go to the change list (at most CHG_CAP are stored)
-__device__ void phase_codes(const RebuildArgs& A, bool listing, float* s_red, float* s_frame) {
+__device__ void phase_codes(const RebuildArgs& A, bool listing, float* s_red, float* s_frame, f3 (&cen)[BOX_BATCH],
+                            uint32_t (&old)[BOX_BATCH]) {
     float r[6] = {100.0f, 100.0f, 100.0f, -100.0f, -100.0f, -100.0f};
     for (int c = threadIdx.x; c < (int)gridDim.x; c += RB) {
 #pragma unroll
@@ -394,26 +433,27 @@ __device__ void phase_codes(const RebuildArgs& A, bool listing, float* s_red, fl
     const bool flat = length(ext) == 0.0f;
     const int lane = threadIdx.x & 31;
     const int stride = gridDim.x * RB;
-    for (int base = blockIdx.x * RB; base < A.nt; base += 2 * stride) {  // warp-uniform bounds
-        // both triangles' loads first
-        float4 blo[2], bhi[2];
-        uint32_t old[2] = {0u, 0u};
+    const int first = blockIdx.x * RB;
+    for (int base = first; base < A.nt; base += BOX_BATCH * stride) {  // warp-uniform bounds
+        // all triangles' loads first
+        if (base != first)
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int t = base + q * stride + threadIdx.x;
-            if (t < A.nt) {
-                blo[q] = __ldcg(A.tri_box + 2 * t);
-                bhi[q] = __ldcg(A.tri_box + 2 * t + 1);
-                if (listing) old[q] = A.codes[t];
+            for (int q = 0; q < BOX_BATCH; ++q) {
+                const int t = base + q * stride + threadIdx.x;
+                if (t < A.nt) {
+                    const f4x2 b = ld8_cg(A.tri_box + 2 * t);
+                    cen[q] = divs(add(xyz(b.a), xyz(b.b)), 2.0f);
+                    if (listing) old[q] = A.codes[t];
+                }
             }
-        }
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < BOX_BATCH; ++q) {
             const int t = base + q * stride + threadIdx.x;
+            if (base + q * stride >= A.nt) break;
             bool changed = false;
             uint32_t code = 0u;
             if (t < A.nt) {
-                const f3 c = divs(add(xyz(blo[q]), xyz(bhi[q])), 2.0f);  // BBox::centroid
+                const f3 c = cen[q];
                 f3 u = mk3(0.0f, 0.0f, 0.0f);
                 if (!flat) u = divv(sub(c, fmn), ext);  // BBox::getUnitcubePosOf
                 const float x = fminf(fmaxf(__fmul_rn(u.x, 1024.0f), 0.0f), 1023.0f);
@@ -459,6 +499,24 @@ __device__ __forceinline__ int lower_bound64(const unsigned long long* a, int n,
     return lo;
 }
 
+// rank[i] += the keys of a[0, n) below a[i] (distinct keys, n <= RB, rank zero before), by
+// comparing all pairs: the CTA's threads share out n rows and, for a short list, parts of
+// the columns.  For the few hundred keys it is used on this takes a third of the time of
+// a bitonic sort, whose stages are all exchange: 128 keys 0.3 us.
+__device__ __forceinline__ void rank_keys(const unsigned long long* a, int n, uint32_t* rank) {
+    int rows = 32;
+    while (rows < n) rows <<= 1;  // at most RB
+    const int parts = RB / rows, part = (int)threadIdx.x / rows, i = (int)threadIdx.x & (rows - 1);
+    if (i < n) {
+        const unsigned long long x = a[i];
+        const int j1 = (part + 1) * n / parts;
+        uint32_t r = 0;
+#pragma unroll 8
+        for (int j = part * n / parts; j < j1; ++j) r += a[j] < x ? 1u : 0u;
+        atomicAdd(&rank[i], r);
+    }
+}
+
 // Merge of the nc changed entries into the last build's sorted list ko/vo (all nt
 // triangles by (code, triangle), old codes): every CTA sorts the changed entries by
 // new key (knew) and by old key (kold), then walks its slice of the old list.  For
@@ -471,67 +529,56 @@ __device__ __forceinline__ int lower_bound64(const unsigned long long* a, int n,
 // positions j (CTA 0).  Positions are a permutation of [0, nt); each is checked.
 __device__ void phase_merge(const RebuildArgs& A, int nc, const uint32_t* ko, const uint32_t* vo, uint32_t* kn,
                             uint32_t* vn, MergeSmem& S) {
-    int P = 1;
-    while (P < nc) P <<= 1;
-    for (int k = threadIdx.x; k < P; k += RB) {
-        if (k < nc) {
-            const uint32_t t = __ldcg(A.chg + 1 + 3 * k);
-            S.knew[k] = key64(__ldcg(A.chg + 2 + 3 * k), t);
-            S.kold[k] = key64(__ldcg(A.chg + 3 + 3 * k), t);
-        } else {
-            S.knew[k] = S.kold[k] = ~0ull;
-        }
+    for (int k = threadIdx.x; k < nc; k += RB) {
+        const uint32_t t = __ldcg(A.chg + 1 + 3 * k);
+        S.in[0][k] = key64(__ldcg(A.chg + 2 + 3 * k), t);
+        S.in[1][k] = key64(__ldcg(A.chg + 3 + 3 * k), t);
+        S.rank[0][k] = S.rank[1][k] = 0u;
     }
     __syncthreads();
-    for (int k = 2; k <= P; k <<= 1)  // bitonic sort of both arrays, ascending
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P; i += RB) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    const unsigned long long a = S.knew[i], b = S.knew[l];
-                    if ((a > b) == up) {
-                        S.knew[i] = b;
-                        S.knew[l] = a;
-                    }
-                    const unsigned long long c = S.kold[i], d = S.kold[l];
-                    if ((c > d) == up) {
-                        S.kold[i] = d;
-                        S.kold[l] = c;
-                    }
-                }
-            }
-            __syncthreads();
-        }
+    rank_keys(S.in[0], nc, S.rank[0]);
+    rank_keys(S.in[1], nc, S.rank[1]);
+    __syncthreads();
+    for (int k = threadIdx.x; k < nc; k += RB) {
+        S.knew[S.rank[0][k]] = S.in[0][k];
+        S.kold[S.rank[1][k]] = S.in[1][k];
+    }
+    __syncthreads();
     const int nt = A.nt;
     const int per = (nt + gridDim.x - 1) / gridDim.x;
     const int a = blockIdx.x * per, b = min(nt, a + per);
     constexpr int MB = 3;  // slots a thread loads before it searches
-    for (int s0 = a + threadIdx.x; s0 < b; s0 += MB * RB) {
-        unsigned long long ks[MB], k1[MB];
+    const int lane = (int)(threadIdx.x & 31u);
+    for (int w0 = a + ((int)threadIdx.x & ~31); w0 < b; w0 += MB * RB) {  // warp-uniform
+        unsigned long long ks[MB];
+#pragma unroll
+        for (int u = 0; u < MB; ++u) {  // lane 31's next slot is searched for by nobody else: load it too
+            const int s = w0 + u * RB + lane;
+            ks[u] = s < nt ? key64(ko[s], vo[s]) : ~0ull;
+        }
+        unsigned long long kx[MB];
 #pragma unroll
         for (int u = 0; u < MB; ++u) {
-            const int s = s0 + u * RB;
-            ks[u] = s < b ? key64(ko[s], vo[s]) : ~0ull;
-            k1[u] = s < b && s + 1 < nt ? key64(ko[s + 1], vo[s + 1]) : ~0ull;
+            const int s = w0 + u * RB + 32;
+            kx[u] = lane == 31 && s < nt ? key64(ko[s], vo[s]) : ~0ull;
         }
 #pragma unroll
         for (int u = 0; u < MB; ++u) {
-            const int s = s0 + u * RB;
-            if (s >= b) break;
-            const int q = lower_bound64(S.kold, nc, ks[u]);
-            const int r = lower_bound64(S.knew, nc, ks[u]);
+            const int s = w0 + u * RB + lane;
+            const int q = lower_bound64(S.kold, nc, ks[u]), r = lower_bound64(S.knew, nc, ks[u]);
+            // the next slot's counts: the next lane's
+            int q1 = __shfl_down_sync(0xffffffffu, q, 1), r1 = __shfl_down_sync(0xffffffffu, r, 1);
+            if (lane == 31) {
+                q1 = lower_bound64(S.kold, nc, kx[u]);
+                r1 = lower_bound64(S.knew, nc, kx[u]);
+            }
+            if (s >= b) continue;
             if (!(q < nc && S.kold[q] == ks[u])) {  // unchanged
                 const int pos = s - q + r;
                 if ((unsigned)pos < (unsigned)nt) {
                     kn[pos] = (uint32_t)(ks[u] >> 32);
                     vn[pos] = (uint32_t)ks[u];
                 }
-            }
-            int r1 = nc, q1 = nc;
-            if (s + 1 < nt) {
-                r1 = lower_bound64(S.knew, nc, k1[u]);
-                q1 = lower_bound64(S.kold, nc, k1[u]);
             }
             for (int j = r; j < r1; ++j) {
                 const int pos = j + s + 1 - q1;
@@ -547,6 +594,133 @@ __device__ void phase_merge(const RebuildArgs& A, int nc, const uint32_t* ko, co
         for (int j = threadIdx.x; j < r0; j += RB) {
             kn[j] = (uint32_t)(S.knew[j] >> 32);
             vn[j] = (uint32_t)S.knew[j];
+        }
+    }
+}
+
+// ---- sort: buckets -------------------------------------------------------------------------------
+// Too many codes changed for a merge (an animated body): splitters cut the keys (code,
+// triangle) into nb buckets of at least about BK_TARGET; phase_scatter puts every
+// triangle's key into its bucket's slots (in any order), and after a grid barrier each
+// bucket is sorted by one CTA in shared memory (phase_bucket_sort).  The splitters are
+// nb - 1 entries at equal distances of the last build's list, whose codes have moved only
+// a little; without one, of a sample.  The keys are distinct, so equal codes do not fill a
+// bucket.  Small buckets, so that a small body's sort takes all SMs.  The slots lie in the
+// node array, which the build writes only later.
+//
+// The i-th of ns sampled triangles: one from each of ns equal parts of the list, at a
+// scrambled place in its part (a mesh's rows repeat: at equal distances the sample of the
+// capsules fell on the same few angles of every ring).
+__device__ __forceinline__ uint32_t sampled(int i, int ns, int nt) {
+    const int64_t t = (int64_t)i * nt / ns, len = (int64_t)(i + 1) * nt / ns - t;
+    return (uint32_t)(t + (len > 1 ? (int64_t)(((uint32_t)i * 2654435761u) >> 8) % len : 0));
+}
+
+// phase_sample: the CTAs rank the sampled keys among themselves, each its share, and
+// leave them in order in A.bkey.
+__device__ void phase_sample(const RebuildArgs& A, int ns, BucketSmem& S) {
+    for (int i = threadIdx.x; i < ns; i += RB) {
+        S.key[i] = key64(__ldcg(A.codes + sampled(i, ns, A.nt)), (uint32_t)i);  // by (code, place): distinct
+    }
+    __syncthreads();
+    const int lane = (int)(threadIdx.x & 31u);
+    for (int i = blockIdx.x * RW + (int)(threadIdx.x >> 5); i < ns; i += gridDim.x * RW) {
+        const unsigned long long x = S.key[i];
+        uint32_t r = 0;
+#pragma unroll 8
+        for (int j = lane; j < ns; j += 32) r += S.key[j] < x ? 1u : 0u;
+        r = __reduce_add_sync(0xffffffffu, r);
+        if (lane == 0) A.bkey[r] = key64((uint32_t)(x >> 32), sampled(i, ns, A.nt));
+    }
+}
+
+__device__ void phase_scatter(const RebuildArgs& A, int nb, const uint32_t* ko, const uint32_t* vo, BucketSmem& S) {
+    const int nt = A.nt;
+    for (int i = threadIdx.x; i < nb - 1; i += RB) {
+        if (ko) {
+            const int p = (int)((int64_t)(i + 1) * nt / nb);
+            S.key[i] = key64(ko[p], vo[p]);
+        } else {
+            S.key[i] = __ldcg(A.bkey + (i + 1) * OVERSAMPLE);
+        }
+    }
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(A.nodes);
+    const int per = (nt + gridDim.x - 1) / gridDim.x;
+    const int a = blockIdx.x * per, b = min(nt, a + per);
+    constexpr int ITEMS = 4;
+    for (int s0 = a; s0 < b; s0 += ITEMS * RB) {
+        for (int k = threadIdx.x; k < nb; k += RB) S.cnt[k] = 0u;
+        __syncthreads();
+        unsigned long long key[ITEMS];
+        uint32_t rank[ITEMS];
+        int bk[ITEMS];
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u) {
+            const int t = s0 + u * RB + threadIdx.x;
+            key[u] = t < b ? key64(__ldcg(A.codes + t), (uint32_t)t) : ~0ull;
+        }
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u)
+            if (key[u] != ~0ull) {
+                bk[u] = lower_bound64(S.key, nb - 1, key[u] + 1ull);  // splitters <= key
+                rank[u] = atomicAdd(&S.cnt[bk[u]], 1u);
+            }
+        __syncthreads();
+        for (int k = threadIdx.x; k < nb; k += RB)
+            if (S.cnt[k]) S.base[k] = atomicAdd(A.bcnt + k, S.cnt[k]);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u)
+            if (key[u] != ~0ull) {
+                const uint32_t pos = S.base[bk[u]] + rank[u];
+                if (pos < (uint32_t)BK_CAP) slots[(size_t)bk[u] * BK_CAP + pos] = key[u];  // else: see buckets_fit
+            }
+        __syncthreads();
+    }
+}
+
+// whether no bucket was given more than it holds (the same answer in every CTA); S.cnt
+// then holds the counts and S.base the places of the buckets in the sorted list
+__device__ bool buckets_fit(const RebuildArgs& A, int nb, BucketSmem& S, uint32_t* s_scan) {
+    constexpr int E = BK_MAX / RB;
+    uint32_t c[E], sum = 0;
+    bool over = false;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = E * (int)threadIdx.x + e;
+        c[e] = i < nb ? __ldcg(A.bcnt + i) : 0u;
+        sum += c[e];
+        over |= c[e] > (uint32_t)BK_CAP;
+    }
+    uint32_t off = block_scan_incl(sum, s_scan) - sum;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = E * (int)threadIdx.x + e;
+        S.cnt[i] = c[e];
+        S.base[i] = off;
+        off += c[e];
+    }
+    return __syncthreads_or(over ? 1 : 0) == 0;
+}
+
+__device__ void phase_bucket_sort(const RebuildArgs& A, int nb, uint32_t* kn, uint32_t* vn, BucketSmem& S) {
+    const unsigned long long* slots = reinterpret_cast<const unsigned long long*>(A.nodes);
+    const int i = (int)threadIdx.x;
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        const int n = (int)S.cnt[b];
+        const uint32_t off = S.base[b];
+        const unsigned long long k = i < n ? __ldcg(slots + (size_t)b * BK_CAP + i) : 0ull;
+        S.rank[i] = 0u;
+        if (i < n) S.key[i] = k;
+        __syncthreads();
+        rank_keys(S.key, n, S.rank);
+        __syncthreads();
+        if (i < n) {
+            const uint32_t o = off + S.rank[i];
+            if (o < (uint32_t)A.nt) {
+                kn[o] = (uint32_t)(k >> 32);
+                vn[o] = (uint32_t)k;
+            }
         }
     }
 }
@@ -687,67 +861,7 @@ __device__ void phase_sort_pass(const RebuildArgs& A, int p, SortSmem& S, uint32
     }
 }
 
-// ---- unique ------------------------------------------------------------------------------------
-// CTA c takes positions [c * per, (c + 1) * per) of the sorted list; position p is a
-// leaf when p == 0 or its code differs from p - 1's
-__device__ __forceinline__ bool first_of_code(const uint32_t* K, int p) {
-    return p == 0 || __ldcg(K + p) != __ldcg(K + p - 1);
-}
-
-__device__ void phase_unique_count(const RebuildArgs& A, const uint32_t* K, uint32_t* s_scan) {
-    const int per = (A.nt + gridDim.x - 1) / gridDim.x;
-    const int a = blockIdx.x * per, b = min(A.nt, a + per);
-    uint32_t c = 0;
-    for (int p = a + threadIdx.x; p < b; p += RB) c += first_of_code(K, p) ? 1u : 0u;
-    const uint32_t tot = block_sum(c, s_scan);
-    if (threadIdx.x == 0) A.ucnt[blockIdx.x] = tot;
-}
-
-// the leaves of this CTA's slice at its offset (the counts of the CTAs before it);
-// returns the number of leaves in all
-__device__ int phase_unique_write(const RebuildArgs& A, const uint32_t* K, const uint32_t* V, uint32_t* s_scan) {
-    uint32_t before = 0, all = 0;
-    for (int c = threadIdx.x; c < (int)gridDim.x; c += RB) {
-        const uint32_t v = __ldcg(A.ucnt + c);
-        all += v;
-        if (c < (int)blockIdx.x) before += v;
-    }
-    before = block_sum(before, s_scan);
-    all = block_sum(all, s_scan);
-    const int per = (A.nt + gridDim.x - 1) / gridDim.x;
-    const int a = blockIdx.x * per, b = min(A.nt, a + per);
-    uint32_t off = before;
-    for (int base = a; base < b; base += RB * UNIQ_ITEMS) {
-        const int p0 = base + threadIdx.x * UNIQ_ITEMS;
-        uint32_t fl = 0;
-#pragma unroll
-        for (int j = 0; j < UNIQ_ITEMS; ++j)
-            if (p0 + j < b && first_of_code(K, p0 + j)) fl |= 1u << j;
-        const uint32_t cnt = __popc(fl);
-        const uint32_t incl = block_scan_incl(cnt, s_scan);
-        const uint32_t tile_total = s_scan[RW - 1];
-        uint32_t o = off + incl - cnt;
-#pragma unroll
-        for (int j = 0; j < UNIQ_ITEMS; ++j)
-            if (fl & (1u << j)) {
-                if (o < (uint32_t)A.nt) {
-                    A.ucode[o] = __ldcg(K + p0 + j);
-                    A.utri[o] = __ldcg(V + p0 + j);
-                }
-                ++o;
-            }
-        off += tile_total;
-        __syncthreads();  // s_scan is read above before the next scan overwrites it
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) A.root->n_leaves = (int)min(all, (uint32_t)A.nt);
-    return (int)min(all, (uint32_t)A.nt);
-}
-
 // ---- build ---------------------------------------------------------------------------------------
-__device__ __forceinline__ int delta_at(const uint32_t* c, int i, int j, int n) {
-    return (j < 0 || j >= n) ? -1 : __clz((int)(__ldcg(c + i) ^ __ldcg(c + j)));
-}
-
 // identity box (min +100, max -100) expanded by child A then child B
 __device__ __forceinline__ void merge_ab(float4 alo, float4 ahi, float4 blo, float4 bhi, float4& lo, float4& hi) {
     lo = make_float4(fminf(fminf(100.0f, alo.x), blo.x), fminf(fminf(100.0f, alo.y), blo.y),
@@ -757,19 +871,13 @@ __device__ __forceinline__ void merge_ab(float4 alo, float4 ahi, float4 blo, flo
 }
 
 // The child (lo, hi, link) over leaves [l, r] enters its parent g: its side of the
-// node and of the node's leaf range.  hi.w carries delta at the boundary beyond the
-// child's far end (l - 1 for child A, r for child B).
+// node and of the node's leaf range.
 __device__ __forceinline__ void write_side(Node* nodes, int2* range, int g, bool is_a, float4 lo, float4 hi, int link,
-                                           int l, int r, int dfar) {
-    if (is_a) {
-        nodes[g].a_lo = make_float4(lo.x, lo.y, lo.z, __int_as_float(link));
-        nodes[g].a_hi = make_float4(hi.x, hi.y, hi.z, __int_as_float(dfar));
-        range[g].x = l;  // leaf ranges of the nodes (read by the export)
-    } else {
-        nodes[g].b_lo = make_float4(lo.x, lo.y, lo.z, __int_as_float(link));
-        nodes[g].b_hi = make_float4(hi.x, hi.y, hi.z, __int_as_float(dfar));
-        range[g].y = r;
-    }
+                                           int l, int r) {
+    st8(is_a ? &nodes[g].a_lo : &nodes[g].b_lo, make_float4(lo.x, lo.y, lo.z, __int_as_float(link)),
+        make_float4(hi.x, hi.y, hi.z, 0.0f));
+    if (is_a) range[g].x = l;  // leaf ranges of the nodes (read by the export)
+    else range[g].y = r;
 }
 
 // box union (fminf / fmaxf: exact, so any grouping gives the same box)
@@ -779,11 +887,9 @@ __device__ __forceinline__ void box_union(float4& lo, float4& hi, float4 lo2, fl
 }
 __device__ __forceinline__ float4 ident_lo() { return make_float4(100.0f, 100.0f, 100.0f, 0.0f); }
 __device__ __forceinline__ float4 ident_hi() { return make_float4(-100.0f, -100.0f, -100.0f, 0.0f); }
-__device__ __forceinline__ float4 shfl_f4(float4 v, int o, bool up) {
-    return up ? make_float4(__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o),
-                            __shfl_up_sync(0xffffffffu, v.z, o), 0.0f)
-              : make_float4(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o),
-                            __shfl_down_sync(0xffffffffu, v.z, o), 0.0f);
+__device__ __forceinline__ float4 shfl_f4(float4 v, int o) {  // from the lane o below
+    return make_float4(__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o),
+                       __shfl_up_sync(0xffffffffu, v.z, o), 0.0f);
 }
 __device__ __forceinline__ void warp_box_reduce(float4& lo, float4& hi) {
 #pragma unroll
@@ -796,344 +902,285 @@ __device__ __forceinline__ void warp_box_reduce(float4& lo, float4& hi) {
     }
 }
 
-// entries of each level for n leaves
-__device__ __forceinline__ void level_counts(int n, int cnt[NLEV]) {
-    cnt[0] = (n + BUILD_LEAVES - 1) / BUILD_LEAVES;
-#pragma unroll
-    for (int v = 1; v < NLEV; ++v) cnt[v] = (cnt[v - 1] + 31) / 32;
-}
+// a child's far range end (a leaf of the chunk) with delta at the boundary beyond it, so
+// that the climb need not look the delta up again
+__device__ __forceinline__ int far_end(int leaf, int delta) { return leaf | (delta + 1) << 16; }
+__device__ __forceinline__ int far_leaf(int w) { return w & 0xffff; }
+__device__ __forceinline__ int far_delta(int w) { return (w >> 16) - 1; }
 
-// Bottom-up build of the chunk-local nodes, and the chunk summaries.  The CTA owns
-// the BUILD_LEAVES sorted leaves [c0, c1) of `chunk` and stages delta of the
-// boundaries c0 - 1 .. c1 - 1.  The climb goes through the nodes split inside the
-// chunk (c0 <= g <= c1 - 2) in shared memory only: each child leaves its box, link
-// and far range end in its side of the node's slot; the first to arrive stops, the
-// second merges (A then B) and climbs on.  After the barrier the nodes both of
-// whose children arrived are written out; a climb that stopped at a node whose
-// other child lies in another chunk, or at a node split outside the chunk, writes
-// its side into that node.  The remaining nodes span chunks; phase_top finishes them
-// from the chunk summaries written here:
-//   * the boundaries that can end such a node's range inside this chunk: the strict
-//     suffix minima of delta (the nearest smaller delta to the left of a node
-//     further right) and the strict prefix minima (to the right of a node further
-//     left), at most 30 each, with the union of the chunk's leaf boxes beyond /
-//     up to each of them;
-//   * the chunk's min delta and leaf box union;
-//   * the nodes of the chunk that span chunks (no smaller delta on one side inside
-//     the chunk, and the boundary to the next chunk).
-__device__ void build_chunk(const RebuildArgs& A, int chunk, int n, BuildSmem& S) {
+// De-duplication, bottom-up build of the chunk-local nodes, and the chunk summary.  A
+// chunk is RB positions [p0, p0 + m) of the sorted list; its leaves are the positions
+// whose code differs from the one before (remove_redundant, Utilities.h:35-55: the first
+// triangle of every code).  The chunk works in its own leaf numbers; where its leaves
+// begin in the whole is the sum of the counts that the chunks before it publish, read
+// when its climb is done (every CTA publishes a chunk's count before it waits, and takes
+// its chunks in ascending order, so every count that is waited for comes).
+//
+// The climb goes through the nodes split inside the chunk in shared memory only: each
+// child leaves its box, link and far range end in its side of the node's slot; the first
+// to arrive stops, the second merges (A then B) and climbs on.  Nodes both of whose
+// children arrived are written out.  What stays unjoined are pieces: subtrees over
+// consecutive leaves whose parent needs another chunk.  A piece's side is written into
+// its parent, and the boundaries after the pieces are the nodes that span chunks, which
+// phase_top finishes from the summary:
+//   * a node elsewhere whose range ends inside this chunk ends at a boundary after a
+//     piece (a boundary inside a piece has a larger delta than the piece's ends), so the
+//     records are the strict suffix minima of delta over those boundaries (the nearest
+//     smaller delta to the left of a node further right) and the strict prefix minima (to
+//     the right of a node further left), at most 31 each, with the union of the
+//     chunk's leaf boxes beyond / up to each of them;
+//   * the chunk's min delta and leaf box union.
+// Two warps make the summary of at most 63 pieces, two per lane, from either end.
+__device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, const uint32_t* V, BuildSmem& S) {
     const ChunkView& cv = A.cv;
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nt = A.nt;
-    const int c0 = chunk * BUILD_LEAVES;
-    const int c1 = min(c0 + BUILD_LEAVES, n);
-    S.flag[tid] = 0u;
-    const int i = c0 + tid;
-    int l = i, r = i, link = ~i;  // the current subtree: leaf range, link
+    const int nt = A.nt, p0 = chunk * RB, m = min(RB, nt - p0), p = p0 + tid;
+    const bool in = tid < m;
+    uint32_t k = 0u, t = 0u;
     float4 lo = ident_lo(), hi = ident_hi();
-    bool live = i < n;  // still climbing
-    int pend = -1;      // node where the climb stopped as the first local arrival
-    int out = -1;       // node split outside the chunk where the climb stopped
-    int dl = -1, dr = -1;
-    bool is_a = false;
-    uint32_t t = 0;  // the leaf's triangle
-    if (live) {
-        t = min(__ldcg(A.utri + i), (uint32_t)(nt - 1));
-        lo = __ldcg(A.tri_box + 2 * t);
-        hi = __ldcg(A.tri_box + 2 * t + 1);
+    if (in) {
+        k = __ldcg(K + p);
+        t = min(__ldcg(V + p), (uint32_t)(nt - 1));
+        const f4x2 b = ld8_cg(A.tri_box + 2 * t);
+        lo = b.a;
+        hi = b.b;
     }
-    {
-        const int j = c0 + tid;
-        S.delta[tid + 1] = delta_at(A.ucode, j, j + 1, n);  // -1 beyond the last leaf
-        if (tid == 0) S.delta[0] = c0 < n ? delta_at(A.ucode, c0, c0 - 1, n) : -1;
+    // the counts of the chunks before (most are there by the time they are needed)
+    uint32_t cw = tid < chunk ? ld_volatile(A.ucnt + tid) : CNT_READY;
+    S.code[tid + 1] = k;
+    if (tid == 0) S.code[0] = p0 > 0 ? __ldcg(K + p0 - 1) : 0u;
+    if (warp == 0) S.next[lane] = p0 + m + lane < nt ? __ldcg(K + p0 + m + lane) : 0xffffffffu;
+    S.flag[tid] = 0u;
+    if (lane == 0) S.pbits[warp] = 0u;
+    __syncthreads();
+    const bool first = in && (p == 0 || k != S.code[tid]);
+    const unsigned fb = __ballot_sync(0xffffffffu, first);
+    if (lane == 0) S.wcnt[warp] = (uint32_t)__popc(fb);
+    __syncthreads();
+    const uint32_t wc = lane < RW ? S.wcnt[lane] : 0u;
+    const int cnt = (int)__reduce_add_sync(0xffffffffu, wc);
+    const int rank = (int)__reduce_add_sync(0xffffffffu, lane < warp ? wc : 0u) + __popc(fb & ((1u << lane) - 1u));
+    if (tid == 0) st_volatile(A.ucnt + chunk, CNT_READY | (uint32_t)cnt);
+    if (first && rank == 0) S.delta[0] = p == 0 ? -1 : __clz((int)(k ^ S.code[tid]));
+    const uint32_t* lc = S.code + 1;  // the leaves' codes
+    if (cnt != m) {                   // some position is not a leaf: close the ranks up
+        lc = S.lcode;
+        if (first) {
+            S.lcode[rank] = k;
+            S.ltri[rank] = t;
+            S.lo[rank][0] = lo;
+            S.hi[rank][0] = hi;
+        }
+        __syncthreads();
+        if (tid < cnt) {
+            k = S.lcode[tid];
+            t = S.ltri[tid];
+            lo = S.lo[tid][0];
+            hi = S.hi[tid][0];
+        }
+    }
+    f4x2 leaf{};
+    if (tid < cnt) leaf = ld8_cg(A.tri_leaf + 2 * t);
+    if (tid + 1 < cnt) S.delta[tid + 1] = __clz((int)(k ^ lc[tid + 1]));
+    if (warp == 0 && cnt > 0) {  // the boundary to the next leaf, wherever it is
+        const uint32_t last = lc[cnt - 1];
+        const int e = p0 + m;
+        const unsigned b = __ballot_sync(0xffffffffu, e + lane < nt && S.next[lane] != last);
+        if (lane == 0) {
+            int d = -1;
+            if (b) {
+                d = __clz((int)(last ^ S.next[__ffs(b) - 1]));
+            } else if (e + 32 < nt) {  // more than 32 copies of the code follow: the first larger one
+                int l = e + 32, len = nt - l;
+                while (len > 0) {
+                    const int h = len >> 1;
+                    if (__ldcg(K + l + h) <= last) {
+                        l += h + 1;
+                        len -= h + 1;
+                    } else {
+                        len = h;
+                    }
+                }
+                if (l < nt) d = __clz((int)(last ^ __ldcg(K + l)));
+            }
+            S.delta[cnt] = d;
+        }
     }
     __syncthreads();
-    if (live && n == 1) {
-        A.root->root = -1;
-        A.root->top_lo = lo;
-        A.root->top_hi = hi;
-        live = false;
-    }
-    const float4 leaf_lo = lo, leaf_hi = hi;  // identity box for threads past the last leaf
-    int level = 0;
-    while (live) {
-        if (++level > 64) {  // a climb is at most 31 levels over distinct 30-bit codes
+    int l = tid, r = tid, link = ~tid;  // the current subtree: leaf range, link (local numbers)
+    bool live = tid < cnt;              // still climbing
+    bool is_root = false, is_a = false;
+    int pend = -1, out = -2;  // local node where the climb stopped: one of the chunk's, or one outside it
+    int dl = live ? S.delta[l] : 0, dr = live ? S.delta[r + 1] : 0;  // boundaries l - 1 and r
+    for (int level = 0; live; ++level) {
+        if (level > 64) {  // a climb is at most 31 levels over distinct 30-bit codes
             atomicOr(A.err, ERR_TIMEOUT);
             break;
         }
-        dl = S.delta[l - c0];      // boundary l - 1
-        dr = S.delta[r - c0 + 1];  // boundary r
-        is_a = dr > dl;            // the parent extends to the right: this node is child A
+        if (dl < 0 && dr < 0) {
+            is_root = true;
+            break;
+        }
+        is_a = dr > dl;  // the parent extends to the right: this node is child A
         const int g = is_a ? r : l - 1;
-        if (g < c0 || g > c1 - 2) {  // split outside the chunk
+        if (g < 0 || g > cnt - 2) {  // split outside the chunk
             out = g;
             break;
         }
-        const int k = g - c0, side = is_a ? 0 : 1;
-        S.lo[k][side] = make_float4(lo.x, lo.y, lo.z, __int_as_float(link));
-        S.hi[k][side] = make_float4(hi.x, hi.y, hi.z, __int_as_float(is_a ? l : r));
+        const int side = is_a ? 0 : 1;
+        S.lo[g][side] = make_float4(lo.x, lo.y, lo.z, __int_as_float(link));
+        S.hi[g][side] = make_float4(hi.x, hi.y, hi.z, __int_as_float(is_a ? far_end(l, dl) : far_end(r, dr)));
         __threadfence_block();
-        if (atomicOr(&S.flag[k], 1u << side) == 0u) {  // first to arrive: the sibling may be in another chunk
+        if (atomicOr(&S.flag[g], 1u << side) == 0u) {  // first to arrive: the sibling may be in another chunk
             pend = g;
             break;
         }
         __threadfence_block();
         // second to arrive: the sibling's side of the slot is complete
-        const float4 olo = S.lo[k][side ^ 1], ohi = S.hi[k][side ^ 1];
+        const float4 olo = S.lo[g][side ^ 1], ohi = S.hi[g][side ^ 1];
         const int far = __float_as_int(ohi.w);
         if (is_a) {
             merge_ab(lo, hi, olo, ohi, lo, hi);
-            r = far;
+            r = far_leaf(far);
+            dr = far_delta(far);
         } else {
             merge_ab(olo, ohi, lo, hi, lo, hi);
-            l = far;
+            l = far_leaf(far);
+            dl = far_delta(far);
         }
         link = g;
-        if (l == 0 && r == n - 1) {
-            A.root->root = g;
-            A.root->top_lo = lo;
-            A.root->top_hi = hi;
-            break;
+    }
+    // leaves before the chunk
+    uint32_t before = 0;
+    for (int c = tid; c < chunk; c += RB) {
+        int spins = 0;
+        if (c != tid) cw = ld_volatile(A.ucnt + c);
+        while (!(cw & CNT_READY)) {
+            if (++spins > SPIN_LIMIT) {
+                atomicOr(A.err, ERR_TIMEOUT);
+                break;
+            }
+            __nanosleep(32);
+            cw = ld_volatile(A.ucnt + c);
         }
+        before += cw & ~CNT_READY;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) S.wsum[warp] = before;
+    __syncthreads();
+    const int base = (int)__reduce_add_sync(0xffffffffu, lane < RW ? S.wsum[lane] : 0u);
+    const auto global_link = [&](float w) {
+        const int v = __float_as_int(w);
+        return __int_as_float(v >= 0 ? v + base : v - base);
+    };
+    if (tid == 0 && chunk == A.chunks - 1) A.root->n_leaves = base + cnt;
+    if (is_root) {  // the whole tree in one chunk; a single leaf has no root node
+        A.root->root = l == r ? -1 : link + base;
+        A.root->top_lo = make_float4(lo.x, lo.y, lo.z, 0.0f);
+        A.root->top_hi = make_float4(hi.x, hi.y, hi.z, 0.0f);
+    }
+    int up = -2;  // a piece's parent
+    if (out != -2) up = out;
+    else if (pend >= 0 && S.flag[pend] != 3u) up = pend;
+    const bool piece = tid < cnt && up != -2;
+    if (piece) atomicOr(&S.pbits[l >> 5], 1u << (l & 31));
+    __syncthreads();
+    if (piece) {
+        int ord = __popc(S.pbits[l >> 5] & ((1u << (l & 31)) - 1u));
+        for (int w = 0; w < (l >> 5); ++w) ord += __popc(S.pbits[w]);
+        if (ord < MAX_PIECES) {
+            S.plo[ord][0] = lo.x; S.plo[ord][1] = lo.y; S.plo[ord][2] = lo.z;
+            S.phi[ord][0] = hi.x; S.phi[ord][1] = hi.y; S.phi[ord][2] = hi.z;
+            S.pend[ord] = r;
+        }
+        if (up + base >= 0)  // always, unless a wait for the counts gave up
+            write_side(A.nodes, A.range, up + base, is_a, lo, hi, link >= 0 ? link + base : link - base, l + base,
+                       r + base);
     }
     __syncthreads();
-    if (i < n) {
-        A.leaves[2 * i] = __ldcg(A.tri_leaf + 2 * t);
-        A.leaves[2 * i + 1] = __ldcg(A.tri_leaf + 2 * t + 1);
-    }
-    // nodes of the chunk whose children both arrived here
-    {
-        const int g = c0 + tid;
-        if (g <= c1 - 2 && S.flag[tid] == 3u) {
-            const float4 alo = S.lo[tid][0], ahi = S.hi[tid][0], blo = S.lo[tid][1], bhi = S.hi[tid][1];
-            const int la = __float_as_int(ahi.w), rb = __float_as_int(bhi.w);
-            A.nodes[g].a_lo = alo;
-            A.nodes[g].a_hi = make_float4(ahi.x, ahi.y, ahi.z, __int_as_float(S.delta[la - c0]));
-            A.nodes[g].b_lo = blo;
-            A.nodes[g].b_hi = make_float4(bhi.x, bhi.y, bhi.z, __int_as_float(S.delta[rb - c0 + 1]));
-            A.range[g] = make_int2(la, rb);
-        }
-    }
-    // a climb that stopped at a node another chunk completes: its side, in the node
-    {
-        int g = out;
-        if (g < 0 && pend >= 0 && S.flag[pend - c0] != 3u) g = pend;
-        if (g >= 0) write_side(A.nodes, A.range, g, is_a, lo, hi, link, l, r, is_a ? dl : dr);
-    }
-    if (c0 < n) {
-        // thread tid: boundary j = c0 + tid (delta dk, BIG_DELTA past the last boundary)
-        // and leaf c0 + tid (its box, the identity box past the last leaf)
-        const int j = c0 + tid;
-        const int dk = j <= n - 2 ? S.delta[tid + 1] : BIG_DELTA;
-        int pm = dk, sm = dk;  // inclusive prefix / suffix min over the warp
-        float4 plo = leaf_lo, phi = leaf_hi, slo = leaf_lo, shi = leaf_hi;  // inclusive prefix / suffix unions
+    if (warp < 2) {  // warp 0 from the left (prefix records), warp 1 from the right (suffix records)
+        const bool right = warp == 1;
+        int np = lane < RW ? __popc(S.pbits[lane]) : 0;
+        np = min((int)__reduce_add_sync(0xffffffffu, np), MAX_PIECES);
+        int d[2], j[2], m2 = BIG_DELTA;
+        float4 blo[2], bhi[2], lo2 = ident_lo(), hi2 = ident_hi();  // and of the lane's pair
 #pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int e = right ? MAX_PIECES - 1 - (2 * lane + q) : 2 * lane + q;
+            const bool ok = e < np;
+            j[q] = ok ? S.pend[e] : 0;
+            d[q] = ok ? S.delta[j[q] + 1] : BIG_DELTA;
+            if (d[q] < 0) d[q] = BIG_DELTA;  // past the last boundary
+            blo[q] = ok ? make_float4(S.plo[e][0], S.plo[e][1], S.plo[e][2], 0.0f) : ident_lo();
+            bhi[q] = ok ? make_float4(S.phi[e][0], S.phi[e][1], S.phi[e][2], 0.0f) : ident_hi();
+            m2 = min(m2, d[q]);
+            box_union(lo2, hi2, blo[q], bhi[q]);
+        }
+        // one copy of the scan's step: this code runs once per chunk, so its length is
+        // instruction fetch time (2.4 us for both directions unrolled in one warp)
+#pragma unroll 1
         for (int o = 1; o < 32; o <<= 1) {
-            const int a = __shfl_up_sync(0xffffffffu, pm, o), b = __shfl_down_sync(0xffffffffu, sm, o);
-            const float4 al = shfl_f4(plo, o, true), ah = shfl_f4(phi, o, true);
-            const float4 bl = shfl_f4(slo, o, false), bh = shfl_f4(shi, o, false);
+            const int x = __shfl_up_sync(0xffffffffu, m2, o);
+            const float4 xl = shfl_f4(lo2, o), xh = shfl_f4(hi2, o);
             if (lane >= o) {
-                pm = min(pm, a);
-                box_union(plo, phi, al, ah);
-            }
-            if (lane + o < 32) {
-                sm = min(sm, b);
-                box_union(slo, shi, bl, bh);
+                m2 = min(m2, x);
+                box_union(lo2, hi2, xl, xh);
             }
         }
-        if (lane == 31) {
-            S.wmin[warp] = pm;
-            S.wlo[warp] = plo;
-            S.whi[warp] = phi;
+        if (lane == 31 && !right) {
+            cv.cmin[chunk] = m2;
+            st8(cv.cbox + 2 * chunk, lo2, hi2);
         }
-        __syncthreads();
-        if (warp == 0) {  // exclusive prefix / suffix over the warps, lane w for warp w
-            const bool in = lane < RW;
-            int a = in ? S.wmin[lane] : BIG_DELTA, b = a;  // inclusive scans, then shifted
-            float4 al = in ? S.wlo[lane] : ident_lo(), ah = in ? S.whi[lane] : ident_hi();
-            float4 bl = al, bh = ah;
-#pragma unroll
-            for (int o = 1; o < RW; o <<= 1) {
-                const int pa = __shfl_up_sync(0xffffffffu, a, o), pb = __shfl_down_sync(0xffffffffu, b, o);
-                const float4 pal = shfl_f4(al, o, true), pah = shfl_f4(ah, o, true);
-                const float4 pbl = shfl_f4(bl, o, false), pbh = shfl_f4(bh, o, false);
-                if (lane >= o) {
-                    a = min(a, pa);
-                    box_union(al, ah, pal, pah);
-                }
-                if (lane + o < RW) {
-                    b = min(b, pb);
-                    box_union(bl, bh, pbl, pbh);
-                }
-            }
-            // exclusive: the inclusive value of the neighbour (identity at the ends)
-            const int ea = __shfl_up_sync(0xffffffffu, a, 1), eb = __shfl_down_sync(0xffffffffu, b, 1);
-            const float4 eal = shfl_f4(al, 1, true), eah = shfl_f4(ah, 1, true);
-            const float4 ebl = shfl_f4(bl, 1, false), ebh = shfl_f4(bh, 1, false);
-            if (in) {
-                S.xpm[lane] = lane > 0 ? ea : BIG_DELTA;
-                S.xsm[lane] = lane + 1 < RW ? eb : BIG_DELTA;
-                S.xplo[lane] = lane > 0 ? eal : ident_lo();
-                S.xphi[lane] = lane > 0 ? eah : ident_hi();
-                S.xslo[lane] = lane + 1 < RW ? ebl : ident_lo();
-                S.xshi[lane] = lane + 1 < RW ? ebh : ident_hi();
-            }
-        }
-        __syncthreads();
-        const int wpm = S.xpm[warp], wsm = S.xsm[warp];
-        // strict prefix (suffix) minimum: delta below every delta to its left (right)
-        // in the chunk
-        const int ppm = __shfl_up_sync(0xffffffffu, pm, 1), nsm = __shfl_down_sync(0xffffffffu, sm, 1);
-        const int epm = min(wpm, lane > 0 ? ppm : BIG_DELTA);
-        const int esm = min(wsm, lane < 31 ? nsm : BIG_DELTA);
-        const bool pre = dk < epm, suf = dk < esm;
-        // the chunk's leaves up to leaf j, and after it
-        float4 up_lo = S.xplo[warp], up_hi = S.xphi[warp];
-        box_union(up_lo, up_hi, plo, phi);
-        float4 af_lo = S.xslo[warp], af_hi = S.xshi[warp];
-        {
-            const float4 nl = shfl_f4(slo, 1, false), nh = shfl_f4(shi, 1, false);
-            if (lane < 31) box_union(af_lo, af_hi, nl, nh);
-        }
-        // node of boundary j spans chunks: no smaller delta on one side inside the chunk,
-        // or j is the boundary to the next chunk
-        const bool span = j <= n - 2 && (j == c1 - 1 || (S.flag[tid] != 3u));
-        const unsigned bs = __ballot_sync(0xffffffffu, suf), bp = __ballot_sync(0xffffffffu, pre);
-        const unsigned bt = __ballot_sync(0xffffffffu, span);
+        // over the lanes before this one
+        int em = __shfl_up_sync(0xffffffffu, m2, 1);
+        float4 elo = shfl_f4(lo2, 1), ehi = shfl_f4(hi2, 1);
         if (lane == 0) {
-            S.wsr[warp] = __popc(bs);
-            S.wpr[warp] = __popc(bp);
-            S.wtop[warp] = __popc(bt);
+            em = BIG_DELTA;
+            elo = ident_lo();
+            ehi = ident_hi();
         }
-        __syncthreads();
-        if (warp == 0) {  // counts over the warps before / after warp `lane`, and in all
-            const bool in = lane < RW;
-            const int vs = in ? S.wsr[lane] : 0, vp = in ? S.wpr[lane] : 0, vt = in ? S.wtop[lane] : 0;
-            int is = vs, ip = vp, it = vt;  // inclusive prefix sums
+        const bool rec[2] = {d[0] < em, d[1] < min(em, d[0])}, span[2] = {d[0] != BIG_DELTA, d[1] != BIG_DELTA};
+        const unsigned lt = (1u << lane) - 1u;
+        const unsigned r_0 = __ballot_sync(0xffffffffu, rec[0]), r_1 = __ballot_sync(0xffffffffu, rec[1]);
+        const unsigned t_0 = __ballot_sync(0xffffffffu, span[0]), t_1 = __ballot_sync(0xffffffffu, span[1]);
+        int ir = __popc(r_0 & lt) + __popc(r_1 & lt), it = __popc(t_0 & lt) + __popc(t_1 & lt);
+        int2* const out_rec = (right ? cv.srec : cv.prec) + 32 * chunk;
+        float4* const out_box = (right ? cv.sbox : cv.pbox) + 64 * chunk;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int qs = __shfl_up_sync(0xffffffffu, is, o), qp = __shfl_up_sync(0xffffffffu, ip, o);
-                const int qt = __shfl_up_sync(0xffffffffu, it, o);
-                if (lane >= o) {
-                    is += qs;
-                    ip += qp;
-                    it += qt;
-                }
+        for (int q = 0; q < 2; ++q) {
+            // the chunk's leaves up to the boundary include the piece before it; those after it do not
+            float4 ilo = elo, ihi = ehi;
+            box_union(ilo, ihi, blo[q], bhi[q]);
+            if (rec[q] && ir < 32) {
+                out_rec[ir] = make_int2(j[q] + base, d[q]);
+                st8(out_box + 2 * ir, right ? elo : ilo, right ? ehi : ihi);
+                ++ir;
             }
-            const int ts = __shfl_sync(0xffffffffu, is, 31), tp = __shfl_sync(0xffffffffu, ip, 31);
-            const int tt = __shfl_sync(0xffffffffu, it, 31);
-            if (in) {
-                S.xos[lane] = ts - is;  // suffix records after warp `lane`
-                S.xop[lane] = ip - vp;
-                S.xot[lane] = it - vt;
-            }
-            if (lane == 0) {
-                S.nrec[0] = ts;
-                S.nrec[1] = tp;
-                S.nrec[2] = tt;
-            }
+            if (span[q] && !right) cv.top[MAX_PIECES * chunk + it++] = make_int2(j[q] + base, d[q]);
+            elo = ilo;
+            ehi = ihi;
         }
-        __syncthreads();
-        const int os = __popc(bs & ~((2u << lane) - 1u)) + S.xos[warp];
-        const int op = __popc(bp & ((1u << lane) - 1u)) + S.xop[warp];
-        const int ot = __popc(bt & ((1u << lane) - 1u)) + S.xot[warp];
-        if (suf && os < 32) {
-            cv.srec[32 * chunk + os] = make_int2(j, dk);
-            cv.sbox[2 * (32 * chunk + os)] = af_lo;
-            cv.sbox[2 * (32 * chunk + os) + 1] = af_hi;
+        if (lane == 0) {
+            cv.rcnt[2 * chunk + (right ? 1 : 0)] =
+                (uint32_t)min(__popc(r_0) + __popc(r_1), 32) | (uint32_t)(__popc(t_0) + __popc(t_1)) << 16;
         }
-        if (pre && op < 32) {
-            cv.prec[32 * chunk + op] = make_int2(j, dk);
-            cv.pbox[2 * (32 * chunk + op)] = up_lo;
-            cv.pbox[2 * (32 * chunk + op) + 1] = up_hi;
-        }
-        if (tid == BUILD_LEAVES - 1) {  // holds the whole chunk's prefix
-            cv.rcnt[3 * chunk] = min(S.nrec[0], 32);
-            cv.rcnt[3 * chunk + 1] = min(S.nrec[1], 32);
-            cv.rcnt[3 * chunk + 2] = min(S.nrec[2], 64);
-            cv.cmin[chunk] = min(wpm, pm);
-            cv.cbox[2 * chunk] = up_lo;
-            cv.cbox[2 * chunk + 1] = up_hi;
-        }
-        if (span && ot < 64) cv.top[64 * chunk + ot] = make_int2(j, dk);  // at most 61 per chunk
+    }
+    // meanwhile the other warps write the leaves, and the nodes whose children both arrived here
+    if (tid < cnt) {
+        st8(A.leaves + 2 * (base + tid), leaf.a, leaf.b);
+        A.ucode[base + tid] = k;
+        A.utri[base + tid] = t;
+    }
+    if (tid < cnt - 1 && S.flag[tid] == 3u) {
+        const int g = base + tid;
+        const float4 nal = S.lo[tid][0], nah = S.hi[tid][0], nbl = S.lo[tid][1], nbh = S.hi[tid][1];
+        st8(&A.nodes[g].a_lo, make_float4(nal.x, nal.y, nal.z, global_link(nal.w)),
+            make_float4(nah.x, nah.y, nah.z, 0.0f));
+        st8(&A.nodes[g].b_lo, make_float4(nbl.x, nbl.y, nbl.z, global_link(nbl.w)),
+            make_float4(nbh.x, nbh.y, nbh.z, 0.0f));
+        A.range[g] = make_int2(far_leaf(__float_as_int(nah.w)) + base, far_leaf(__float_as_int(nbh.w)) + base);
     }
     __syncthreads();  // the shared arrays are reused by the CTA's next chunk
-}
-
-// After chunk c's summary: the summaries per 32, 1024 and 32768 chunks.  Each entry
-// of level v counts its members as they finish (the CTA fences its writes, then
-// counts); the CTA that brings the count to the group's size reduces the group
-// into the level-v entry and counts that entry into level v + 1.
-__device__ void level_up(const RebuildArgs& A, int c, int n, int* s_last) {
-    const ChunkView& cv = A.cv;
-    const int lane = threadIdx.x & 31;
-    int cnt[NLEV];
-    level_counts(n, cnt);
-    int e = c;  // the finished entry of level v - 1
-    for (int v = 1; v < NLEV; ++v) {
-        const int grp = e >> 5;
-        __threadfence();  // every thread's summary writes before the count
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const uint32_t members = (uint32_t)min(32, cnt[v - 1] - 32 * grp);
-            *s_last = atomicAdd(A.gdone + cv.lev_off[v] + grp, 1u) == members - 1u ? 1 : 0;
-            __threadfence();  // the other members' writes before this CTA's reads
-        }
-        __syncthreads();
-        const bool last = *s_last != 0;
-        __syncthreads();  // s_last is rewritten on the next level
-        if (!last) return;
-        if (threadIdx.x < 32) {
-            const int k = 32 * grp + lane;
-            int m = BIG_DELTA;
-            float4 blo = ident_lo(), bhi = ident_hi();
-            if (k < cnt[v - 1]) {
-                m = __ldcg(cv.cmin + cv.lev_off[v - 1] + k);
-                blo = __ldcg(cv.cbox + 2 * (cv.lev_off[v - 1] + k));
-                bhi = __ldcg(cv.cbox + 2 * (cv.lev_off[v - 1] + k) + 1);
-            }
-            warp_box_reduce(blo, bhi);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (lane == 0) {
-                cv.cmin[cv.lev_off[v] + grp] = m;
-                cv.cbox[2 * (cv.lev_off[v] + grp)] = blo;
-                cv.cbox[2 * (cv.lev_off[v] + grp) + 1] = bhi;
-            }
-        }
-        e = grp;
-    }
-}
-
-// Nearest entry of level 0 (a chunk) left of chunk c (right, with right) whose min
-// delta is below d, through the summary levels: scan the 32 entries of the current
-// group, climb a level while nothing qualifies, then descend into the first group
-// that does.  -1: none.
-__device__ int nearest_chunk(const ChunkView& cv, const int cnt[NLEV], int c, int d, bool right, int lane, int* err) {
-    int idx = c;
-    for (int v = 0; v < NLEV; ++v) {
-        const int* m = cv.cmin + cv.lev_off[v];
-        const int base = idx & ~31, e = base + lane;
-        const bool hit = (right ? e > idx : e < idx) && e < cnt[v] && __ldcg(m + e) < d;
-        unsigned b = __ballot_sync(0xffffffffu, hit);
-        if (b) {
-            int f = right ? base + __ffs(b) - 1 : base + 31 - __clz(b);
-            for (int u = v - 1; u >= 0; --u) {  // descend: the first qualifying entry of group f
-                const int b2 = 32 * f, e2 = b2 + lane;
-                const bool h2 = e2 < cnt[u] && __ldcg(cv.cmin + cv.lev_off[u] + e2) < d;
-                b = __ballot_sync(0xffffffffu, h2);
-                if (!b) {  // the group's min said otherwise: corrupt summaries
-                    if (lane == 0) atomicOr(err, ERR_TIMEOUT);
-                    return -1;
-                }
-                f = right ? b2 + __ffs(b) - 1 : b2 + 31 - __clz(b);
-            }
-            return f;
-        }
-        if (right ? base + 32 >= cnt[v] : base == 0) return -1;  // no group beyond this one
-        idx >>= 5;
-    }
-    return -1;
 }
 
 // First record (in the records' order) of chunk c with delta below d whose position is
@@ -1149,94 +1196,151 @@ __device__ __forceinline__ int first_record(const int2* rec, int count, int g, i
     return k;
 }
 
-// union of the leaf boxes of chunks [a, b] (warp-uniform a, b), in every lane
-__device__ void chunk_union(const ChunkView& cv, const int cnt[NLEV], int a, int b, int lane, float4& lo,
-                            float4& hi) {
-    float4 ul = ident_lo(), uh = ident_hi();
-    for (int v = 0; v < NLEV && a <= b; ++v) {
-        const float4* bx = cv.cbox + 2 * cv.lev_off[v];
-        if ((a >> 5) == (b >> 5) || v == NLEV - 1) {
-            for (int e = a + lane; e <= b; e += 32) box_union(ul, uh, __ldcg(bx + 2 * e), __ldcg(bx + 2 * e + 1));
-            break;
+// The chunk summaries as the spanning nodes read them: from shared memory (STAGED) or,
+// for bodies of more than TOP_STAGED chunks, where they are.
+template <bool STAGED>
+struct Summaries {
+    const ChunkView& cv;
+    const TopSmem& S;
+    __device__ __forceinline__ int min_delta(int c) const { return STAGED ? S.cmin[c] : __ldcg(cv.cmin + c); }
+    // records of chunk c from the left / from the right, and its nodes that span chunks
+    __device__ __forceinline__ int prefixes(int c) const { return (int)(counts(2 * c) & 0xffffu); }
+    __device__ __forceinline__ int suffixes(int c) const { return (int)(counts(2 * c + 1) & 0xffffu); }
+    __device__ __forceinline__ int nodes(int c) const { return (int)(counts(2 * c) >> 16); }
+    __device__ __forceinline__ uint32_t counts(int i) const { return STAGED ? S.rcnt[i] : __ldcg(cv.rcnt + i); }
+    __device__ __forceinline__ void add_box(int c, float4& lo, float4& hi) const {
+        if (STAGED)
+            box_union(lo, hi, make_float4(S.lo[c][0], S.lo[c][1], S.lo[c][2], 0.0f),
+                      make_float4(S.hi[c][0], S.hi[c][1], S.hi[c][2], 0.0f));
+        else {
+            const f4x2 b = ld8_cg(cv.cbox + 2 * c);
+            box_union(lo, hi, b.a, b.b);
         }
-        const int e1 = a + lane, e2 = (b & ~31) + lane;
-        if (e1 <= (a | 31)) box_union(ul, uh, __ldcg(bx + 2 * e1), __ldcg(bx + 2 * e1 + 1));
-        if (e2 <= b) box_union(ul, uh, __ldcg(bx + 2 * e2), __ldcg(bx + 2 * e2 + 1));
-        a = (a >> 5) + 1;
-        b = (b >> 5) - 1;
     }
-    warp_box_reduce(ul, uh);
-    box_union(lo, hi, ul, uh);
-}
-
-// The nodes whose leaf range spans chunks, one warp each, independently: the range
-// ends are the nearest boundaries with a smaller delta on either side (the first
-// suffix / prefix record past the node with a smaller delta, in the node's chunk or
-// in the nearest chunk with a smaller min), the box is the union of the leaf boxes in
-// the range (the records' partial unions and whole chunks between), and the node
-// enters its parent (the range end with the larger delta) as the climb would have
-// put it there.
-__device__ void phase_top(const RebuildArgs& A, int n) {
-    const ChunkView& cv = A.cv;
-    int cnt[NLEV];
-    level_counts(n, cnt);
-    const int lane = (int)(threadIdx.x & 31u);
-    // each chunk's nodes that span chunks sit in its 64 slots; iteration `it` takes slot
-    // it / F of chunk it % F, so the (few, low) occupied slots spread over all warps
-    const uint32_t F = (uint32_t)cnt[0], slots = 64u * F;
-    const uint32_t nw = gridDim.x * RW;
-    for (uint32_t it = blockIdx.x * RW + (threadIdx.x >> 5); it < slots; it += nw) {
-        const uint32_t ch = it % F, sl = it / F;
-        if ((int)sl >= __ldcg(cv.rcnt + 3 * ch + 2)) continue;
-        const int2 item = __ldcg(cv.top + 64 * ch + sl);
-        const int g = item.x, d = item.y, c = g / BUILD_LEAVES;
-        if (g < 0 || g > n - 2 || c >= cnt[0]) {
-            if (lane == 0) atomicOr(A.err, ERR_TIMEOUT);
-            continue;
-        }
-        // left end: boundary jl (leaves from jl + 1), -1 = none
-        int2 q;
-        int jl = -1, dlft = -1, cl = -1;
-        float4 lo = ident_lo(), hi = ident_hi();
-        int k = first_record(cv.srec + 32 * c, __ldcg(cv.rcnt + 3 * c), g, d, false, lane, q);
-        int cc = c;
-        if (k < 0) {
-            cc = nearest_chunk(cv, cnt, c, d, false, lane, A.err);
-            if (cc >= 0) k = first_record(cv.srec + 32 * cc, __ldcg(cv.rcnt + 3 * cc), -1, d, false, lane, q);
-        }
-        if (k >= 0) {
-            jl = q.x;
-            dlft = q.y;
-            cl = cc;
-            box_union(lo, hi, __ldcg(cv.sbox + 2 * (32 * cc + k)), __ldcg(cv.sbox + 2 * (32 * cc + k) + 1));
-        }
-        // right end: boundary jr (leaves up to jr), n - 1 = none
-        int jr = n - 1, drgt = -1, cr = cnt[0] - 1;
-        k = first_record(cv.prec + 32 * c, __ldcg(cv.rcnt + 3 * c + 1), g, d, true, lane, q);
-        cc = c;
-        if (k < 0) {
-            cc = nearest_chunk(cv, cnt, c, d, true, lane, A.err);
-            if (cc >= 0) k = first_record(cv.prec + 32 * cc, __ldcg(cv.rcnt + 3 * cc + 1), -1, d, true, lane, q);
-        }
-        if (k >= 0) {
-            jr = q.x;
-            drgt = q.y;
-            cr = cc;
-            box_union(lo, hi, __ldcg(cv.pbox + 2 * (32 * cc + k)), __ldcg(cv.pbox + 2 * (32 * cc + k) + 1));
-        } else {
-            box_union(lo, hi, __ldcg(cv.cbox + 2 * cr), __ldcg(cv.cbox + 2 * cr + 1));  // the last chunk
-        }
-        chunk_union(cv, cnt, cl + 1, cr - 1, lane, lo, hi);
-        if (lane == 0) {
-            if (jl < 0 && jr == n - 1) {
-                A.root->root = g;
-                A.root->top_lo = lo;
-                A.root->top_hi = hi;
-            } else {
-                const bool is_a = drgt > dlft;
-                write_side(A.nodes, A.range, is_a ? jr : jl, is_a, lo, hi, g, jl + 1, jr, is_a ? dlft : drgt);
+    // nearest chunk left of c (right of c) whose min delta is below d; -1: none
+    __device__ int nearest(int c, int F, int d, bool right, int lane) const {
+        constexpr int W = STAGED ? 1 : 4;  // groups of 32 in flight
+        for (int b = right ? c + 1 : c - 1; right ? b < F : b >= 0; b += right ? 32 * W : -32 * W) {
+            int v[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const int i = right ? b + 32 * w + lane : b - 32 * w - lane;
+                v[w] = i >= 0 && i < F ? min_delta(i) : BIG_DELTA;
+            }
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const unsigned h = __ballot_sync(0xffffffffu, v[w] < d);
+                if (h) return right ? b + 32 * w + __ffs(h) - 1 : b - 32 * w - (__ffs(h) - 1);
             }
         }
+        return -1;
+    }
+};
+
+// One node that spans chunks, by one warp: the range ends are the nearest boundaries
+// with a smaller delta on either side (the first suffix / prefix record past the node
+// with a smaller delta, in the node's chunk or in the nearest chunk with a smaller min),
+// the box is the union of the leaf boxes in the range (the records' partial unions and
+// whole chunks between), and the node enters its parent (the range end with the larger
+// delta) as the climb would have put it there.
+template <bool STAGED>
+__device__ void top_node(const RebuildArgs& A, const Summaries<STAGED>& sum, int c, int sl, int n, int F, int lane) {
+    const ChunkView& cv = A.cv;
+    const int2 item = __ldcg(cv.top + MAX_PIECES * c + sl);
+    const int g = item.x, d = item.y;
+    if (g < 0 || g > n - 2) {
+        if (lane == 0) atomicOr(A.err, ERR_TIMEOUT);
+        return;
+    }
+    // both sides' searches first, then the loads they lead to
+    int2 ql, qr;
+    int kl = first_record(cv.srec + 32 * c, sum.suffixes(c), g, d, false, lane, ql), cl = c;
+    int kr = first_record(cv.prec + 32 * c, sum.prefixes(c), g, d, true, lane, qr), cr = c;
+    if (kl < 0) {
+        cl = sum.nearest(c, F, d, false, lane);
+        if (cl >= 0) kl = first_record(cv.srec + 32 * cl, sum.suffixes(cl), -1, d, false, lane, ql);
+    }
+    if (kr < 0) {
+        cr = sum.nearest(c, F, d, true, lane);
+        if (cr >= 0) kr = first_record(cv.prec + 32 * cr, sum.prefixes(cr), -1, d, true, lane, qr);
+    }
+    int jl = -1, dlft = -1, jr = n - 1, drgt = -1;  // leaves jl + 1 .. jr
+    float4 lo = ident_lo(), hi = ident_hi();
+    if (kl >= 0) {
+        jl = ql.x;
+        dlft = ql.y;
+        const f4x2 b = ld8_cg(cv.sbox + 2 * (32 * cl + kl));
+        box_union(lo, hi, b.a, b.b);
+    } else {
+        cl = -1;
+    }
+    if (kr >= 0) {
+        jr = qr.x;
+        drgt = qr.y;
+        const f4x2 b = ld8_cg(cv.pbox + 2 * (32 * cr + kr));
+        box_union(lo, hi, b.a, b.b);
+    } else {
+        cr = F;
+    }
+    float4 ul = ident_lo(), uh = ident_hi();
+    for (int e = cl + 1 + lane; e < cr; e += 32) sum.add_box(e, ul, uh);
+    warp_box_reduce(ul, uh);
+    box_union(lo, hi, ul, uh);
+    if (lane == 0) {
+        if (jl < 0 && jr == n - 1) {
+            A.root->root = g;
+            A.root->top_lo = lo;
+            A.root->top_hi = hi;
+        } else {
+            const bool is_a = drgt > dlft;
+            write_side(A.nodes, A.range, is_a ? jr : jl, is_a, lo, hi, g, jl + 1, jr);
+        }
+    }
+}
+
+// The nodes whose leaf range spans chunks, one warp each, independently.  Each CTA stages
+// the summaries it searches (28 bytes a chunk) and the running count of the chunks' nodes,
+// by which the warps share the nodes out.
+__device__ void phase_top(const RebuildArgs& A, TopSmem& S, uint32_t* s_scan) {
+    const ChunkView& cv = A.cv;
+    const int lane = (int)(threadIdx.x & 31u), F = A.chunks;
+    const int n = __ldcg(&A.root->n_leaves);
+    const uint32_t w0 = blockIdx.x * RW + (threadIdx.x >> 5), nw = gridDim.x * RW;
+    if (F > TOP_STAGED) {  // slot s of every chunk before slot s + 1 of any: the low ones are occupied
+        const Summaries<false> sum{cv, S};
+        for (uint64_t it = w0; it < (uint64_t)F * MAX_PIECES; it += nw) {
+            const int c = (int)(it % (uint32_t)F), sl = (int)(it / (uint32_t)F);
+            if (sl < sum.nodes(c)) top_node<false>(A, sum, c, sl, n, F, lane);
+        }
+        return;
+    }
+    const int i = 2 * (int)threadIdx.x;
+    const uint2 r0 = i < F ? __ldcg(reinterpret_cast<const uint2*>(cv.rcnt) + i) : make_uint2(0u, 0u);
+    const uint2 r1 = i + 1 < F ? __ldcg(reinterpret_cast<const uint2*>(cv.rcnt) + i + 1) : make_uint2(0u, 0u);
+    const uint32_t c0 = r0.x >> 16, c1 = r1.x >> 16;
+    reinterpret_cast<uint2*>(S.rcnt)[i] = r0;
+    reinterpret_cast<uint2*>(S.rcnt)[i + 1] = r1;
+    for (int c = threadIdx.x; c < F; c += RB) {
+        const f4x2 b = ld8_cg(cv.cbox + 2 * c);
+        S.cmin[c] = __ldcg(cv.cmin + c);
+        S.lo[c][0] = b.a.x; S.lo[c][1] = b.a.y; S.lo[c][2] = b.a.z;
+        S.hi[c][0] = b.b.x; S.hi[c][1] = b.b.y; S.hi[c][2] = b.b.z;
+    }
+    const uint32_t incl = block_scan_incl(c0 + c1, s_scan);
+    S.pre[i] = incl - c0 - c1;
+    S.pre[i + 1] = incl - c1;
+    if (i == TOP_STAGED - 2) S.pre[TOP_STAGED] = incl;
+    __syncthreads();
+    const Summaries<true> sum{cv, S};
+    const uint32_t total = S.pre[TOP_STAGED];
+    for (uint32_t it = w0; it < total; it += nw) {
+        int lo = 0, hi = F;  // the chunk: S.pre[lo] <= it < S.pre[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (S.pre[mid] <= it) lo = mid;
+            else hi = mid;
+        }
+        top_node<true>(A, sum, lo, (int)(it - S.pre[lo]), n, F, lane);
     }
 }
 
@@ -1253,32 +1357,42 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
     // before any CTA can change the root record
     const bool coherent = A.coherent && ld_volatile(reinterpret_cast<const uint32_t*>(&A.root->perm_valid)) != 0u;
     const int cur = coherent ? (int)ld_volatile(reinterpret_cast<const uint32_t*>(&A.root->sorted)) & 1 : 1;
-    const int n_prev = A.root->n_leaves;
     // what the later phases need at zero (read only after the next barrier)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.chg[0] = 0u;
         A.root->n_tris = nt;
     }
     {
+        const int k0 = blockIdx.x * RB + threadIdx.x, step = gridDim.x * RB;
         const size_t zw = (size_t)PASSES * RADIX + (size_t)PASSES * A.tiles_sort * RADIX + PASSES;
-        for (size_t k = (size_t)blockIdx.x * RB + threadIdx.x; k < zw; k += (size_t)gridDim.x * RB) A.ghist[k] = 0u;
-        for (int k = blockIdx.x * RB + threadIdx.x; k < A.n_entries; k += gridDim.x * RB) A.gdone[k] = 0u;
+        for (size_t k = k0; k < zw; k += step) A.ghist[k] = 0u;
+        for (int k = k0; k < BK_MAX; k += step) A.bcnt[k] = 0u;
+        for (int k = k0; k < A.chunks; k += step) A.ucnt[k] = 0u;
     }
     phase_verts(A);
-    bool ok = grid_barrier(A.sync, target, true, A.err, &s_ok);
-    if (ok) phase_boxes(A, s_red);
+    bool ok = true;
+    f3 cen[BOX_BATCH];
+    uint32_t old[BOX_BATCH];  // the last build's codes of the same triangles
+#pragma unroll
+    for (int q = 0; q < BOX_BATCH; ++q) {
+        const int t = (blockIdx.x + q * gridDim.x) * RB + threadIdx.x;
+        cen[q] = mk3(0.0f, 0.0f, 0.0f);
+        old[q] = coherent && t < nt ? A.codes[t] : 0u;
+    }
+    if (A.direct) {
+        phase_boxes<true>(A, s_red, cen);
+    } else {
+        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+        if (ok) phase_boxes<false>(A, s_red, cen);
+    }
     ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
-    if (ok) phase_codes(A, coherent, s_red, s_frame);
+    if (ok) phase_codes(A, coherent, s_red, s_frame, cen, old);
     ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
     // the sort: same decision in every CTA (from words complete at the barrier)
     const uint32_t nchg = ld_volatile(A.chg);
-    const bool merge = coherent && nchg <= (uint32_t)CHG_CAP;
     int after = cur;  // buffer holding this build's sorted list
-    bool fresh = true;  // the sorted list changed: de-duplicate it again
-    if (merge) {
-        if (nchg == 0u) {
-            fresh = false;  // every code as before: the last build's list and leaves stand
-        } else {
+    if (coherent && nchg <= (uint32_t)CHG_CAP) {
+        if (nchg > 0u) {  // else every code is as before: the last build's list stands
             after = cur ^ 1;
             if (ok)
                 phase_merge(A, (int)nchg, A.keys[cur], A.vals[cur], A.keys[after], A.vals[after],
@@ -1286,20 +1400,32 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
             ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
         }
     } else {
-        if (ok) phase_hist(A, reinterpret_cast<uint32_t*>(rb_smem));
-        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
-        for (int p = 0; p < PASSES; ++p) {
-            if (ok) phase_sort_pass(A, p, *reinterpret_cast<SortSmem*>(rb_smem), s_scan, &s_claim);
+        bool sorted = false;
+        if (coherent ? nt <= BK_MAX * (BK_CAP / 2) : nt <= SAMPLED_MAX) {
+            BucketSmem& S = *reinterpret_cast<BucketSmem*>(rb_smem);
+            const int nb = min((nt + BK_TARGET - 1) / BK_TARGET, BK_MAX);
+            after = cur ^ 1;
+            if (!coherent && nb > 1) {
+                if (ok) phase_sample(A, nb * OVERSAMPLE, S);
+                ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+            }
+            if (ok) phase_scatter(A, nb, coherent ? A.keys[cur] : nullptr, A.vals[cur], S);
             ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+            sorted = buckets_fit(A, nb, S, s_scan);
+            if (sorted) {
+                if (ok) phase_bucket_sort(A, nb, A.keys[after], A.vals[after], S);
+                ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+            }
         }
-        after = (PASSES - 1) & 1;
-    }
-    int n = n_prev;
-    if (fresh) {
-        if (ok) phase_unique_count(A, A.keys[after], s_scan);
-        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
-        if (ok) n = phase_unique_write(A, A.keys[after], A.vals[after], s_scan);
-        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+        if (!sorted) {
+            if (ok) phase_hist(A, reinterpret_cast<uint32_t*>(rb_smem));
+            ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+            for (int p = 0; p < PASSES; ++p) {
+                if (ok) phase_sort_pass(A, p, *reinterpret_cast<SortSmem*>(rb_smem), s_scan, &s_claim);
+                ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+            }
+            after = (PASSES - 1) & 1;
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // the sort buffers now hold this build's list, unless some wait gave up
@@ -1307,15 +1433,11 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
         A.root->perm_valid = bad ? 0 : 1;
         A.root->sorted = after;
     }
-    n = min(n, nt);
-    const int chunks = (n + BUILD_LEAVES - 1) / BUILD_LEAVES;
     if (ok)
-        for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
-            build_chunk(A, c, n, *reinterpret_cast<BuildSmem*>(rb_smem));
-            level_up(A, c, n, &s_claim);
-        }
+        for (int c = blockIdx.x; c < A.chunks; c += gridDim.x)
+            build_chunk(A, c, A.keys[after], A.vals[after], *reinterpret_cast<BuildSmem*>(rb_smem));
     ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
-    if (ok) phase_top(A, n);
+    if (ok) phase_top(A, *reinterpret_cast<TopSmem*>(rb_smem), s_scan);
     // the last CTA out leaves both counters at zero for the next launch
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1368,7 +1490,10 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals) {
     nt = nt_;
     has_normals = normals;
     tiles_sort = nt > 0 ? cdiv(nt, SORT_TILE) : 0;
-    max_ctas = std::max(1, cdiv(std::max(nt, 1), RB));
+    chunks = cdiv(std::max(nt, 1), RB);
+    // a chunk per CTA at most, but for a small body enough CTAs that the phases before
+    // the build spread over the SMs
+    max_ctas = std::max(chunks, std::min(SPREAD_CTAS, cdiv(std::max(nt, 1), RB / 4)));
     int ni = nt > 1 ? nt - 1 : 1;
     a.want(&xyz_in, (size_t)nv * 3 + 4);
     a.want(&nrm_in, (size_t)nv * 3 + 4);
@@ -1386,32 +1511,25 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals) {
     a.want(&nodes, (size_t)ni);
     a.want(&leaves, (size_t)nt * 2 + 2);
     a.want(&range, (size_t)ni);
-    chunks = cdiv(std::max(nt, 1), BUILD_LEAVES);
-    int entries = 0, e = chunks;
-    for (int v = 0; v < NLEV; ++v) {
-        lev_off[v] = entries;
-        entries += e;
-        e = cdiv(e, 32);
-    }
-    a.want(&cmin, (size_t)entries);
-    a.want(&cbox, 2 * (size_t)entries);
+    a.want(&cmin, (size_t)chunks);
+    a.want(&cbox, 2 * (size_t)chunks);
     a.want(&srec, 32 * (size_t)chunks);
     a.want(&sbox, 64 * (size_t)chunks);
     a.want(&prec, 32 * (size_t)chunks);
     a.want(&pbox, 64 * (size_t)chunks);
-    a.want(&rcnt, 3 * (size_t)chunks);
-    a.want(&top, 64 * (size_t)chunks);
+    a.want(&rcnt, 2 * (size_t)chunks);
+    a.want(&top, (size_t)MAX_PIECES * chunks);
     a.want(&root, 1);
     // histograms | sort status (PASSES x tiles x RADIX) | sort counters (the launch
-    // clears them) | CTA box unions | CTA leaf counts | change list | barrier counters
+    // clears them) | bucket counts | CTA box unions | chunk leaf counts | change list | barrier counters
     scratch_words = (size_t)PASSES * RADIX + (size_t)PASSES * tiles_sort * RADIX + PASSES;
     a.want(&scratch, scratch_words);
+    a.want(&bcnt, (size_t)BK_MAX);
+    a.want(&bkey, (size_t)SAMPLES);
     a.want(&part, 8 * (size_t)max_ctas);
-    a.want(&ucnt, (size_t)max_ctas);
+    a.want(&ucnt, (size_t)chunks);
     a.want(&chg, 1 + 3 * (size_t)CHG_CAP);
     a.want(&sync, 2);
-    n_entries = entries;
-    a.want(&gdone, (size_t)entries);
 }
 
 cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_err, cudaStream_t s, const float* xyz,
@@ -1431,6 +1549,7 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.thickness = thickness;
     A.depth = box_depth;
     A.coherent = b.coherent ? 1 : 0;
+    A.direct = b.nt <= DIRECT_MAX ? 1 : 0;
     A.tiles_sort = b.tiles_sort;
     A.verts = b.verts;
     A.tri_box = b.tri_box;
@@ -1446,8 +1565,7 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.leaves = b.leaves;
     A.range = b.range;
     A.root = b.root;
-    A.cv = ChunkView{b.cmin, b.cbox, b.srec, b.sbox, b.prec, b.pbox, b.rcnt, b.top,
-                     {b.lev_off[0], b.lev_off[1], b.lev_off[2], b.lev_off[3]}};
+    A.cv = ChunkView{b.cmin, b.cbox, b.srec, b.sbox, b.prec, b.pbox, b.rcnt, b.top};
     A.ghist = b.scratch;
     A.sstat = A.ghist + PASSES * RADIX;
     A.scount = A.sstat + (size_t)PASSES * b.tiles_sort * RADIX;
@@ -1455,8 +1573,9 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.ucnt = b.ucnt;
     A.chg = b.chg;
     A.sync = b.sync;
-    A.gdone = b.gdone;
-    A.n_entries = b.n_entries;
+    A.bcnt = b.bcnt;
+    A.bkey = b.bkey;
+    A.chunks = b.chunks;
     A.err = d_err;
     const int grid = std::min(res, b.max_ctas);
     void* args[] = {&A};

@@ -57,54 +57,43 @@ int scratch_address(void** out) {
 
 // Reference layout of the links (BRTreeNode, cudaBRT.h:34-115): the root is
 // internal node 0; an internal node that is child A takes the index of its last
-// leaf, child B of its first.  Pass 1 gives every internal node its index.
-// Both passes run only on a build that reported no error, and check every index
-// they read from the tree before using it: a build whose bounded wait gave up can
-// leave the shared array with another call's nodes, and nothing read from there may
-// send a store outside the caller's arrays.  A bad index sets ERR_INDEX instead.
-__device__ __forceinline__ bool tree_ok(const BvhRoot* root, const int* err, int n_tris, int& n) {
-    n = root->n_leaves;
-    return *err == 0 && n >= 2 && n <= n_tris;
-}
-
-__global__ void k_karras_index(const Node* __restrict__ nodes, const int2* __restrict__ range,
-                               const BvhRoot* __restrict__ root, int* __restrict__ kidx, int n_tris, int* err) {
-    int n;
-    if (!tree_ok(root, err, n_tris, n)) return;
+// leaf, child B of its first; links are +(i+1) internal, -(i+1) leaf.  The node split
+// at g over the leaves [l, r] has children over [l, g] and [g + 1, r], so their indices
+// are g and g + 1, and it is child A itself when its right end has the longer common
+// prefix: each node's links follow from its own range and four codes, in one pass.
+// The leaf count goes to the caller from the same launch; -1 if a bounded wait of the
+// build gave up or an index was out of range (a triangle's vertex index, or a range
+// read from the tree).  The pass runs only on a build that reported no error, and checks
+// the range it read before using it: a build whose bounded wait gave up can leave the
+// shared array with another call's nodes, and nothing read from there may send a store
+// outside the caller's arrays.
+// err: [0] the build's error word, [1] blocks of this launch that are done.
+__global__ void k_karras(const int2* __restrict__ range, const uint32_t* __restrict__ codes,
+                         const BvhRoot* __restrict__ root, int32_t* __restrict__ child_a,
+                         int32_t* __restrict__ child_b, int n_tris, int* err, int32_t* n_leaves) {
+    const int n = root->n_leaves;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n - 1) return;
-    if (g == root->root) kidx[g] = 0;
-    const int la = __float_as_int(nodes[g].a_lo.w), lb = __float_as_int(nodes[g].b_lo.w);
-    if (la >= n - 1 || lb >= n - 1) {
-        atomicOr(err, ERR_INDEX);
-        return;
+    if (*reinterpret_cast<volatile int*>(err) == 0 && n >= 2 && n <= n_tris && g < n - 1) {
+        const int2 q = range[g];
+        int k = -1;
+        if (q.x >= 0 && q.x <= g && q.y > g && q.y < n) {
+            const int dl = q.x > 0 ? __clz((int)(codes[q.x - 1] ^ codes[q.x])) : -1;
+            const int dr = q.y < n - 1 ? __clz((int)(codes[q.y] ^ codes[q.y + 1])) : -1;
+            k = q.x == 0 && q.y == n - 1 ? 0 : dr > dl ? q.y : q.x;
+        }
+        if (k < 0 || k > n - 2) {
+            atomicOr(err, ERR_INDEX);
+        } else {
+            child_a[k] = q.x == g ? -(g + 1) : g + 1;
+            child_b[k] = q.y == g + 1 ? -(g + 2) : g + 2;
+        }
     }
-    if (la >= 0) kidx[la] = range[la].y;
-    if (lb >= 0) kidx[lb] = range[lb].x;
-}
-
-// Pass 2: child links in the reference encoding (+(i+1) internal, -(i+1) leaf).
-__global__ void k_karras_links(const Node* __restrict__ nodes, const BvhRoot* __restrict__ root,
-                               const int* __restrict__ kidx, int32_t* __restrict__ child_a,
-                               int32_t* __restrict__ child_b, int n_tris, int* err) {
-    int n;
-    if (!tree_ok(root, err, n_tris, n)) return;
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n - 1) return;
-    const int k = kidx[g];
-    const int la = __float_as_int(nodes[g].a_lo.w), lb = __float_as_int(nodes[g].b_lo.w);
-    if (k < 0 || k >= n - 1 || la >= n - 1 || lb >= n - 1) {
-        atomicOr(err, ERR_INDEX);
-        return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(err + 1, 1) == (int)gridDim.x - 1)
+            *n_leaves = atomicAdd(err, 0) ? -1 : n;
     }
-    child_a[k] = la < 0 ? -(~la) - 1 : kidx[la] + 1;
-    child_b[k] = lb < 0 ? -(~lb) - 1 : kidx[lb] + 1;
-}
-
-// Leaf count to the caller; -1 if a bounded wait of the build gave up or an index
-// was out of range (a triangle's vertex index, or one read from the tree).
-__global__ void k_report(const BvhRoot* __restrict__ root, const int* __restrict__ err, int32_t* n_leaves) {
-    *n_leaves = *err ? -1 : root->n_leaves;
 }
 
 }  // namespace
@@ -128,9 +117,7 @@ extern "C" int visg_lbvh_build_noalloc(const float* d_xyz, const float* d_normal
     Arena plan;
     b.plan(plan, n_vertices, n_tris, d_normals != nullptr);
     int* d_err = nullptr;
-    int* kidx = nullptr;
     plan.want(&d_err, 4);
-    plan.want(&kidx, (size_t)n_tris + 1);
     size_t used = 0;
     for (auto& pl : plan.plan) used += pl.second;
     if (used > kScratchBytes) return bad(VISG_ERR_UNSUPPORTED);  // cannot happen within the size limits
@@ -145,20 +132,15 @@ extern "C" int visg_lbvh_build_noalloc(const float* d_xyz, const float* d_normal
     b.ucode = d_sorted_codes;
     b.utri = reinterpret_cast<uint32_t*>(d_sorted_tris);
 
-    // what must start at zero: the error word and the build's grid-barrier counters
-    // (the array holds the last call's data, laid out for its sizes); the build
-    // clears its histograms, look-back status words and tile counters itself
-    cudaError_t e = cudaMemsetAsync(d_err, 0, 4, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.sync, 0, 2 * sizeof(uint32_t), s);
+    // what must start at zero: the build's grid-barrier counters and the error word, which
+    // the plan lays side by side at its end (the array holds the last call's data, laid
+    // out for its sizes); the build clears its histograms, look-back status words and
+    // counters itself
+    cudaError_t e = cudaMemsetAsync(b.sync, 0, (size_t)((char*)(d_err + 2) - (char*)b.sync), s);
     if (e == cudaSuccess) e = lbvh_build(b, thickness, box_depth, d_err, s);
-    if (e == cudaSuccess && n_tris > 1) {
-        const unsigned grid = (unsigned)((n_tris + 255) / 256);
-        k_karras_index<<<grid, 256, 0, s>>>(b.nodes, b.range, b.root, kidx, n_tris, d_err);
-        k_karras_links<<<grid, 256, 0, s>>>(b.nodes, b.root, kidx, d_child_a, d_child_b, n_tris, d_err);
-        e = cudaGetLastError();
-    }
     if (e == cudaSuccess) {
-        k_report<<<1, 1, 0, s>>>(b.root, d_err, d_n_leaves);
+        k_karras<<<(unsigned)((n_tris + 255) / 256), 256, 0, s>>>(b.range, b.ucode, b.root, d_child_a, d_child_b,
+                                                                  n_tris, d_err, d_n_leaves);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? VISG_OK : bad(VISG_ERR_CUDA);

@@ -50,6 +50,30 @@ __device__ __forceinline__ f3 normalize(f3 v) { return mul(v, __frcp_rn(__fsqrt_
 
 __device__ __forceinline__ f3 xyz(float4 v) { return f3{v.x, v.y, v.z}; }
 
+// ---- 32-byte records: one 256-bit access (sm_100+) per record -----------------------------
+// A record of two float4 (state, leaf, box, one side of a node) is one sector; as two
+// 16-byte accesses each warp touches every sector twice.  Addresses are 32-byte aligned.
+struct f4x2 {
+    float4 a, b;
+};
+#define VISG_LD8(name, op, vol)                                                                                  \
+    __device__ __forceinline__ f4x2 name(const float4* p) {                                                     \
+        f4x2 r;                                                                                                 \
+        asm vol(op ".v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"                                            \
+                : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z),    \
+                  "=f"(r.b.w)                                                                                   \
+                : "l"(p));                                                                                      \
+        return r;                                                                                               \
+    }
+VISG_LD8(ld8_nc, "ld.global.nc", )           // data no one writes during the launch
+VISG_LD8(ld8_cg, "ld.global.cg", volatile)   // through L2: data another CTA wrote earlier in the launch
+#undef VISG_LD8
+__device__ __forceinline__ void st8(float4* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+                 "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(p)
+                 : "memory");
+}
+
 // ---- packed pairs (sm_100+ f32x2 instructions) -----------------------------------------
 // Two floats in one 64-bit register pair; every packed operation rounds each lane
 // to nearest on its own, so a lane gets exactly the bits the scalar intrinsic
