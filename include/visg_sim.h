@@ -64,7 +64,10 @@ typedef struct VisgParams {
     int32_t use_graph;     /* 1: replay multi-step loops as CUDA graphs (default), 0: launches  */
     int32_t split_collision; /* 1: collision in its own kernel over the vertices inside a body's
                                 box (default), 0: fused into the step kernel; same results.
-                                visg_autotune / visg_batch_autotune may change it.             */
+                                visg_autotune / visg_batch_autotune may change it.  A single
+                                garment of at most 512 vertices per SM is always stepped fused
+                                (collision_margin on): helper warps of the same kernel answer
+                                its queries beside the spring sums.                           */
     int32_t stage_neighbours; /* 1: each tile's block of spring entries is staged in shared
                                 memory by TMA bulk copies, 0: read through the L1 (default);
                                 same results.  visg_autotune / visg_batch_autotune may change it. */

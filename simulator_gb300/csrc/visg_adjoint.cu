@@ -90,9 +90,9 @@ __device__ int first_hit_d(const BvhView& bv, V q, int* err) {
             atomicOr(err, ERR_STACK);
             return -1;
         }
-        const Node& nd = bv.nodes[node];
-        const int la = __float_as_int(nd.a_lo.w), lb = __float_as_int(nd.b_lo.w);
-        const bool ol = in_box_d(p, nd.a_lo, nd.a_hi), orr = in_box_d(p, nd.b_lo, nd.b_hi);
+        const f4x2 a = ld8_nc(&bv.nodes[node].a_lo), b = ld8_nc(&bv.nodes[node].b_lo);
+        const int la = __float_as_int(a.a.w), lb = __float_as_int(b.a.w);
+        const bool ol = in_box_d(p, a.a, a.b), orr = in_box_d(p, b.a, b.b);
         if (ol && la < 0) return ~la;
         if (orr && lb < 0) return ~lb;
         const bool tl = ol && la >= 0, tr = orr && lb >= 0;

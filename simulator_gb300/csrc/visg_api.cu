@@ -56,6 +56,12 @@ constexpr int kBlocks[kNumBlocks] = {128, 256, 512, 1024};
 // memory: 16 entries per vertex (14 for 1024, whose two buffers must fit the 227 KB a
 // CTA may hold); two buffers take 32 / 64 / 128 / 224 KB
 constexpr int kStageCap[kNumBlocks] = {2048, 4096, 8192, 14336};
+// vertices per SM up to which a step has helper warps (twice the threads): beyond, the
+// main warps alone fill the SMs (64 registers: 1,024 threads an SM).  Step kernel with
+// contacts, without -> with: 64 x 64 sheet 10.7 -> 7.8 us, 131 x 127 damped mesh 9.2 and
+// 14.0 in the collision's own kernel -> 14.0 in all, 112 x 112 sheet over a body that has
+// just moved 17.9 -> 12.7
+constexpr int HELP_PER_SM = 512;
 int block_index(int b) {
     for (int i = 0; i < kNumBlocks; ++i)
         if (kBlocks[i] == b) return i;
@@ -150,6 +156,7 @@ struct Engine {
     uint32_t* d_wild = nullptr;                      // sticky: a record was not tame
     int stage = 0;                                   // stage sliced-ELL blocks (autotuned)
     BvhView* d_views = nullptr;
+    BvhRoot* d_roots = nullptr;                      // per garment (unset without a body)
     std::vector<BvhBuffers> bvh;
     int* d_err = nullptr;
     uint32_t* d_check = nullptr;
@@ -453,6 +460,7 @@ struct Engine {
         arena.want(&d_vcount, h_vcount.size());
         arena.want(&d_wild, 4);
         arena.want(&d_views, (size_t)G);
+        arena.want(&d_roots, (size_t)G);
         arena.want(&d_err, 4);
         arena.want(&d_check, 4);
         arena.want(&d_cand, (size_t)N + 1);
@@ -461,10 +469,11 @@ struct Engine {
         bvh.resize(G);
         for (int g = 0; g < G; ++g)
             if (gin[g].nt > 0) {
-                bvh[g].plan(arena, gin[g].nv, gin[g].nt, !gin[g].bnrm.empty());
+                bvh[g].plan(arena, gin[g].nv, gin[g].nt, !gin[g].bnrm.empty(), false);
                 bvh[g].coherent = true;  // rebuilt in place: the last build's order is at hand
             }
         CU(arena.commit());
+        for (int g = 0; g < G; ++g) bvh[g].root = d_roots + g;
         // upload
         std::vector<float4> st(2 * (size_t)N);
         float xo_is_x_bits;
@@ -510,6 +519,7 @@ struct Engine {
             std::vector<float>().swap(g.bnrm);
             std::vector<uint32_t>().swap(g.tris);
         }
+        if (N <= (int64_t)sm_count * kBlocks[0]) block = kBlocks[0];  // tiles for as many SMs as there can be
         finalized = true;
         return sync();
     }
@@ -518,15 +528,22 @@ struct Engine {
         int v = variant();
         const int bi = block_index(blk);
         if (stage && bi >= 0 && win_cap[bi] > 0) v |= SV_STAGED;
+        else if ((v & SV_COLLIDE) && blk <= kHelpBlockMax && helped())
+            v |= SV_HELP;
         return v;
     }
+
+    // whether the garments are few enough for helper warps beside the step's own
+    bool helped() const { return p.collide && any_body && p.collision_margin && N <= (int64_t)sm_count * HELP_PER_SM; }
 
     int variant() const {  // without the launch-shape dependent bits
         int v = 0;
         if (perk) v |= SV_PERK;
         if (p.verlet_damping == 1.0f) v |= SV_REFV;
         if (p.collide && any_body) v |= SV_COLLIDE;
-        if (p.collide && any_body && split) v |= SV_SPLIT;
+        // a single garment small enough for helper warps steps fused: they leave the step's
+        // end short, and a second kernel costs more than its queries
+        if (p.collide && any_body && split && !(G == 1 && helped())) v |= SV_SPLIT;
         if (p.check_every > 0) v |= SV_CHECK;
         uint32_t kdbits;
         std::memcpy(&kdbits, &p.spring_damping, 4);
@@ -571,7 +588,7 @@ struct Engine {
         const int t0 = (two && grp == 1) ? tsplit[bi] : 0, t1 = (two && grp == 0) ? tsplit[bi] : n_tiles[bi];
         a.tiles = d_tiles[bi] + t0;
         a.n_tiles = t1 - t0;
-        a.bodies = d_views;
+        a.roots = d_roots;
         a.err = d_err;
         a.check = d_check;
         a.cand = d_cand + ((two && grp == 1) ? vsplit : 0);  // a group queues at most its own vertices
@@ -1200,10 +1217,14 @@ struct Engine {
             const int bi = sv % kNumBlocks;
             const int blk = kBlocks[bi];
             if (stage && win_cap[bi] == 0) continue;
+            // few vertices: what a step takes then is the latency of its contacts, which the
+            // state at hand may not show (a sheet still falling); only shapes with helper warps
+            if (helped() && (stage || blk > kHelpBlockMax)) continue;
             const int occ = step_max_ctas_per_sm(variant(blk), blk, win_cap[bi]);
             std::vector<int> ctas;
             for (int c = 1; c <= occ; c *= 2) ctas.push_back(c);
             if (occ > 0 && ctas.back() != occ) ctas.push_back(occ);
+            if (helped()) ctas.clear();
             ctas.push_back(0);  // one tile per CTA
             for (int c : ctas) {
                 const int gr = c == 0 ? 0 : c * sm_count;

@@ -73,15 +73,19 @@ struct __align__(32) Node {
     float4 b_hi;  // child B max xyz
 };
 
-struct __align__(16) BvhRoot {
-    int root;      // root internal node, -1 when there are fewer than two leaves
-    int n_leaves;  // T' (after de-duplication)
-    int n_tris;    // T
-    int perm_valid;  // codes and keys/vals[sorted] hold the last build's codes and sorted list
-    float4 frame_lo, frame_hi;  // Morton frame: identity box U every expanded triangle box
+// Root record.  The first 64 bytes are what a query starts from, so that it begins with one
+// load round; an engine's records are one array, indexed by garment.
+struct __align__(64) BvhRoot {
+    int root;                   // root internal node, -1 when there are fewer than two leaves
+    int n_leaves;               // T' (after de-duplication)
+    const Node* nodes;          // (every build writes both pointers)
+    const float4* leaves;       // 2 per leaf: (v0.xyz, n.x) (n.y, n.z, triangle, 0)
+    long long pad_;
     float4 top_lo, top_hi;      // box of the root node (identity U children), or of the only leaf
-    int sorted;                 // which of the two sort buffers holds the last build's list
-    int pad_[3];
+    float4 frame_lo, frame_hi;  // Morton frame: identity box U every expanded triangle box
+    int n_tris;                 // T
+    int perm_valid;  // codes and keys/vals[sorted] hold the last build's codes and sorted list
+    int sorted;      // which of the two sort buffers holds the last build's list
 };
 
 // device view of one body's LBVH, as the step and query kernels use it
@@ -143,7 +147,8 @@ struct BvhBuffers {
     uint32_t* chg = nullptr;     // count + the triangles whose code changed since the last build
     uint32_t* sync = nullptr;    // grid-barrier counters, zero between builds
 
-    void plan(Arena& a, int nv_, int nt_, bool normals);
+    // everything but the root record when `own_root` is false (the caller provides `root`)
+    void plan(Arena& a, int nv_, int nt_, bool normals, bool own_root);
     BvhView view() const { return BvhView{nodes, leaves, root}; }
 };
 
@@ -177,7 +182,7 @@ struct StepArgs {
     const float* kent;
     const int4* tiles;
     int n_tiles;
-    const BvhView* bodies;  // per garment
+    const BvhRoot* roots;  // per garment
     int* err;
     uint32_t* check;  // [0] max |dx| bits, [1] non-finite count
     int2* cand;       // split collision: {vertex, garment} of the vertices inside their body's box
@@ -200,7 +205,9 @@ enum StepVariant : int {
     SV_KD0 = 16,      // spring damping exactly +0
     SV_SPLIT = 32,    // collision in its own kernel over a compacted candidate list
     SV_STAGED = 64,   // sliced-ELL blocks staged in shared memory by TMA bulk copies
+    SV_HELP = 128,    // helper warps answer the queries at the start positions beside the spring sums
 };
+constexpr int kHelpBlockMax = 256;  // tile sizes up to which there are kernels with helper warps
 // dynamic shared memory of a launch: two stage buffers of win_cap entries + barriers
 int step_smem_bytes(int variant, int win_cap);
 cudaError_t launch_step(const StepArgs& a, int variant, int block, int grid, cudaStream_t s);

@@ -1361,6 +1361,8 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.chg[0] = 0u;
         A.root->n_tris = nt;
+        A.root->nodes = A.nodes;
+        A.root->leaves = A.leaves;
     }
     {
         const int k0 = blockIdx.x * RB + threadIdx.x, step = gridDim.x * RB;
@@ -1485,7 +1487,7 @@ int resident_ctas() {
 
 }  // namespace
 
-void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals) {
+void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool own_root) {
     nv = nv_;
     nt = nt_;
     has_normals = normals;
@@ -1519,7 +1521,7 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals) {
     a.want(&pbox, 64 * (size_t)chunks);
     a.want(&rcnt, 2 * (size_t)chunks);
     a.want(&top, (size_t)MAX_PIECES * chunks);
-    a.want(&root, 1);
+    if (own_root) a.want(&root, 1);
     // histograms | sort status (PASSES x tiles x RADIX) | sort counters (the launch
     // clears them) | bucket counts | CTA box unions | chunk leaf counts | change list | barrier counters
     scratch_words = (size_t)PASSES * RADIX + (size_t)PASSES * tiles_sort * RADIX + PASSES;

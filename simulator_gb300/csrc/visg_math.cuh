@@ -66,6 +66,8 @@ struct f4x2 {
         return r;                                                                                               \
     }
 VISG_LD8(ld8_nc, "ld.global.nc", )           // data no one writes during the launch
+VISG_LD8(ld8, "ld.global", volatile)
+VISG_LD8(ld8_once, "ld.global.nc", volatile) // the same, not merged with an earlier load of the address
 VISG_LD8(ld8_cg, "ld.global.cg", volatile)   // through L2: data another CTA wrote earlier in the launch
 #undef VISG_LD8
 __device__ __forceinline__ void st8(float4* p, float4 a, float4 b) {

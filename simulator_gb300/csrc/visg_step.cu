@@ -20,6 +20,7 @@
 //   first-hit leaf (cudaBRT.cu:239-285) -> plane test (primitive.cu:110-125)
 //   -> x' += |dist| n, xo' = x', n_prev' = n; else n_prev' = 0
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <map>
@@ -58,80 +59,76 @@ __device__ __forceinline__ float box_inner(f3 p, float4 lo, float4 hi) {
                  fminf(__fsub_rd(p.z, lo.z), __fsub_rd(hi.z, p.z)));
 }
 
+// The box test as one number: the largest signed gap, rounded down.  A rounded-down
+// difference has the sign of the exact one (a difference of two floats is zero only if they
+// are equal), so a point without NaN is in the closed box exactly when this is not positive;
+// outside it is box_gap.
+__device__ __forceinline__ float box_side(f3 p, float4 lo, float4 hi) { return box_gap(p, lo, hi); }
+
 // D_BVH::intersect semantics: children tested pairwise; an overlapping leaf child is
 // returned before any descent (A before B); both internal -> descend A, push B.
 // The answer is therefore the first leaf, in a fixed order of the tree's leaves,
 // whose box contains p (a node's box contains its children's).  A depth-first walk
 // visits every internal node at most once, so `budget` (the number of internal
 // nodes) bounds the loop even on a corrupted tree.
-// With MARGIN, m receives a distance a point may move from p and keep the answer:
+// m receives a distance a point may move from p and keep the answer:
 // every leaf before the answer lies under a box the walk rejected (min of their
 // gaps), and the answer's own box must keep containing it (its inner distance).
-template <bool MARGIN>
+// A walk is one chain of dependent loads (285 cycles each when they miss the L1) and of
+// what is computed between them, which with a branch per outcome took longer than the
+// load: the lanes of a warp part at every visit.  So a visit has no branch but the loop's:
+// one signed gap per box serves the test and the margin, the next link is selected (a
+// leaf's or the empty stack's is negative and ends the walk), and the stack is written and
+// read at every visit, used or not, with its top in a register.
+// p has no NaN (query_margin sees to it).
 __device__ __forceinline__ int first_hit(const Node* __restrict__ nodes, int node, int budget, f3 p, int* err,
                                          float& m) {
+    constexpr int kEmpty = INT_MIN;
+    const float inf = __int_as_float(0x7f800000);
     int stack[kStack];
-    int sp = 0;
-    while (true) {
-        if (--budget < 0) {
-            atomicOr(err, ERR_STACK);
-            m = 0.0f;
-            return -1;
-        }
-        const Node* nd = nodes + node;
-        const float4 alo = __ldg(&nd->a_lo), ahi = __ldg(&nd->a_hi);
-        const float4 blo = __ldg(&nd->b_lo), bhi = __ldg(&nd->b_hi);
-        const int la = __float_as_int(alo.w), lb = __float_as_int(blo.w);
-        const bool ol = in_box(p, alo, ahi), orr = in_box(p, blo, bhi);
-        if (ol && la < 0) {
-            if (MARGIN) m = fminf(m, box_inner(p, alo, ahi));
-            return ~la;
-        }
-        if (MARGIN && !ol) m = fminf(m, box_gap(p, alo, ahi));
-        if (orr && lb < 0) {
-            if (MARGIN) m = fminf(m, box_inner(p, blo, bhi));
-            return ~lb;
-        }
-        if (MARGIN && !orr) m = fminf(m, box_gap(p, blo, bhi));
-        const bool tl = ol && la >= 0, tr = orr && lb >= 0;
-        if (!tl && !tr) {
-            if (sp == 0) return -1;
-            node = stack[--sp];
-        } else {
-            node = tl ? la : lb;
-            if (tl && tr) {
-                if (sp == kStack) {
-                    atomicOr(err, ERR_STACK);
-                    m = 0.0f;
-                    return -1;
-                }
-                stack[sp++] = lb;
-            }
-        }
+    int sp = 0, top = kEmpty;
+    f4x2 a, b;
+    bool hit_a;
+    do {
+        a = ld8_nc(&nodes[node].a_lo);
+        b = ld8_nc(&nodes[node].b_lo);
+        stack[sp] = top;
+        const int below = stack[max(sp - 1, 0)];
+        const int la = __float_as_int(a.a.w), lb = __float_as_int(b.a.w);
+        const float ga = box_side(p, a.a, a.b), gb = box_side(p, b.a, b.b);
+        const bool in_a = !(ga > 0.0f), in_b = !(gb > 0.0f);
+        hit_a = in_a && la < 0;
+        const bool hit_b = in_b && lb < 0 && !hit_a;
+        m = fminf(m, fminf(in_a ? inf : ga, in_b || hit_a ? inf : gb));
+        node = hit_b ? lb : in_a ? la : in_b ? lb : top;
+        const bool push = in_a && in_b, pop = !in_a && !in_b;
+        top = push ? lb : pop ? below : top;
+        sp += push ? 1 : pop ? -1 : 0;
+    } while (node >= 0 && --budget > 0 && sp < kStack);
+    if (node >= 0) {
+        atomicOr(err, ERR_STACK);
+        m = 0.0f;
+        return -1;
     }
+    if (node == kEmpty) return -1;
+    m = fminf(m, hit_a ? box_inner(p, a.a, a.b) : box_inner(p, b.a, b.b));
+    return ~node;
 }
 
 // The whole first-hit query of one body (root box, single leaf, walk) with its margin.
-__device__ __forceinline__ int query_margin(const BvhView& bv, f3 p, int* err, float& m) {
-    const int nl = bv.root->n_leaves;
-    const float4 lo = bv.root->top_lo, hi = bv.root->top_hi;
-    if (!in_box(p, lo, hi)) {
+__device__ __forceinline__ int query_margin(const BvhRoot* __restrict__ rt, f3 p, int* err, float& m) {
+    const f4x2 box = ld8_nc(&rt->top_lo);
+    const float4 lo = box.a, hi = box.b;
+    if (!in_box(p, lo, hi)) {  // also a NaN
         m = fminf(m, box_gap(p, lo, hi));
         return -1;
     }
+    const int nl = __ldg(&rt->n_leaves);
     if (nl == 1) {
         m = fminf(m, box_inner(p, lo, hi));
         return 0;
     }
-    return first_hit<true>(bv.nodes, bv.root->root, nl, p, err, m);
-}
-
-__device__ __forceinline__ int query_leaf(const BvhView& bv, int n_leaves, int root, float4 top_lo, float4 top_hi,
-                                          f3 p, int* err) {
-    if (n_leaves <= 0 || !in_box(p, top_lo, top_hi)) return -1;
-    if (n_leaves == 1) return 0;
-    float m = 0.0f;
-    return first_hit<false>(bv.nodes, root, n_leaves, p, err, m);
+    return first_hit(rt->nodes, __ldg(&rt->root), nl, p, err, m);
 }
 
 // Force of one spring on the vertex at x moving with velocity vel (verlet.cu:64-84):
@@ -180,13 +177,6 @@ __device__ __forceinline__ void spring_pair(fp2 xxy, float xz, float4 ta, float4
     fz_b = __fmul_rn(cb, __fmul_rn(dzb, ib));
 }
 
-// One 16-byte load that the compiler may not merge with an earlier load of the same
-// address (a value read again later instead of being held in registers meanwhile).
-__device__ __forceinline__ float4 ld_once(const float4* p) {
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
 
 // Contact data a vertex will read after its spring sum (its cached leaf, its stored
 // normal), prefetched when the vertex starts: 0 = not prefetched, 1 = into L1, 2 = L2.
@@ -205,6 +195,7 @@ struct GlobalRecords {
     const float4* __restrict__ p;
     __device__ __forceinline__ float4 r0(int j) const { return __ldg(p + 2 * j); }
     __device__ __forceinline__ float4 r1(int j) const { return __ldg(p + 2 * j + 1); }
+    __device__ __forceinline__ f4x2 both(int j) const { return ld8_nc(p + 2 * j); }
 };
 
 // A row's sliced-ELL entries (entry e at p[32 e]): in global memory, or in the tile's
@@ -250,21 +241,18 @@ __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const floa
     for (; e + 1 < end; e += 2) {
         const uint2 ea = ep[e], eb = ep[e + 1];
         const int ja = (int)(ea.x & END_MASK), jb = (int)(eb.x & END_MASK);
-        const float4 a0 = rec.r0(ja), b0 = rec.r0(jb);
-        const float4 a1 = FAST ? a0 : rec.r1(ja), b1 = FAST ? b0 : rec.r1(jb);
+        const f4x2 ra = rec.both(ja), rb = rec.both(jb);
         const float ka = perk ? -__ldg(kp + 32 * e) : nk;
         const float kb = perk ? -__ldg(kp + 32 * (e + 1)) : nk;
-        const f3 fa = spring_force<FAST>(x, vel, a0, a1, ka, __uint_as_float(ea.y), kd, eps3, drec, dt);
-        const f3 fb = spring_force<FAST>(x, vel, b0, b1, kb, __uint_as_float(eb.y), kd, eps3, drec, dt);
+        const f3 fa = spring_force<FAST>(x, vel, ra.a, ra.b, ka, __uint_as_float(ea.y), kd, eps3, drec, dt);
+        const f3 fb = spring_force<FAST>(x, vel, rb.a, rb.b, kb, __uint_as_float(eb.y), kd, eps3, drec, dt);
         acc = add(add(acc, fa), fb);
     }
     if (e < end) {
         const uint2 ea = ep[e];
-        const int ja = (int)(ea.x & END_MASK);
-        const float4 a0 = rec.r0(ja);
-        const float4 a1 = FAST ? a0 : rec.r1(ja);
+        const f4x2 ra = rec.both((int)(ea.x & END_MASK));
         const float ka = perk ? -__ldg(kp + 32 * e) : nk;
-        acc = add(acc, spring_force<FAST>(x, vel, a0, a1, ka, __uint_as_float(ea.y), kd, eps3, drec, dt));
+        acc = add(acc, spring_force<FAST>(x, vel, ra.a, ra.b, ka, __uint_as_float(ea.y), kd, eps3, drec, dt));
     }
     return acc;
 }
@@ -301,15 +289,59 @@ __device__ __forceinline__ bool tame_d(f3 x, f3 d, float dmax) {
            fabsf(d.z) < dmax;
 }
 
+// Helper warps (SV_HELP).  A first-hit walk is 10 to 40 dependent node loads of about 0.2 us
+// each, and at the end of a step it follows the spring sum.  Where the SMs have room, a
+// CTA has as many warps again: while the main warps sum the springs, helper lane j
+// answers the query of vertex j where its last displacement would take it again, if the
+// vertex's cached answer is unlikely to last (its margin is below twice that
+// displacement).  The answer comes with its own margin, so the main lane takes it over as
+// it takes a cached one: it holds if the step ends within the margin of the point that was
+// asked about, that is if the step's acceleration moved the vertex by less.  What neither
+// covers is queried (or queued) as before, by then with the walk's nodes in the L1.
+struct HelperAnswers {
+    int* leaf;
+    float* margin;     // 0: not asked
+    float (*point)[3];
+};
+__device__ __forceinline__ void pair_arrive(int pair) {
+    asm volatile("bar.arrive %0, 64;" ::"r"(pair + 1) : "memory");
+}
+__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); }
+
+__device__ __forceinline__ void helper_query(const StepArgs& a, const int4 td, const int j, const HelperAnswers& h) {
+    const int i = td.y + j;
+    int leaf = -1;
+    float m = 0.0f;
+    if ((td.x & TILE_BODY) && i < td.z && !(__ldg(&a.vcount[i].y) & PIN_BIT)) {
+        const f4x2 rec = ld8_nc(a.state_in + 2 * i);
+        f3 d = mk3(rec.a.w, rec.b.x, rec.b.y);  // D, or v
+        if (!a.p.drec) d = mul(d, a.p.dt);
+        if (!(rec.b.w > 2.0f * fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z))))) {
+            const BvhRoot* const rt = a.roots + (td.x & TILE_GARMENT);
+            const f3 p = add(mk3(rec.a.x, rec.a.y, rec.a.z), mul(a.p.gamma, d));
+            h.point[j][0] = p.x;
+            h.point[j][1] = p.y;
+            h.point[j][2] = p.z;
+            m = __int_as_float(0x7f800000);  // +inf
+            leaf = query_margin(rt, p, a.err, m);
+            if (leaf >= 0) prefetch_contact(rt->leaves + 2 * leaf);
+        }
+    }
+    h.leaf[j] = leaf;
+    h.margin[j] = m;
+    __syncwarp();
+    pair_arrive(j >> 5);
+}
+
 // One thread's vertex of tile td = {garment, first vertex, end vertex, first slice}.
 // State record of vertex i in buffer b: [x.xyz, v.x] [v.y, v.z, flags, 0] with
 // v = (x - x_old) / dt.  x_old is x itself when FLAG_XO_IS_X is set (after a
 // contact, a pin or update_vertex) and otherwise the previous step's x, which is
 // still in the other buffer: the step reads it there before overwriting it.
-template <bool COLL, bool KD0, bool SPLIT, bool SMEM_ENT>
+template <bool COLL, bool KD0, bool SPLIT, bool SMEM_ENT, bool HELP>
 __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, const uint2* ebase, const uint32_t e0,
                                             const int refv, const int check, const int perk, const bool wild,
-                                            float& my_disp, uint32_t& my_bad) {
+                                            const HelperAnswers& help, float& my_disp, uint32_t& my_bad) {
     const GlobalRecords rec{a.state_in};
     const StepParams& P = a.p;
     const f3 grav = mk3(P.gx, P.gy, P.gz);
@@ -325,8 +357,8 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         // the record's flags word (the sector s0 came in): start the loads that a cached
         // contact answer and a stored normal need after the spring sum
         const uint32_t fl0 = __float_as_uint(__ldg(reinterpret_cast<const float*>(a.state_in + 2 * ii + 1) + 2));
-        if (fl0 & FLAG_LEAF_CACHED)
-            prefetch_contact(a.bodies[td.x & TILE_GARMENT].leaves + 2 * (fl0 >> LEAF_SHIFT));
+        const BvhRoot* const rt = a.roots + (td.x & TILE_GARMENT);
+        if (fl0 & FLAG_LEAF_CACHED) prefetch_contact(rt->leaves + 2 * (fl0 >> LEAF_SHIFT));
         if (fl0 & FLAG_HAS_NORMAL) prefetch_contact(a.normal + ii);
     }
     f3 xn = x, xon = x, nn = mk3(0.0f, 0.0f, 0.0f);
@@ -365,7 +397,8 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
             F = row_forces<false>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
         }
         // the record again (a second read of a line this thread has just read)
-        const float4 r0 = ld_once(a.state_in + 2 * ii), r1 = ld_once(a.state_in + 2 * ii + 1);
+        const f4x2 own = ld8_once(a.state_in + 2 * ii);
+        const float4 r0 = own.a, r1 = own.b;
         const f3 rv = mk3(r0.w, r1.x, r1.y);  // v, or D = x - x_old with drec
         flags = __float_as_uint(r1.z);
         margin = r1.w;
@@ -399,15 +432,25 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         const bool body = (td.x & TILE_BODY) != 0;  // the garment has a body (its tree has leaves)
         bool query = false;
         int leaf = -1;
+        if (HELP) {
+            __syncwarp();
+            pair_sync((int)(threadIdx.x >> 5));
+        }
         if (body && active && !pinned) {
-            const float rem = P.margin ? __fsub_rd(margin, disp_bound(xn, x)) : 0.0f;
+            float rem = P.margin ? __fsub_rd(margin, disp_bound(xn, x)) : 0.0f;
+            if (rem > 0.0f) {
+                if (flags & FLAG_LEAF_CACHED) leaf = (int)(flags >> LEAF_SHIFT);
+            } else if (HELP && help.margin[threadIdx.x] > 0.0f) {
+                const float* q = help.point[threadIdx.x];
+                rem = __fsub_rd(help.margin[threadIdx.x], disp_bound(xn, mk3(q[0], q[1], q[2])));
+                leaf = help.leaf[threadIdx.x];
+            }
             if (rem > 0.0f) {
                 skin = rem;
-                if (flags & FLAG_LEAF_CACHED) {
-                    leaf = (int)(flags >> LEAF_SHIFT);
-                    leaf_bits = (flags & ~7u) | FLAG_LEAF_CACHED;
-                }
+                if (leaf >= 0 && leaf < kLeafCacheMax) leaf_bits = ((uint32_t)leaf << LEAF_SHIFT) | FLAG_LEAF_CACHED;
+                else if (leaf >= 0) skin = 0.0f;  // the leaf does not fit the flags word: not cached
             } else {
+                leaf = -1;
                 query = true;
             }
         }
@@ -424,16 +467,16 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
             }
         } else if (__any_sync(0xffffffffu, query) && query) {
             float m = __int_as_float(0x7f800000);  // +inf
-            leaf = query_margin(a.bodies[g], xn, a.err, m);
+            leaf = query_margin(a.roots + g, xn, a.err, m);
             if (P.margin) {
                 skin = m;
                 if (leaf >= 0 && leaf < kLeafCacheMax) leaf_bits = ((uint32_t)leaf << LEAF_SHIFT) | FLAG_LEAF_CACHED;
             }
         }
         if (leaf >= 0) {  // plane test of the first-hit leaf (primitive.cu:110-125)
-            const float4* const leaves = a.bodies[g].leaves;
-            const float4 L0 = __ldg(&leaves[2 * leaf]);
-            const float4 L1 = __ldg(&leaves[2 * leaf + 1]);
+            const float4* const leaves = a.roots[g].leaves;
+            const f4x2 lf = ld8_nc(leaves + 2 * leaf);
+            const float4 L0 = lf.a, L1 = lf.b;
             const f3 n = mk3(L0.w, L1.x, L1.y);
             const float d = dot(sub(xn, mk3(L0.x, L0.y, L0.z)), n);
             if (!(d > 0.0f)) {
@@ -454,8 +497,8 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         untamed = P.drec ? !tame_d(xn, dn, P.dmax) : !tame(xn, vn);
         const uint32_t fl = (has_n ? FLAG_HAS_NORMAL : 0u) | (xo_is_x ? FLAG_XO_IS_X : 0u) |
                             (skin > 0.0f ? leaf_bits : 0u);
-        a.state_out[2 * i] = make_float4(xn.x, xn.y, xn.z, vn.x);
-        a.state_out[2 * i + 1] = make_float4(vn.y, vn.z, __uint_as_float(fl), skin > 0.0f ? skin : 0.0f);
+        st8(a.state_out + 2 * i, make_float4(xn.x, xn.y, xn.z, vn.x),
+            make_float4(vn.y, vn.z, __uint_as_float(fl), skin > 0.0f ? skin : 0.0f));
         if (has_n) a.normal[i] = make_float4(nn.x, nn.y, nn.z, 0.0f);
         if (check) {
             const float dd = fmaxf(fabsf(__fsub_rn(xn.x, x.x)),
@@ -546,16 +589,26 @@ __device__ __forceinline__ void stage_entries(const StepArgs& a, int tile, uint3
 // gives up after kWaitNs sets ERR_TIMEOUT, the iteration's stager waits (again
 // bounded) for the copies in flight, and the warp exits; warps left waiting on a
 // copy that is never issued give up the same way.
-template <int BLOCK, bool COLL, bool KD0, bool SPLIT, bool STAGED>
-__global__ void __launch_bounds__(BLOCK) k_step(const StepArgs a, const int refv, const int check, const int perk) {
+//
+// HELP: BLOCK more threads are helper warps (above); one tile per CTA.
+template <int BLOCK, bool COLL, bool KD0, bool SPLIT, bool STAGED, bool HELP>
+__global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK)
+    k_step(const StepArgs a, const int refv, const int check, const int perk) {
     extern __shared__ __align__(128) unsigned char dyn_smem[];
+    __shared__ int s_leaf[HELP ? BLOCK : 1];
+    __shared__ float s_margin[HELP ? BLOCK : 1], s_point[HELP ? BLOCK : 1][3];
+    const HelperAnswers help{s_leaf, s_margin, s_point};
+    if (HELP && threadIdx.x >= BLOCK) {
+        helper_query(a, __ldg(&a.tiles[blockIdx.x]), (int)threadIdx.x - BLOCK, help);
+        return;
+    }
     float my_disp = 0.0f;
     uint32_t my_bad = 0;
     const bool wild = *reinterpret_cast<const volatile uint32_t*>(a.wild) != 0u;
     if (!STAGED) {
         for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x)
-            vertex_step<COLL, KD0, SPLIT, false>(a, __ldg(&a.tiles[tile]), a.sell, 0u, refv, check, perk, wild,
-                                                 my_disp, my_bad);
+            vertex_step<COLL, KD0, SPLIT, false, HELP>(a, __ldg(&a.tiles[tile]), a.sell, 0u, refv, check, perk, wild,
+                                                       help, my_disp, my_bad);
     } else {
         // two-buffer ring: full[b] completes when buffer b holds its tile's block,
         // empty[b] when every warp is done reading it
@@ -598,10 +651,11 @@ __global__ void __launch_bounds__(BLOCK) k_step(const StepArgs a, const int refv
             const int4 td = __ldg(&a.tiles[tile]);
             const int2 tw = __ldg(&a.twin[tile]);
             if (tw.y > 0)
-                vertex_step<COLL, KD0, SPLIT, true>(a, td, sbuf + (size_t)b * a.win_cap, (uint32_t)tw.x, refv, check,
-                                                    perk, wild, my_disp, my_bad);
+                vertex_step<COLL, KD0, SPLIT, true, false>(a, td, sbuf + (size_t)b * a.win_cap, (uint32_t)tw.x, refv,
+                                                           check, perk, wild, help, my_disp, my_bad);
             else
-                vertex_step<COLL, KD0, SPLIT, false>(a, td, a.sell, 0u, refv, check, perk, wild, my_disp, my_bad);
+                vertex_step<COLL, KD0, SPLIT, false, false>(a, td, a.sell, 0u, refv, check, perk, wild, help, my_disp,
+                                                            my_bad);
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + 8u * b);
         }
@@ -630,17 +684,18 @@ __global__ void __launch_bounds__(COLLIDE_BLOCK) k_collide(const StepArgs a) {
     const float dt = a.p.dt;
     for (uint32_t k = blockIdx.x * COLLIDE_BLOCK + threadIdx.x; k < n; k += gridDim.x * COLLIDE_BLOCK) {
         const int2 c = a.cand[k];
-        const BvhView bv = a.bodies[c.y];
-        float4 s0 = a.state_out[2 * c.x], s1 = a.state_out[2 * c.x + 1];
+        const BvhRoot* const rt = a.roots + c.y;
+        const f4x2 rec = ld8(a.state_out + 2 * c.x);
+        float4 s0 = rec.a, s1 = rec.b;
         f3 xn = mk3(s0.x, s0.y, s0.z);
         float m = __int_as_float(0x7f800000);  // +inf
-        const int leaf = query_margin(bv, xn, a.err, m);
+        const int leaf = query_margin(rt, xn, a.err, m);
         uint32_t fl = __float_as_uint(s1.z);
         float skin = a.p.margin ? m : 0.0f;
         if (leaf >= 0) {
             if (a.p.margin && leaf < kLeafCacheMax) fl |= ((uint32_t)leaf << LEAF_SHIFT) | FLAG_LEAF_CACHED;
-            const float4 L0 = __ldg(&bv.leaves[2 * leaf]);
-            const float4 L1 = __ldg(&bv.leaves[2 * leaf + 1]);
+            const f4x2 lf = ld8_nc(rt->leaves + 2 * leaf);
+            const float4 L0 = lf.a, L1 = lf.b;
             const f3 nrm = mk3(L0.w, L1.x, L1.y);
             const float d = dot(sub(xn, mk3(L0.x, L0.y, L0.z)), nrm);
             if (!(d > 0.0f)) {
@@ -652,7 +707,6 @@ __global__ void __launch_bounds__(COLLIDE_BLOCK) k_collide(const StepArgs a) {
                 s1.x = vn.y;
                 s1.y = vn.z;
                 fl |= FLAG_HAS_NORMAL | FLAG_XO_IS_X;
-                a.state_out[2 * c.x] = s0;
                 a.normal[c.x] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
                 if (!tame(xn, vn)) atomicOr(a.wild, 1u);
             }
@@ -661,21 +715,32 @@ __global__ void __launch_bounds__(COLLIDE_BLOCK) k_collide(const StepArgs a) {
             skin = 0.0f;
             fl &= 7u & ~FLAG_LEAF_CACHED;
         }
-        a.state_out[2 * c.x + 1] = make_float4(s1.x, s1.y, __uint_as_float(fl), skin);
+        st8(a.state_out + 2 * c.x, s0, make_float4(s1.x, s1.y, __uint_as_float(fl), skin));
     }
 }
 
 int g_collide_grid = 0;
 
 // the step kernel instance of a variant
-template <int BLOCK, bool KD0, bool STAGED>
 using StepKernel = void (*)(const StepArgs, const int, const int, const int);
 
-template <int BLOCK, bool KD0, bool STAGED>
-StepKernel<BLOCK, KD0, STAGED> step_kernel(bool coll, bool split) {
-    if (coll && split) return k_step<BLOCK, true, KD0, true, STAGED>;
-    if (coll) return k_step<BLOCK, true, KD0, false, STAGED>;
-    return k_step<BLOCK, false, KD0, false, STAGED>;
+template <int BLOCK, bool KD0, bool STAGED, bool HELP>
+StepKernel step_kernel(bool coll, bool split) {
+    if (coll && split) return k_step<BLOCK, true, KD0, true, STAGED, HELP>;
+    if (coll || HELP) return k_step<BLOCK, true, KD0, false, STAGED, HELP>;
+    return k_step<BLOCK, false, KD0, false, STAGED, false>;
+}
+
+template <int BLOCK>
+StepKernel step_kernel(int variant) {
+    const bool coll = (variant & SV_COLLIDE) != 0, split = (variant & SV_SPLIT) != 0, kd0 = (variant & SV_KD0) != 0;
+    if (variant & SV_STAGED) return kd0 ? step_kernel<BLOCK, true, true, false>(coll, split)
+                                        : step_kernel<BLOCK, false, true, false>(coll, split);
+    if constexpr (BLOCK <= kHelpBlockMax)
+        if (variant & SV_HELP) return kd0 ? step_kernel<BLOCK, true, false, true>(coll, split)
+                                          : step_kernel<BLOCK, false, false, true>(coll, split);
+    return kd0 ? step_kernel<BLOCK, true, false, false>(coll, split)
+               : step_kernel<BLOCK, false, false, false>(coll, split);
 }
 
 // largest dynamic shared memory each kernel instance has been opened up to (per device)
@@ -699,20 +764,24 @@ cudaError_t allow_smem(const void* fn, int bytes) {
 // (kernel timing; null = none)
 thread_local cudaEvent_t t_before_step = nullptr, t_after_step = nullptr;
 
-template <int BLOCK, bool KD0, bool STAGED>
-cudaError_t launch_kd(const StepArgs& a, bool coll, bool split, int refv, int check, int perk, int grid, int smem,
-                      cudaStream_t s) {
-    const auto fn = step_kernel<BLOCK, KD0, STAGED>(coll, split);
+template <int BLOCK>
+cudaError_t launch_block(const StepArgs& a, int variant, int grid, cudaStream_t s) {
+    // helper warps need one tile per CTA and the entries read from global memory
+    const bool help = BLOCK <= kHelpBlockMax && (variant & SV_HELP) && !(variant & SV_STAGED) && grid == a.n_tiles;
+    const StepKernel fn = step_kernel<BLOCK>(help ? variant : variant & ~SV_HELP);
+    const bool split = (variant & SV_COLLIDE) && (variant & SV_SPLIT);
+    const int smem = step_smem_bytes(variant, a.win_cap);
     cudaError_t e = allow_smem((const void*)fn, smem);
     if (e != cudaSuccess) return e;
-    if (coll && split) {
+    if (split) {
         e = cudaMemsetAsync(a.cand_count, 0, sizeof(uint32_t), s);
         if (e != cudaSuccess) return e;
     }
     if (t_before_step) cudaEventRecord(t_before_step, s);
-    fn<<<grid, BLOCK, smem, s>>>(a, refv, check, perk);
+    fn<<<grid, help ? 2 * BLOCK : BLOCK, smem, s>>>(a, (variant & SV_REFV) ? 1 : 0, (variant & SV_CHECK) ? 1 : 0,
+                                                    (variant & SV_PERK) ? 1 : 0);
     if (t_after_step) cudaEventRecord(t_after_step, s);
-    if (coll && split) {
+    if (split) {
         if (g_collide_grid == 0) {
             int dev = 0, sms = 0, occ = 0;
             cudaGetDevice(&dev);
@@ -728,38 +797,13 @@ cudaError_t launch_kd(const StepArgs& a, bool coll, bool split, int refv, int ch
 }
 
 template <int BLOCK>
-cudaError_t launch_block(const StepArgs& a, int variant, int grid, cudaStream_t s) {
-    const int refv = (variant & SV_REFV) ? 1 : 0;
-    const int check = (variant & SV_CHECK) ? 1 : 0;
-    const int perk = (variant & SV_PERK) ? 1 : 0;
-    const bool coll = (variant & SV_COLLIDE) != 0, split = (variant & SV_SPLIT) != 0;
-    const int smem = step_smem_bytes(variant, a.win_cap);
-    if (variant & SV_STAGED) {
-        if (variant & SV_KD0) return launch_kd<BLOCK, true, true>(a, coll, split, refv, check, perk, grid, smem, s);
-        return launch_kd<BLOCK, false, true>(a, coll, split, refv, check, perk, grid, smem, s);
-    }
-    if (variant & SV_KD0) return launch_kd<BLOCK, true, false>(a, coll, split, refv, check, perk, grid, 0, s);
-    return launch_kd<BLOCK, false, false>(a, coll, split, refv, check, perk, grid, 0, s);
-}
-
-template <int BLOCK, bool KD0, bool STAGED>
-int occupancy_kd(bool coll, bool split, int smem) {
-    const auto fn = step_kernel<BLOCK, KD0, STAGED>(coll, split);
+int occupancy_block(int variant, int win_cap) {
+    const StepKernel fn = step_kernel<BLOCK>(variant & ~SV_HELP);
+    const int smem = step_smem_bytes(variant, win_cap);
     if (allow_smem((const void*)fn, smem) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, BLOCK, smem) != cudaSuccess) return 0;
     return n;
-}
-
-template <int BLOCK>
-int occupancy_block(int variant, int win_cap) {
-    const bool coll = (variant & SV_COLLIDE) != 0, split = (variant & SV_SPLIT) != 0;
-    const int smem = step_smem_bytes(variant, win_cap);
-    if (variant & SV_STAGED)
-        return (variant & SV_KD0) ? occupancy_kd<BLOCK, true, true>(coll, split, smem)
-                                  : occupancy_kd<BLOCK, false, true>(coll, split, smem);
-    return (variant & SV_KD0) ? occupancy_kd<BLOCK, true, false>(coll, split, 0)
-                              : occupancy_kd<BLOCK, false, false>(coll, split, 0);
 }
 
 __global__ void k_query(BvhView bv, const float* __restrict__ pts, int n, int* leaf, int* inside, float* dist,
@@ -767,8 +811,8 @@ __global__ void k_query(BvhView bv, const float* __restrict__ pts, int n, int* l
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const f3 p = mk3(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
-    const int nl = bv.root->n_leaves;
-    const int lf = query_leaf(bv, nl, bv.root->root, bv.root->top_lo, bv.root->top_hi, p, err);
+    float m = 0.0f;
+    const int lf = bv.root->n_leaves > 0 ? query_margin(bv.root, p, err, m) : -1;
     float d = 0.0f;
     f3 nn = mk3(0.0f, 0.0f, 0.0f);
     int in = 0;
