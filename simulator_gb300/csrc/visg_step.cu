@@ -152,16 +152,20 @@ __device__ __forceinline__ f3 spring_force(f3 x, f3 vel, float4 t0, float4 t1, f
     return mul(c, mul(dP, __frcp_rn(dist)));  // normalize(dP) = dP * (1 / |dP|)
 }
 
-// Two springs of one vertex at once, spring damping exactly +0 (spring_force<true>
-// on each spring, operation for operation).  The x and y components of a spring's
+// Two springs of one vertex at once (spring_force on each spring, operation for
+// operation).  The x and y components of a spring's
 // vectors travel as one packed pair (a record's x, y are adjacent words), z alone;
 // the two springs' scalar chains (|dP|^2, the square root and its reciprocal, the
-// rest-length term) travel as one pair.  Every packed operation rounds each lane as
-// the scalar intrinsic would, and sqrt_rcp_pair returns __fsqrt_rn / __frcp_rn's
-// bits, so each force is bit-identical to the scalar form in fewer instructions
-// (sm_100+ f32x2 arithmetic).
-__device__ __forceinline__ void spring_pair(fp2 xxy, float xz, float4 ta, float4 tb, fp2 nk, fp2 rest, fp2 eps2,
-                                            float eps, fp2& f_xy_a, float& fz_a, fp2& f_xy_b, float& fz_b) {
+// rest-length term, the damping quotient) travel as one pair.  Every packed operation
+// rounds each lane as the scalar intrinsic would, sqrt_rcp_pair returns __fsqrt_rn /
+// __frcp_rn's bits and div_pair __fdiv_rn's, so each force is bit-identical to the scalar
+// form in fewer instructions (sm_100+ f32x2 arithmetic).
+// FAST: spring damping exactly +0; else ta1 / tb1 are the second halves of the records
+// (the neighbours' velocities; such records never carry D) and kd2 the damping.
+template <bool FAST>
+__device__ __forceinline__ void spring_pair(fp2 xxy, float xz, fp2 vxy, float vz, float4 ta, float4 ta1, float4 tb,
+                                            float4 tb1, fp2 nk, fp2 rest, fp2 kd2, fp2 eps2, float eps, fp2& f_xy_a,
+                                            float& fz_a, fp2& f_xy_b, float& fz_b) {
     const fp2 da = add2(sub2(xxy, pk2(ta.x, ta.y)), eps2), db = add2(sub2(xxy, pk2(tb.x, tb.y)), eps2);
     const float dza = __fadd_rn(__fsub_rn(xz, ta.z), eps), dzb = __fadd_rn(__fsub_rn(xz, tb.z), eps);
     const fp2 qa = mul2(da, da), qb = mul2(db, db);
@@ -169,14 +173,19 @@ __device__ __forceinline__ void spring_pair(fp2 xxy, float xz, float4 ta, float4
                       __fadd_rn(__fadd_rn(lo2(qb), hi2(qb)), __fmul_rn(dzb, dzb)));  // dot(dP, dP)
     fp2 dist, inv;
     sqrt_rcp_pair(s, dist, inv);
-    const fp2 c = mul2(nk, sub2(dist, rest));  // -k (|dP| - L0)
+    fp2 c = mul2(nk, sub2(dist, rest));  // -k (|dP| - L0)
+    if (!FAST) {
+        const fp2 ga = mul2(sub2(vxy, pk2(ta.w, ta1.x)), da), gb = mul2(sub2(vxy, pk2(tb.w, tb1.x)), db);
+        const fp2 g = pk2(__fadd_rn(__fadd_rn(lo2(ga), hi2(ga)), __fmul_rn(__fsub_rn(vz, ta1.y), dza)),
+                          __fadd_rn(__fadd_rn(lo2(gb), hi2(gb)), __fmul_rn(__fsub_rn(vz, tb1.y), dzb)));  // dot(dV, dP)
+        c = add2(c, mul2(kd2, div_pair(g, s, dist, inv)));
+    }
     const float ca = lo2(c), cb = hi2(c), ia = lo2(inv), ib = hi2(inv);
     f_xy_a = pk2(__fmul_rn(ca, __fmul_rn(lo2(da), ia)), __fmul_rn(ca, __fmul_rn(hi2(da), ia)));
     fz_a = __fmul_rn(ca, __fmul_rn(dza, ia));
     f_xy_b = pk2(__fmul_rn(cb, __fmul_rn(lo2(db), ib)), __fmul_rn(cb, __fmul_rn(hi2(db), ib)));
     fz_b = __fmul_rn(cb, __fmul_rn(dzb, ib));
 }
-
 
 // Contact data a vertex will read after its spring sum (its cached leaf, its stored
 // normal), prefetched when the vertex starts: 0 = not prefetched, 1 = into L1, 2 = L2.
@@ -206,60 +215,68 @@ struct Entries {
     __device__ __forceinline__ uint2 operator[](int e) const { return SMEM ? p[32 * e] : __ldg(p + 32 * e); }
 };
 
+// How a row is summed.  SUM_FAST: spring damping exactly +0, packed pairs; SUM_DAMPED: packed
+// pairs with damping; SUM_SCALAR: spring by spring, any record form (the general formula,
+// also with zero damping: rows that must be recomputed with the damping term).
+enum SumMode { SUM_FAST, SUM_DAMPED, SUM_SCALAR };
+
 // Sum of springs [e, end) of one list of a sliced-ELL row (ep/kp at the row's entry
 // 0, entries 32 apart), in CSR order, two at a time (independent chains).
-template <bool FAST, class Rec, class Ent>
+template <SumMode MODE, class Rec, class Ent>
 __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const float* __restrict__ kp, int e,
                                        const int end, const float nk, const bool perk, f3 x, f3 vel, float kd,
                                        f3 eps3, bool drec, float dt) {
-    f3 acc = mk3(0.0f, 0.0f, 0.0f);
-    if (FAST) {  // two springs per packed evaluation; the sum stays in CSR order
+    constexpr bool FAST = MODE == SUM_FAST;
+    if (MODE != SUM_SCALAR) {  // two springs per packed evaluation; the sum stays in CSR order
         const fp2 xxy = pk2(x.x, x.y), eps2 = splat2(eps3.x), nk2 = splat2(nk);
+        const fp2 vxy = FAST ? eps2 : pk2(vel.x, vel.y), kd2 = FAST ? eps2 : splat2(kd);  // not read with FAST
         fp2 axy = pk2(0.0f, 0.0f);
         float az = 0.0f;
         for (; e + 1 < end; e += 2) {
             const uint2 ea = ep[e], eb = ep[e + 1];
             const int ja = (int)(ea.x & END_MASK), jb = (int)(eb.x & END_MASK);
-            const float4 a0 = rec.r0(ja), b0 = rec.r0(jb);
+            f4x2 ra, rb;
+            if (FAST) {
+                ra.a = rec.r0(ja);
+                rb.a = rec.r0(jb);
+                ra.b = ra.a;
+                rb.b = rb.a;
+            } else {
+                ra = rec.both(ja);
+                rb = rec.both(jb);
+            }
             const fp2 k2 = perk ? pk2(-__ldg(kp + 32 * e), -__ldg(kp + 32 * (e + 1))) : nk2;
             fp2 fa, fb;
             float fza, fzb;
-            spring_pair(xxy, x.z, a0, b0, k2, pk2(__uint_as_float(ea.y), __uint_as_float(eb.y)), eps2, eps3.x, fa, fza,
-                        fb, fzb);
+            spring_pair<FAST>(xxy, x.z, vxy, vel.z, ra.a, ra.b, rb.a, rb.b, k2,
+                              pk2(__uint_as_float(ea.y), __uint_as_float(eb.y)), kd2, eps2, eps3.x, fa, fza, fb, fzb);
             axy = add2(add2(axy, fa), fb);
             az = __fadd_rn(__fadd_rn(az, fza), fzb);
         }
-        acc = mk3(lo2(axy), hi2(axy), az);
+        f3 acc = mk3(lo2(axy), hi2(axy), az);
         if (e < end) {
             const uint2 ea = ep[e];
-            const float4 a0 = rec.r0((int)(ea.x & END_MASK));
+            const int ja = (int)(ea.x & END_MASK);
+            const float4 a0 = rec.r0(ja);
             const float ka = perk ? -__ldg(kp + 32 * e) : nk;
-            acc = add(acc, spring_force<true>(x, vel, a0, a0, ka, __uint_as_float(ea.y), kd, eps3, drec, dt));
+            acc = add(acc, spring_force<FAST>(x, vel, a0, FAST ? a0 : rec.r1(ja), ka, __uint_as_float(ea.y), kd, eps3,
+                                              FAST && drec, dt));
         }
         return acc;
     }
-    for (; e + 1 < end; e += 2) {
-        const uint2 ea = ep[e], eb = ep[e + 1];
-        const int ja = (int)(ea.x & END_MASK), jb = (int)(eb.x & END_MASK);
-        const f4x2 ra = rec.both(ja), rb = rec.both(jb);
-        const float ka = perk ? -__ldg(kp + 32 * e) : nk;
-        const float kb = perk ? -__ldg(kp + 32 * (e + 1)) : nk;
-        const f3 fa = spring_force<FAST>(x, vel, ra.a, ra.b, ka, __uint_as_float(ea.y), kd, eps3, drec, dt);
-        const f3 fb = spring_force<FAST>(x, vel, rb.a, rb.b, kb, __uint_as_float(eb.y), kd, eps3, drec, dt);
-        acc = add(add(acc, fa), fb);
-    }
-    if (e < end) {
+    f3 acc = mk3(0.0f, 0.0f, 0.0f);
+    for (; e < end; ++e) {
         const uint2 ea = ep[e];
-        const f4x2 ra = rec.both((int)(ea.x & END_MASK));
+        const int ja = (int)(ea.x & END_MASK);
         const float ka = perk ? -__ldg(kp + 32 * e) : nk;
-        acc = add(acc, spring_force<FAST>(x, vel, ra.a, ra.b, ka, __uint_as_float(ea.y), kd, eps3, drec, dt));
+        acc = add(acc, spring_force<false>(x, vel, rec.r0(ja), rec.r1(ja), ka, __uint_as_float(ea.y), kd, eps3, drec, dt));
     }
     return acc;
 }
 
 // F + the spring forces of one vertex, list by list as the reference does
 // (force += list sum, verlet.cu:148-149); cnt holds the row's per-list counts.
-template <bool FAST, class Rec, class Ent>
+template <SumMode MODE, class Rec, class Ent>
 __device__ __forceinline__ f3 row_forces(const Rec& rec, const Ent& ep, const float* __restrict__ kp, uint2 cnt,
                                          f3 x, f3 vel, f3 F, const StepParams& P, bool perk, f3 eps3) {
     int e = 0;
@@ -267,7 +284,7 @@ __device__ __forceinline__ f3 row_forces(const Rec& rec, const Ent& ep, const fl
     for (int l = 0; l < VISG_MAX_LISTS; ++l) {
         if (l < P.n_lists) {
             const int n = (int)(((l < 2 ? cnt.x : cnt.y) >> (16 * (l & 1))) & (l == 3 ? 0x7fffu : 0xffffu));
-            F = add(F, list_sum<FAST>(rec, ep, kp, e, e + n, -P.list_k[l], perk, x, vel, P.kd, eps3, P.drec != 0,
+            F = add(F, list_sum<MODE>(rec, ep, kp, e, e + n, -P.list_k[l], perk, x, vel, P.kd, eps3, P.drec != 0,
                                       P.dt));
             e += n;
         }
@@ -392,9 +409,9 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
             // as long as RN(dv.d / |d|) is finite (guaranteed while every record is tame;
             // the wild flag says when one was not) or c is not finite (then F is not
             // finite either: such rows are recomputed with the damping term).
-            F = row_forces<true>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
+            F = row_forces<SUM_FAST>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
         } else {
-            F = row_forces<false>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
+            F = row_forces<SUM_DAMPED>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
         }
         // the record again (a second read of a line this thread has just read)
         const f4x2 own = ld8_once(a.state_in + 2 * ii);
@@ -404,7 +421,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         margin = r1.w;
         if (KD0 && (wild || !(isfinite(F.x) && isfinite(F.y) && isfinite(F.z)))) {
             vel = P.drec ? divs(rv, P.dt) : rv;
-            F = row_forces<false>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
+            F = row_forces<SUM_SCALAR>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
         }
         // x - x_old: from the record (drec), else from x_old in the other buffer
         f3 xo = x, d = rv;
