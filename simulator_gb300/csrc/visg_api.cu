@@ -170,6 +170,9 @@ struct Engine {
     uint32_t* d_fcol = nullptr;
     float* d_fnorm = nullptr;
     int64_t NF = 0;
+    // no tree rebuilt since the last step launch (steps overlap the launch before them; a
+    // replayed graph's first step does not)
+    bool settled = true;
     bool prev_ok = false;  // the other buffer holds the positions the last step started from
     int split = 1;                     // collision in its own kernel (autotuned)
     float* d_stage = nullptr;  // 10*N floats
@@ -600,6 +603,7 @@ struct Engine {
         a.wild = d_wild;
         a.twin = d_twin[bi] + t0;
         a.win_cap = win_cap[bi];
+        a.settled = settled ? 1 : 0;
         a.p = step_params();
         return a;
     }
@@ -667,6 +671,7 @@ struct Engine {
         if (n > 0) prev_ok = true;
         while (n > 0) {
             if (p.use_graph && n >= chunk_steps) {
+                settled = true;
                 if (!chunk_exec[cur]) {
                     int r = capture_chunk(cur);
                     if (r) return r;
@@ -676,6 +681,7 @@ struct Engine {
                 steps_since_check += chunk_steps;
             } else {
                 CU(launch_one(stream, cur));
+                settled = true;
                 cur ^= 1;
                 --n;
                 ++steps_since_check;
@@ -704,6 +710,7 @@ struct Engine {
         for (int k = 0; k < n && e == cudaSuccess; ++k) {
             set_step_timing(ev[0], ev[1]);
             e = launch_step(args(cur, block, 0), variant(block), block, grid, stream);
+            settled = true;
             set_step_timing(nullptr, nullptr);
             if (e == cudaSuccess) e = cudaEventRecord(ev[2], stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);
@@ -759,6 +766,7 @@ struct Engine {
         // staged first.  The build also voids the garment's query-cache margins (the
         // body moves)
         adj.rec_seg = -1;  // a backward pass replays every segment over the body as it is then
+        settled = false;
         const bool dev = kind == cudaMemcpyDeviceToDevice;
         if (!dev) {
             CU(cudaMemcpyAsync(bvh[g].xyz_in, xyz, (size_t)bvh[g].nv * 12, kind, stream));

@@ -194,6 +194,7 @@ struct StepArgs {
     uint32_t* wild;           // sticky: some record had |x| or |v| >= 1e15 (or NaN)
     const int2* twin;         // per tile sliced-ELL block, with SV_STAGED
     int win_cap;              // entries per shared-memory stage buffer
+    int settled;              // the bodies' trees were complete before the launch before this one began
     StepParams p;
 };
 
