@@ -207,6 +207,7 @@ enum StepVariant : int {
     SV_SPLIT = 32,    // collision in its own kernel over a compacted candidate list
     SV_STAGED = 64,   // sliced-ELL blocks staged in shared memory by TMA bulk copies
     SV_HELP = 128,    // helper warps answer the queries at the start positions beside the spring sums
+    SV_OVERLAP = 256, // a launch may begin while the one before it runs (fused collision)
 };
 constexpr int kHelpBlockMax = 256;  // tile sizes up to which there are kernels with helper warps
 // dynamic shared memory of a launch: two stage buffers of win_cap entries + barriers

@@ -693,8 +693,6 @@ __global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK)
             vertex_step<COLL, KD0, SPLIT, false, false>(a, __ldg(&a.tiles[tile]), a.sell, 0u, refv, check, perk, wild,
                                                         help, my_disp, my_bad);
     } else {
-        wait_for_earlier_launches();
-        const bool wild = *reinterpret_cast<const volatile uint32_t*>(a.wild) != 0u;
         // two-buffer ring: full[b] completes when buffer b holds its tile's block,
         // empty[b] when every warp is done reading it
         const uint32_t full = smem_addr(dyn_smem), empty = full + 16u;
@@ -711,6 +709,8 @@ __global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK)
         }
         __syncthreads();
         if (threadIdx.x == 0 && (int)blockIdx.x < a.n_tiles) stage_entries(a, blockIdx.x, buf0, full);
+        wait_for_earlier_launches();  // the springs do not change, so the first are on their way
+        const bool wild = *reinterpret_cast<const volatile uint32_t*>(a.wild) != 0u;
         int it = 0;
         for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++it) {
             const int b = it & 1;
@@ -850,7 +850,10 @@ cudaError_t allow_smem(const void* fn, int bytes) {
 // (wait_for_earlier_launches).  For the short kernels of small simulations, where a launch's
 // own latency is a fifth of a step: dragged 64 x 64 sheet 29.1 -> 22.0 us a frame, body moved
 // before each of 4 steps 165 -> 154; with the queries begun before the wait, 200 steps of a
-// 64 x 64 sheet in contact 1,677 -> 1,358 us, 20 of a 131 x 127 mesh 269 -> 229.
+// 64 x 64 sheet in contact 1,677 -> 1,358 us, 20 of a 131 x 127 mesh 269 -> 229.  Large
+// simulations in one chain of fused steps (SV_OVERLAP) gain the gaps between launches and
+// the first tile's copy: 512 x 512 sheet 437 -> 430 us in 4 steps with as many rebuilds, 123 -> 114 in
+// 4 steps with the output stage.
 template <class... P, class... A>
 cudaError_t launch_after(void (*fn)(P...), int grid, int block, int smem, cudaStream_t s, bool overlap, A... args) {
     cudaLaunchConfig_t c = {};
@@ -884,7 +887,9 @@ cudaError_t launch_block(const StepArgs& a, int variant, int grid, cudaStream_t 
         if (e != cudaSuccess) return e;
     }
     if (t_before_step) cudaEventRecord(t_before_step, s);
-    e = launch_after(fn, grid, help ? 2 * BLOCK : BLOCK, smem, s, help, a, (variant & SV_REFV) ? 1 : 0,
+    // queued collision keeps stream order: a memset comes before the step, the queue's kernel after it
+    const bool overlap = help || ((variant & SV_OVERLAP) && !split);
+    e = launch_after(fn, grid, help ? 2 * BLOCK : BLOCK, smem, s, overlap, a, (variant & SV_REFV) ? 1 : 0,
                      (variant & SV_CHECK) ? 1 : 0, (variant & SV_PERK) ? 1 : 0);
     if (e != cudaSuccess) return e;
     if (t_after_step) cudaEventRecord(t_after_step, s);
