@@ -410,7 +410,7 @@ struct Engine {
                     return fail(VISG_ERR_UNSUPPORTED, "more than 65535 springs of one list at one vertex");
                 h_vcount[v] = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16) | (h_rowp[v] & PIN_BIT));
                 for (uint32_t k = 0; k < n; ++k) {
-                    sell[soff[s] + 32 * (int64_t)k + lane] = ent[rp + k];
+                    sell[soff[s] + 32 * (int64_t)k + lane] = make_uint2(ent[rp + k].x & END_MASK, ent[rp + k].y);
                     if (perk) sellk[soff[s] + 32 * (int64_t)k + lane] = kk[rp + k];
                 }
             }

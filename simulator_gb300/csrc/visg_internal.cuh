@@ -16,7 +16,7 @@
 //   rowp:   u32 per vertex + 1, merged CSR row offsets; bit 31 = vertex pinned
 //   ent:    uint2 per directed spring {end | list << 30, rest}         8 B
 //   kent:   f32 per directed spring, only with per-spring stiffness
-//   sell:   the same springs in sliced-ELL order for the step kernel: a slice is 32
+//   sell:   the same springs {end, rest} in sliced-ELL order for the step kernel: a slice is 32
 //           consecutive vertices of one garment, padded to its longest row; entry k of
 //           lane l of slice s sits at slice_off[s] + 32 k + l, so the k-th springs of a
 //           warp are one contiguous 256-byte run (sellk: stiffness, same layout)
@@ -191,7 +191,7 @@ struct StepArgs {
     const float* sellk;       // per-entry stiffness in the same layout, with SV_PERK
     const uint32_t* slice_off;
     const uint2* vcount;      // per vertex: springs per list, 16 bits each (list 3: 15), bit 63 = pinned
-    uint32_t* wild;           // sticky: some record had |x| or |v| >= 1e15 (or NaN)
+    uint32_t* wild;           // sticky: some record had |x| >= 3e14 or |v| >= 1e15 (or NaN)
     const int2* twin;         // per tile sliced-ELL block, with SV_STAGED
     int win_cap;              // entries per shared-memory stage buffer
     int settled;              // the bodies' trees were complete before the launch before this one began
@@ -254,7 +254,7 @@ cudaError_t launch_count_contacts(const float4* state, int64_t n, unsigned long 
 cudaError_t launch_set_vertices(float4* state, const uint32_t* idx, const float* xyz, int n, float dt, uint32_t* wild,
                                 cudaStream_t s);
 
-// set *wild when some record of [0, n) has a component of |x| or |v| >= 1e15 (or NaN)
+// set *wild when some record of [0, n) has a component of |x| >= 3e14 or |v| >= 1e15 (or NaN)
 cudaError_t launch_check_tame(const float4* state, int64_t n, uint32_t* wild, cudaStream_t s);
 
 // ---- adjoint ----------------------------------------------------------------------------

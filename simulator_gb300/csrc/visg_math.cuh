@@ -96,15 +96,16 @@ __device__ __forceinline__ float hi2(fp2 v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
     return b;
 }
+// Not for a sum with a packed product: the assembler contracts mul.f32x2 and add.f32x2 into
+// one FMA in spite of their .rn (seen against the scalar intrinsics).  Sums of products take
+// scalar additions of the product's lanes, which it leaves alone (add_lanes).
 __device__ __forceinline__ fp2 add2(fp2 a, fp2 b) {
     fp2 r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ fp2 sub2(fp2 a, fp2 b) {
-    fp2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
+__device__ __forceinline__ fp2 add_lanes(fp2 a, fp2 b) {
+    return pk2(__fadd_rn(lo2(a), lo2(b)), __fadd_rn(hi2(a), hi2(b)));
 }
 __device__ __forceinline__ fp2 mul2(fp2 a, fp2 b) {
     fp2 r;
@@ -119,8 +120,8 @@ __device__ __forceinline__ fp2 fma2(fp2 a, fp2 b, fp2 c) {  // a * b + c, one ro
 __device__ __forceinline__ fp2 splat2(float v) { return pk2(v, v); }
 
 // ---- correctly rounded square root and reciprocal, two lanes at once -------------------
-// For s in [2^-100, 2^100):  q = RN(sqrt(s))  and  r = RN(1 / q), bit for bit what
-// __fsqrt_rn(s) and __frcp_rn(__fsqrt_rn(s)) return (checked against them on every
+// For s in [2^-100, 2^100):  q = RN(sqrt(s))  and  nr = -RN(1 / q), bit for bit what
+// __fsqrt_rn(s) and -__frcp_rn(__fsqrt_rn(s)) return (checked against them on every
 // float of that range by visg_selftest_exact_math).  Method: Markstein's correction
 // of a hardware approximation by one Newton step whose residual an FMA forms with a
 // single rounding (P. W. Markstein, "Computation of elementary functions on the IBM RISC
@@ -129,11 +130,12 @@ __device__ __forceinline__ fp2 splat2(float v) { return pk2(v, v); }
 // Itanium-based Systems", Intel Press, 2002, ch. 8):
 //   y ~ 1/sqrt(s) (rsqrt.approx), g = s y, h = y/2;  d = s - g^2 (one FMA);  q = g + d h.
 //   z ~ 1/q (rcp.approx);  e = 1 - q z (one FMA);  r = z + z e.
-// Lanes outside the range take the intrinsics.  (Below 2^-100 the remainder s - g^2
-// can fall among the subnormals and lose the bits the last correction needs.)
+// The reciprocal comes negated because rcp.approx takes -q at no cost and the packed FMA,
+// which has no negated operands, then needs no extra product for the residuals.
+// The caller sees to the range (spring_sum_exact): below 2^-100 the remainder s - g^2 can
+// fall among the subnormals and lose the bits the last correction needs.
 constexpr uint32_t kExactLo = 27u << 23;                     // 2^-100
 constexpr uint32_t kExactSpan = (227u << 23) - (27u << 23);  // up to 2^100
-__device__ __forceinline__ bool exact_fast_domain(float s) { return __float_as_uint(s) - kExactLo < kExactSpan; }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
@@ -146,46 +148,32 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return y;
 }
 
-__device__ __forceinline__ void sqrt_rcp_pair(fp2 s, fp2& q, fp2& r) {
-    const float sa = lo2(s), sb = hi2(s);
-    if (exact_fast_domain(sa) && exact_fast_domain(sb)) {
-        const fp2 y = pk2(rsqrt_approx(sa), rsqrt_approx(sb));
-        const fp2 nh = mul2(y, splat2(-0.5f));  // -h
-        const fp2 g = mul2(s, y);
-        const fp2 dn = fma2(g, g, mul2(s, splat2(-1.0f)));  // g^2 - s
-        q = fma2(dn, nh, g);                                // g + (s - g^2) h
-        const fp2 nq = mul2(q, splat2(-1.0f));
-        fp2 z = pk2(rcp_approx(lo2(q)), rcp_approx(hi2(q)));
-        const fp2 e = fma2(nq, z, splat2(1.0f));
-        r = fma2(z, e, z);
-    } else {
-        const float qa = __fsqrt_rn(sa), qb = __fsqrt_rn(sb);
-        q = pk2(qa, qb);
-        r = pk2(__frcp_rn(qa), __frcp_rn(qb));
-    }
+__device__ __forceinline__ void sqrt_rcp_pair(fp2 s, fp2& q, fp2& nr) {
+    const fp2 y = pk2(rsqrt_approx(lo2(s)), rsqrt_approx(hi2(s)));
+    const fp2 nh = mul2(y, splat2(-0.5f));  // -h
+    const fp2 g = mul2(s, y);
+    const fp2 dn = fma2(g, g, mul2(s, splat2(-1.0f)));  // g^2 - s
+    q = fma2(dn, nh, g);                                // g + (s - g^2) h
+    const fp2 nz = pk2(rcp_approx(-lo2(q)), rcp_approx(-hi2(q)));
+    const fp2 e = fma2(q, nz, splat2(1.0f));
+    nr = fma2(nz, e, nz);
 }
 
-// g / q in both lanes, rounded as __fdiv_rn rounds, given r = RN(1 / q) and q as
+// -g / q in both lanes, rounded as __fdiv_rn rounds, given q and nr = -RN(1 / q) as
 // sqrt_rcp_pair returns them: two corrections of g r by an FMA's exact residual (the same
 // sources).  The first brings the quotient within one unit in the last place of g / q,
 // from where, with r correctly rounded, the second is correctly rounded (Markstein's
-// theorem; 6.9e10 pairs, over every significand of q, showed no other result).  Lanes whose
-// residual could underflow or overflow take the division.  A zero numerator gives a zero,
-// of either sign.  64 x 64 damped sheet: step kernel 7.4 -> 6.1 us.
-constexpr uint32_t kDivLo = (127u - 60u) << 23, kDivSpan = 120u << 23;  // |g| in [2^-60, 2^60)
-__device__ __forceinline__ bool div_fast_domain(float g) {
-    const uint32_t u = __float_as_uint(g) & 0x7fffffffu;
-    return u - kDivLo < kDivSpan || u == 0u;
+// theorem; 6.9e10 pairs, over every significand of q, showed no other result).  The caller
+// sees to it that |g| >= 2^-60 or g = 0, so that no residual underflows, and that the
+// quotient does not overflow.  A zero numerator gives a zero, of either sign.
+__device__ __forceinline__ fp2 div_pair(fp2 g, fp2 q, fp2 nr) {
+    fp2 nd = mul2(g, nr);
+    nd = fma2(fma2(q, nd, g), nr, nd);
+    return fma2(fma2(q, nd, g), nr, nd);
 }
-__device__ __forceinline__ fp2 div_pair(fp2 g, fp2 s, fp2 q, fp2 r) {  // s: q^2 before rounding
-    if (exact_fast_domain(lo2(s)) && exact_fast_domain(hi2(s)) && div_fast_domain(lo2(g)) && div_fast_domain(hi2(g))) {
-        const fp2 nq = mul2(q, splat2(-1.0f));
-        fp2 d = mul2(g, r);
-        d = fma2(fma2(nq, d, g), r, d);
-        return fma2(fma2(nq, d, g), r, d);
-    }
-    return pk2(__fdiv_rn(lo2(g), lo2(q)), __fdiv_rn(hi2(g), hi2(q)));
-}
+constexpr uint32_t kDivLo = (127u - 60u) << 23;  // 2^-60
+// orders |g| as a uint32 with the sign gone and zero last
+__device__ __forceinline__ uint32_t div_order(float g) { return 2u * __float_as_uint(g) - 1u; }
 
 // Order-preserving map float -> uint32 (for atomicMin/atomicMax on floats).
 __device__ __forceinline__ uint32_t f2ord(float f) {

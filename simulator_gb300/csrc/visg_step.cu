@@ -135,56 +135,65 @@ __device__ __forceinline__ int query_margin(const BvhRoot* rt, f3 p, int* err, f
 //   c = -k (|d| - L0) + kd (dv.d) / |d|,  force = c * normalize(d),  d = x - x_j + FLT_EPSILON
 // t0/t1 is the neighbour's record: position and velocity (p2 - p2_old) / dt, stored
 // once per step by the neighbour's own thread with the same IEEE division; nk = -k.
-// FAST drops the damping term, for spring damping exactly +0: see row_forces.
 // With drec the neighbour's record holds D = p2 - p2_old; its velocity is D / dt.
-template <bool FAST>
-__device__ __forceinline__ f3 spring_force(f3 x, f3 vel, float4 t0, float4 t1, float nk, float rest, float kd,
-                                           f3 eps3, bool drec, float dt) {
+__device__ __forceinline__ f3 spring_force(f3 x, f3 vel, float4 t0, float4 t1, float nk, float rest, float kd, f3 eps3,
+                                           bool drec, float dt) {
     const f3 dP = add(sub(x, mk3(t0.x, t0.y, t0.z)), eps3);
     const float dist = __fsqrt_rn(dot(dP, dP));
-    float c = __fmul_rn(nk, __fsub_rn(dist, rest));
-    if (!FAST) {
-        f3 v2 = mk3(t0.w, t1.x, t1.y);
-        if (drec) v2 = divs(v2, dt);
-        const f3 dV = sub(vel, v2);
-        c = __fadd_rn(c, __fmul_rn(kd, __fdiv_rn(dot(dV, dP), dist)));
-    }
+    f3 v2 = mk3(t0.w, t1.x, t1.y);
+    if (drec) v2 = divs(v2, dt);
+    const f3 dV = sub(vel, v2);
+    const float c = __fadd_rn(__fmul_rn(nk, __fsub_rn(dist, rest)), __fmul_rn(kd, __fdiv_rn(dot(dV, dP), dist)));
     return mul(c, mul(dP, __frcp_rn(dist)));  // normalize(dP) = dP * (1 / |dP|)
 }
 
+// Which springs of a row the packed evaluation may not answer for: the least |dP|^2 and
+// damping numerator seen.  While every record is tame the upper ends of their ranges hold by
+// themselves (tame), so one minimum a pair of springs stands in for a test and a branch each.
+struct PairRange {
+    float s = 1.0f;
+    uint32_t g = 0xffffffffu;
+    __device__ __forceinline__ bool exact() const {
+        return __float_as_uint(s) >= kExactLo && g >= 2u * kDivLo - 1u;
+    }
+};
+
 // Two springs of one vertex at once (spring_force on each spring, operation for
-// operation).  The x and y components of a spring's
-// vectors travel as one packed pair (a record's x, y are adjacent words), z alone;
-// the two springs' scalar chains (|dP|^2, the square root and its reciprocal, the
-// rest-length term, the damping quotient) travel as one pair.  Every packed operation
-// rounds each lane as the scalar intrinsic would, sqrt_rcp_pair returns __fsqrt_rn /
-// __frcp_rn's bits and div_pair __fdiv_rn's, so each force is bit-identical to the scalar
-// form in fewer instructions (sm_100+ f32x2 arithmetic).
+// operation): every quantity of theirs is a packed pair, one spring a lane.  The first
+// operation of a spring is a subtraction from x, which writes its result into the pair, so
+// packing costs no moves.  Every packed operation rounds each lane as the scalar intrinsic
+// would, sqrt_rcp_pair returns __fsqrt_rn / __frcp_rn's bits and div_pair __fdiv_rn's within
+// their ranges (rg), so each force is bit-identical to the scalar form in fewer instructions
+// (sm_100+ f32x2 arithmetic).  Both c and 1 / |dP| are formed negated, which changes no bit
+// of their product but a zero's sign in c, and such a zero adds nothing to the sum.
+// Against x and y of one spring in a pair, z apart and a range test with a branch per pair:
+// 200 steps of a 64 x 64 sheet 1,376 -> 1,326 us, 512 x 512 sheet 114 -> 110 in 4 steps with
+// the output stage; batches (bound by the gathers' latency) unchanged.
 // FAST: spring damping exactly +0; else ta1 / tb1 are the second halves of the records
 // (the neighbours' velocities; such records never carry D) and kd2 the damping.
 template <bool FAST>
-__device__ __forceinline__ void spring_pair(fp2 xxy, float xz, fp2 vxy, float vz, float4 ta, float4 ta1, float4 tb,
-                                            float4 tb1, fp2 nk, fp2 rest, fp2 kd2, fp2 eps2, float eps, fp2& f_xy_a,
-                                            float& fz_a, fp2& f_xy_b, float& fz_b) {
-    const fp2 da = add2(sub2(xxy, pk2(ta.x, ta.y)), eps2), db = add2(sub2(xxy, pk2(tb.x, tb.y)), eps2);
-    const float dza = __fadd_rn(__fsub_rn(xz, ta.z), eps), dzb = __fadd_rn(__fsub_rn(xz, tb.z), eps);
-    const fp2 qa = mul2(da, da), qb = mul2(db, db);
-    const fp2 s = pk2(__fadd_rn(__fadd_rn(lo2(qa), hi2(qa)), __fmul_rn(dza, dza)),
-                      __fadd_rn(__fadd_rn(lo2(qb), hi2(qb)), __fmul_rn(dzb, dzb)));  // dot(dP, dP)
-    fp2 dist, inv;
-    sqrt_rcp_pair(s, dist, inv);
-    fp2 c = mul2(nk, sub2(dist, rest));  // -k (|dP| - L0)
+__device__ __forceinline__ void spring_pair(f3 x, f3 vel, float4 ta, float4 ta1, float4 tb, float4 tb1, fp2 k2,
+                                            float rest_a, float rest_b, fp2 kd2, fp2 eps2, fp2& fx, fp2& fy, fp2& fz,
+                                            PairRange& rg) {
+    const fp2 dx = add2(pk2(__fsub_rn(x.x, ta.x), __fsub_rn(x.x, tb.x)), eps2);
+    const fp2 dy = add2(pk2(__fsub_rn(x.y, ta.y), __fsub_rn(x.y, tb.y)), eps2);
+    const fp2 dz = add2(pk2(__fsub_rn(x.z, ta.z), __fsub_rn(x.z, tb.z)), eps2);
+    const fp2 s = add_lanes(add_lanes(mul2(dx, dx), mul2(dy, dy)), mul2(dz, dz));  // dot(dP, dP)
+    rg.s = fminf(fminf(rg.s, lo2(s)), hi2(s));
+    fp2 dist, ninv;
+    sqrt_rcp_pair(s, dist, ninv);
+    fp2 nc = mul2(k2, pk2(__fsub_rn(lo2(dist), rest_a), __fsub_rn(hi2(dist), rest_b)));  // k (|dP| - L0)
     if (!FAST) {
-        const fp2 ga = mul2(sub2(vxy, pk2(ta.w, ta1.x)), da), gb = mul2(sub2(vxy, pk2(tb.w, tb1.x)), db);
-        const fp2 g = pk2(__fadd_rn(__fadd_rn(lo2(ga), hi2(ga)), __fmul_rn(__fsub_rn(vz, ta1.y), dza)),
-                          __fadd_rn(__fadd_rn(lo2(gb), hi2(gb)), __fmul_rn(__fsub_rn(vz, tb1.y), dzb)));  // dot(dV, dP)
-        c = add2(c, mul2(kd2, div_pair(g, s, dist, inv)));
+        const fp2 gx = mul2(pk2(__fsub_rn(vel.x, ta.w), __fsub_rn(vel.x, tb.w)), dx);
+        const fp2 gy = mul2(pk2(__fsub_rn(vel.y, ta1.x), __fsub_rn(vel.y, tb1.x)), dy);
+        const fp2 gz = mul2(pk2(__fsub_rn(vel.z, ta1.y), __fsub_rn(vel.z, tb1.y)), dz);
+        const fp2 g = add_lanes(add_lanes(gx, gy), gz);  // dot(dV, dP)
+        rg.g = min(min(rg.g, div_order(lo2(g))), div_order(hi2(g)));
+        nc = add_lanes(nc, mul2(kd2, div_pair(g, dist, ninv)));
     }
-    const float ca = lo2(c), cb = hi2(c), ia = lo2(inv), ib = hi2(inv);
-    f_xy_a = pk2(__fmul_rn(ca, __fmul_rn(lo2(da), ia)), __fmul_rn(ca, __fmul_rn(hi2(da), ia)));
-    fz_a = __fmul_rn(ca, __fmul_rn(dza, ia));
-    f_xy_b = pk2(__fmul_rn(cb, __fmul_rn(lo2(db), ib)), __fmul_rn(cb, __fmul_rn(hi2(db), ib)));
-    fz_b = __fmul_rn(cb, __fmul_rn(dzb, ib));
+    fx = mul2(nc, mul2(dx, ninv));
+    fy = mul2(nc, mul2(dy, ninv));
+    fz = mul2(nc, mul2(dz, ninv));
 }
 
 // Contact data a vertex will read after its spring sum (its cached leaf, its stored
@@ -230,55 +239,48 @@ enum SumMode { SUM_FAST, SUM_DAMPED, SUM_SCALAR };
 
 // Sum of springs [e, end) of one list of a sliced-ELL row (ep/kp at the row's entry
 // 0, entries 32 apart), in CSR order, two at a time (independent chains).
-template <SumMode MODE, int UNROLL, class Rec, class Ent>
+template <SumMode MODE, int UNROLL, bool PERK, class Rec, class Ent>
 __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const float* __restrict__ kp, int e,
-                                       const int end, const float nk, const bool perk, f3 x, f3 vel, float kd,
-                                       f3 eps3, bool drec, float dt) {
+                                       const int end, const float k, f3 x, f3 vel, float kd, f3 eps3, bool drec,
+                                       float dt, PairRange& rg) {
     constexpr bool FAST = MODE == SUM_FAST;
+    f3 acc = mk3(0.0f, 0.0f, 0.0f);
     if (MODE != SUM_SCALAR) {  // two springs per packed evaluation; the sum stays in CSR order
-        const fp2 xxy = pk2(x.x, x.y), eps2 = splat2(eps3.x), nk2 = splat2(nk);
-        const fp2 vxy = FAST ? eps2 : pk2(vel.x, vel.y), kd2 = FAST ? eps2 : splat2(kd);  // not read with FAST
-        fp2 axy = pk2(0.0f, 0.0f);
-        float az = 0.0f;
-#pragma unroll UNROLL
-        for (; e + 1 < end; e += 2) {
-            const uint2 ea = ep[e], eb = ep[e + 1];
-            const int ja = (int)(ea.x & END_MASK), jb = (int)(eb.x & END_MASK);
+        const fp2 eps2 = splat2(eps3.x), k2 = splat2(k), kd2 = FAST ? eps2 : splat2(kd);  // kd2 not read with FAST
+        auto pair = [&](int ea_at, int eb_at, fp2& fx, fp2& fy, fp2& fz) {
+            const uint2 ea = ep[ea_at], eb = ep[eb_at];
             f4x2 ra, rb;
             if (FAST) {
-                ra.a = rec.r0(ja);
-                rb.a = rec.r0(jb);
+                ra.a = rec.r0((int)ea.x);
+                rb.a = rec.r0((int)eb.x);
                 ra.b = ra.a;
                 rb.b = rb.a;
             } else {
-                ra = rec.both(ja);
-                rb = rec.both(jb);
+                ra = rec.both((int)ea.x);
+                rb = rec.both((int)eb.x);
             }
-            const fp2 k2 = perk ? pk2(-__ldg(kp + 32 * e), -__ldg(kp + 32 * (e + 1))) : nk2;
-            fp2 fa, fb;
-            float fza, fzb;
-            spring_pair<FAST>(xxy, x.z, vxy, vel.z, ra.a, ra.b, rb.a, rb.b, k2,
-                              pk2(__uint_as_float(ea.y), __uint_as_float(eb.y)), kd2, eps2, eps3.x, fa, fza, fb, fzb);
-            axy = add2(add2(axy, fa), fb);
-            az = __fadd_rn(__fadd_rn(az, fza), fzb);
+            const fp2 kk = PERK ? pk2(__ldg(kp + 32 * ea_at), __ldg(kp + 32 * eb_at)) : k2;
+            spring_pair<FAST>(x, vel, ra.a, ra.b, rb.a, rb.b, kk, __uint_as_float(ea.y), __uint_as_float(eb.y), kd2,
+                              eps2, fx, fy, fz, rg);
+        };
+        fp2 fx, fy, fz;
+#pragma unroll UNROLL
+        for (; e + 1 < end; e += 2) {
+            pair(e, e + 1, fx, fy, fz);
+            acc = mk3(__fadd_rn(__fadd_rn(acc.x, lo2(fx)), hi2(fx)), __fadd_rn(__fadd_rn(acc.y, lo2(fy)), hi2(fy)),
+                      __fadd_rn(__fadd_rn(acc.z, lo2(fz)), hi2(fz)));
         }
-        f3 acc = mk3(lo2(axy), hi2(axy), az);
-        if (e < end) {
-            const uint2 ea = ep[e];
-            const int ja = (int)(ea.x & END_MASK);
-            const float4 a0 = rec.r0(ja);
-            const float ka = perk ? -__ldg(kp + 32 * e) : nk;
-            acc = add(acc, spring_force<FAST>(x, vel, a0, FAST ? a0 : rec.r1(ja), ka, __uint_as_float(ea.y), kd, eps3,
-                                              FAST && drec, dt));
+        if (e < end) {  // the last of an odd number, in both lanes
+            pair(e, e, fx, fy, fz);
+            acc = mk3(__fadd_rn(acc.x, lo2(fx)), __fadd_rn(acc.y, lo2(fy)), __fadd_rn(acc.z, lo2(fz)));
         }
         return acc;
     }
-    f3 acc = mk3(0.0f, 0.0f, 0.0f);
     for (; e < end; ++e) {
         const uint2 ea = ep[e];
-        const int ja = (int)(ea.x & END_MASK);
-        const float ka = perk ? -__ldg(kp + 32 * e) : nk;
-        acc = add(acc, spring_force<false>(x, vel, rec.r0(ja), rec.r1(ja), ka, __uint_as_float(ea.y), kd, eps3, drec, dt));
+        const int ja = (int)ea.x;
+        const float nk = PERK ? -__ldg(kp + 32 * e) : -k;
+        acc = add(acc, spring_force(x, vel, rec.r0(ja), rec.r1(ja), nk, __uint_as_float(ea.y), kd, eps3, drec, dt));
     }
     return acc;
 }
@@ -287,34 +289,41 @@ __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const floa
 // (force += list sum, verlet.cu:148-149); cnt holds the row's per-list counts.
 // UNROLL pairs are in flight: 1 where many warps hide the gathers (more registers would
 // cost warps), 2 where there are few.
-template <SumMode MODE, int UNROLL, class Rec, class Ent>
-__device__ __forceinline__ f3 row_forces(const Rec& rec, const Ent& ep, const float* __restrict__ kp, uint2 cnt,
-                                         f3 x, f3 vel, f3 F, const StepParams& P, bool perk, f3 eps3) {
+template <SumMode MODE, int UNROLL, bool PERK, class Rec, class Ent>
+__device__ __forceinline__ f3 row_lists(const Rec& rec, const Ent& ep, const float* __restrict__ kp, uint2 cnt, f3 x,
+                                        f3 vel, f3 F, const StepParams& P, f3 eps3, PairRange& rg) {
     int e = 0;
 #pragma unroll
     for (int l = 0; l < VISG_MAX_LISTS; ++l) {
         if (l < P.n_lists) {
             const int n = (int)(((l < 2 ? cnt.x : cnt.y) >> (16 * (l & 1))) & (l == 3 ? 0x7fffu : 0xffffu));
-            F = add(F, list_sum<MODE, UNROLL>(rec, ep, kp, e, e + n, -P.list_k[l], perk, x, vel, P.kd, eps3, P.drec != 0,
-                                      P.dt));
+            F = add(F, list_sum<MODE, UNROLL, PERK>(rec, ep, kp, e, e + n, P.list_k[l], x, vel, P.kd, eps3, P.drec != 0,
+                                                    P.dt, rg));
             e += n;
         }
     }
     return F;
 }
+template <SumMode MODE, int UNROLL, class Rec, class Ent>
+__device__ __forceinline__ f3 row_forces(const Rec& rec, const Ent& ep, const float* __restrict__ kp, uint2 cnt, f3 x,
+                                         f3 vel, f3 F, const StepParams& P, bool perk, f3 eps3, PairRange& rg) {
+    return perk ? row_lists<MODE, UNROLL, true>(rec, ep, kp, cnt, x, vel, F, P, eps3, rg)
+                : row_lists<MODE, UNROLL, false>(rec, ep, kp, cnt, x, vel, F, P, eps3, rg);
+}
 
-// |x| < 1e15 and |v| < 1e15 in every component (false for NaN): while every record
-// satisfies this, RN(dv.d / |d|) is finite for every spring (|dv.d| < 3 (2e15)^2,
-// |d| within a factor ~2 of max |d_i| unless it underflows to 0).
+// |x| < 3e14 and |v| < 1e15 in every component (false for NaN): while every record
+// satisfies this, |dP|^2 < 12 (3e14)^2 < 2^100 and |dv.d| < 3 (2e15)^2 for every spring, and
+// RN(dv.d / |d|) is finite (|d| within a factor ~2 of max |d_i| unless it underflows to 0).
+constexpr float kTameX = 3e14f;
 __device__ __forceinline__ bool tame(f3 x, f3 v) {
     const float m = 1e15f;
-    return fabsf(x.x) < m && fabsf(x.y) < m && fabsf(x.z) < m && fabsf(v.x) < m && fabsf(v.y) < m && fabsf(v.z) < m;
+    return fabsf(x.x) < kTameX && fabsf(x.y) < kTameX && fabsf(x.z) < kTameX && fabsf(v.x) < m && fabsf(v.y) < m &&
+           fabsf(v.z) < m;
 }
 // the same for a record that carries D = x - x_old (dmax = 0.5e15 dt, so |D / dt| < 1e15)
 __device__ __forceinline__ bool tame_d(f3 x, f3 d, float dmax) {
-    const float m = 1e15f;
-    return fabsf(x.x) < m && fabsf(x.y) < m && fabsf(x.z) < m && fabsf(d.x) < dmax && fabsf(d.y) < dmax &&
-           fabsf(d.z) < dmax;
+    return fabsf(x.x) < kTameX && fabsf(x.y) < kTameX && fabsf(x.z) < kTameX && fabsf(d.x) < dmax &&
+           fabsf(d.y) < dmax && fabsf(d.z) < dmax;
 }
 
 // Helper warps (SV_HELP).  A first-hit walk is 10 to 40 dependent node loads of about 0.2 us
@@ -443,6 +452,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         const Entries<SMEM_ENT> ep{ebase + (sb - e0)};
         const float* kp = perk ? a.sellk + sb : nullptr;
         f3 F;
+        PairRange rg;
         if (KD0) {
             // Spring damping is +0: the reference adds +0 * RN(dv.d / |d|) to every c.
             // Without it c differs at most in the sign of a zero, which changes no sum
@@ -450,9 +460,9 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
             // as long as RN(dv.d / |d|) is finite (guaranteed while every record is tame;
             // the wild flag says when one was not) or c is not finite (then F is not
             // finite either: such rows are recomputed with the damping term).
-            F = row_forces<SUM_FAST, kPairs>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
+            F = row_forces<SUM_FAST, kPairs>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3, rg);
         } else {
-            F = row_forces<SUM_DAMPED, kPairs>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
+            F = row_forces<SUM_DAMPED, kPairs>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3, rg);
         }
         // the record again (a second read of a line this thread has just read)
         const f4x2 own = ld8(a.state_in + 2 * ii);
@@ -460,9 +470,10 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         const f3 rv = mk3(r0.w, r1.x, r1.y);  // v, or D = x - x_old with drec
         flags = __float_as_uint(r1.z);
         margin = r1.w;
-        if (KD0 && (wild || !(isfinite(F.x) && isfinite(F.y) && isfinite(F.z)))) {
+        // what the packed evaluation does not answer for, spring by spring
+        if (wild || !rg.exact() || !(isfinite(F.x) && isfinite(F.y) && isfinite(F.z))) {
             vel = P.drec ? divs(rv, P.dt) : rv;
-            F = row_forces<SUM_SCALAR, 1>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3);
+            F = row_forces<SUM_SCALAR, 1>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3, rg);
         }
         // x - x_old: from the record (drec), else from x_old in the other buffer
         f3 xo = x, d = rv;
@@ -1064,12 +1075,12 @@ __global__ void k_selftest_exact_math(unsigned long long* cnt) {
         const uint32_t b = (uint32_t)u;
         const uint32_t b2 = (b & 0xffff0000u) | (__brev(b) >> 16);  // same exponent, other mantissa
         const float sa = __uint_as_float(b), sb = __uint_as_float(b2);
-        fp2 q, r;
-        sqrt_rcp_pair(pk2(sa, sb), q, r);
+        fp2 q, nr;
+        sqrt_rcp_pair(pk2(sa, sb), q, nr);
         const float qa = __fsqrt_rn(sa), qb = __fsqrt_rn(sb);
         bad_q += (__float_as_uint(lo2(q)) != __float_as_uint(qa)) + (__float_as_uint(hi2(q)) != __float_as_uint(qb));
-        bad_r += (__float_as_uint(lo2(r)) != __float_as_uint(__frcp_rn(qa))) +
-                 (__float_as_uint(hi2(r)) != __float_as_uint(__frcp_rn(qb)));
+        bad_r += (__float_as_uint(-lo2(nr)) != __float_as_uint(__frcp_rn(qa))) +
+                 (__float_as_uint(-hi2(nr)) != __float_as_uint(__frcp_rn(qb)));
         n += 2;
     }
     atomicAdd(&cnt[0], n);
