@@ -1196,6 +1196,8 @@ struct Engine {
             return cuda_fail(e, "autotune backup");
         }
         const int cur0 = cur;
+        const bool prev_ok0 = prev_ok;
+        const int64_t since_check0 = steps_since_check;
         e = cudaMemcpyAsync(bs, d_state[cur], 2 * (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice, stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(bs + 2 * N, d_state[cur ^ 1], 2 * (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice,
@@ -1218,8 +1220,11 @@ struct Engine {
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
-        float best = 1e30f;
-        int best_block = block, best_grid = grid, best_ctas = 0, best_split = split, best_stage = stage;
+        struct Shape {
+            float ms;
+            int block, grid, ctas, split, stage;
+        };
+        std::vector<Shape> shapes;
         const int split0 = split, stage0 = stage;
         const int n_split = (p.collide && any_body) ? 2 : 1;
         for (int sv = 0; sv < 2 * n_split * kNumBlocks && e == cudaSuccess; ++sv) {
@@ -1253,64 +1258,81 @@ struct Engine {
                 if (e == cudaSuccess) e = cudaEventSynchronize(e1);
                 float ms = 0;
                 cudaEventElapsedTime(&ms, e0, e1);
-                if (e == cudaSuccess && ms < best) {
-                    best = ms;
-                    best_block = blk;
-                    best_grid = gr;
-                    best_ctas = c;
-                    best_split = split;
-                    best_stage = stage;
-                }
+                if (e == cudaSuccess) shapes.push_back({ms, blk, gr, c, split, stage});
             }
         }
         split = split0;
         stage = stage0;
         restore();
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e == cudaSuccess &&
-            (best_block != block || best_grid != grid || best_split != split || best_stage != stage || reserve != 0)) {
-            block = best_block;
-            grid = best_grid;
-            split = best_split;
-            stage = best_stage;
-            reserve = 0;
+        std::stable_sort(shapes.begin(), shapes.end(), [](const Shape& a, const Shape& b) { return a.ms < b.ms; });
+        auto use = [&](const Shape& t, int res) {
+            if (t.block == block && t.grid == grid && t.split == split && t.stage == stage && res == reserve) return;
+            block = t.block;
+            grid = t.grid;
+            split = t.split;
+            stage = t.stage;
+            reserve = res;
             destroy_graphs();
-        }
-        // with two overlapping chains of persistent kernels and the collision split out,
-        // time whole steps, replayed from the step graphs as they run (the chains
-        // overlap only there), with SMs left free for the other group's collision pass
-        if (e == cudaSuccess && groups() == 2 && grid > 0 && (variant(block) & SV_SPLIT) && p.use_graph) {
-            float best_r = 1e30f;
-            int best_res = 0;
-            for (int res : {0, 8, 16, 24, 32}) {
-                if (res >= sm_count / 2 || e != cudaSuccess) break;
-                reserve = res;
-                destroy_graphs();
-                restore();
-                if (step(chunk_steps) != VISG_OK) e = cudaErrorUnknown;  // captures this shape's graph
-                if (e == cudaSuccess) e = cudaEventRecord(e0, stream);
-                if (e == cudaSuccess && step(2 * chunk_steps) != VISG_OK) e = cudaErrorUnknown;
-                if (e == cudaSuccess) e = cudaEventRecord(e1, stream);
-                if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-                float ms = 0;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (e == cudaSuccess && ms < best_r) {
-                    best_r = ms;
-                    best_res = res;
+        };
+        // whole steps, replayed from the step graphs as they run
+        auto time_graph = [&]() {
+            restore();
+            if (e == cudaSuccess && step(chunk_steps) != VISG_OK) e = cudaErrorUnknown;  // captures this shape's graph
+            if (e == cudaSuccess) e = cudaEventRecord(e0, stream);
+            if (e == cudaSuccess && step(2 * chunk_steps) != VISG_OK) e = cudaErrorUnknown;
+            if (e == cudaSuccess) e = cudaEventRecord(e1, stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            float ms = 1e30f;
+            if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+            return e == cudaSuccess ? ms : 1e30f;
+        };
+        Shape best = shapes.empty() ? Shape{0.0f, block, grid, 0, split, stage} : shapes[0];
+        if (e == cudaSuccess && groups() == 2 && p.use_graph && !shapes.empty()) {
+            // two chains overlap only in the graphs, and how well depends on the shape: the best
+            // single chain of 30 garments is one CTA of 1,024 threads an SM, the best pair of
+            // chains 4 of 256 (six frames with their read-back 396 -> 380 us).  So the shapes
+            // within a quarter of the best are timed again as they run (at most 10; 2 ms each)
+            float best_ms = 1e30f;
+            for (size_t k = 0; k < shapes.size() && k < 10 && shapes[k].ms <= 1.25f * shapes[0].ms; ++k) {
+                use(shapes[k], 0);
+                const float ms = time_graph();
+                if (ms < best_ms) {
+                    best_ms = ms;
+                    best = shapes[k];
                 }
             }
-            reserve = best_res;
+            use(best, 0);
+            // persistent kernels with the collision split out: SMs left free for the other
+            // group's collision pass
+            if (grid > 0 && (variant(block) & SV_SPLIT)) {
+                int best_res = 0;
+                for (int res : {8, 16, 24, 32}) {
+                    if (res >= sm_count / 2 || e != cudaSuccess) break;
+                    use(best, res);
+                    const float ms = time_graph();
+                    if (ms < best_ms) {
+                        best_ms = ms;
+                        best_res = res;
+                    }
+                }
+                use(best, best_res);
+            }
             restore();
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             destroy_graphs();
+        } else if (e == cudaSuccess) {
+            use(best, 0);
         }
+        prev_ok = prev_ok0;  // the timed steps never happened
+        steps_since_check = since_check0;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         cudaFree(bs);
         cudaFree(bn);
         if (e != cudaSuccess) return cuda_fail(e, "autotune");
         if (out_block) *out_block = block;
-        if (out_ctas) *out_ctas = best_ctas;
+        if (out_ctas) *out_ctas = best.ctas;
         return sync();
     }
 
