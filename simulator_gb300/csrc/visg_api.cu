@@ -52,10 +52,12 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 constexpr int kNumBlocks = 4;
 constexpr int kBlocks[kNumBlocks] = {128, 256, 512, 1024};
-// largest sliced-ELL block (entries) a tile of each block size may stage in shared
-// memory: 16 entries per vertex (14 for 1024, whose two buffers must fit the 227 KB a
-// CTA may hold); two buffers take 32 / 64 / 128 / 224 KB
+// largest sliced-ELL block (entries) of a tile that a launch with helper warps stages in
+// shared memory: 16 entries per vertex
 constexpr int kStageCap[kNumBlocks] = {2048, 4096, 8192, 14336};
+// longest slice that a warp's stage buffer may hold: rows of 24, so that the 32 buffers of a
+// 1,024-thread CTA (192 KB) fit an SM; the buffers are as long as the longest such slice
+constexpr int kSliceCap = 32 * 24;
 // vertices per SM up to which a step has helper warps (twice the threads): beyond, the
 // main warps alone fill the SMs (64 registers: 1,024 threads an SM).  Step kernel with
 // contacts, without -> with: 64 x 64 sheet 10.7 -> 7.8 us, 131 x 127 damped mesh 9.2 and
@@ -130,6 +132,7 @@ struct Engine {
     // boundary vsplit (vertex), i.e. at tile tsplit[b] of each tile table
     int tsplit[kNumBlocks] = {0, 0, 0, 0};
     int64_t vsplit = 0;
+    int ssplit = 0;  // the same boundary in the slice table
     bool finalized = false;
     std::vector<GarmentIn> gin;
     int G = 0;
@@ -147,7 +150,9 @@ struct Engine {
     int4* d_tiles[kNumBlocks] = {nullptr, nullptr, nullptr, nullptr};
     int n_tiles[kNumBlocks] = {0, 0, 0, 0};
     int2* d_twin[kNumBlocks] = {nullptr, nullptr, nullptr, nullptr};  // per tile sliced-ELL block {first entry, count}
-    int win_cap[kNumBlocks] = {0, 0, 0, 0};                           // entries per stage buffer, 0 = no tile staged
+    int win_cap[kNumBlocks] = {0, 0, 0, 0};                           // entries of the longest block
+    int4* d_slices = nullptr;                        // per slice, for the staged step
+    int n_slices = 0, slice_cap = 0;                 // entries per warp's stage buffer, 0 = no slice staged
     uint2* d_sell = nullptr;                         // sliced-ELL springs
     float* d_sellk = nullptr;
     uint32_t* d_slice_off = nullptr;
@@ -414,6 +419,17 @@ struct Engine {
                     if (perk) sellk[soff[s] + 32 * (int64_t)k + lane] = kk[rp + k];
                 }
             }
+        // the slices as the staged step walks them
+        std::vector<int4> slices(S > 0 ? S : 1, make_int4(0, 0, 0, 0));
+        slice_cap = 0;
+        for (int g = 0; g < G; ++g)
+            for (int64_t s = slice0[g]; s < slice0[g + 1]; ++s) {
+                const int64_t v0 = voff[g] + 32 * (s - slice0[g]), cnt = (int64_t)soff[s + 1] - soff[s];
+                slices[s] = make_int4(g | (gin[g].nt > 0 ? TILE_BODY : 0), (int)v0, (int)soff[s],
+                                      (int)(std::min<int64_t>(32, voff[g + 1] - v0) | (cnt / 32) << 6));
+                if (cnt <= kSliceCap) slice_cap = std::max(slice_cap, (int)cnt);
+            }
+        n_slices = (int)S;
         // tiles for each block size, with the sliced-ELL block of each one's slices
         std::vector<std::vector<int4>> tiles(kNumBlocks);
         std::vector<std::vector<int2>> twin(kNumBlocks);
@@ -440,6 +456,7 @@ struct Engine {
             for (int g = 2; g < G; ++g)
                 if (std::llabs(2 * voff[g] - N) < std::llabs(2 * voff[gs] - N)) gs = g;
             vsplit = voff[gs];
+            ssplit = (int)slice0[gs];
             for (int b = 0; b < kNumBlocks; ++b) {
                 tsplit[b] = 0;
                 while (tsplit[b] < (int)tiles[b].size() && (tiles[b][tsplit[b]].x & TILE_GARMENT) < gs) ++tsplit[b];
@@ -457,6 +474,7 @@ struct Engine {
             arena.want(&d_tiles[b], tiles[b].size() + 1);
             arena.want(&d_twin[b], twin[b].size() + 1);
         }
+        arena.want(&d_slices, slices.size());
         arena.want(&d_sell, sell.size());
         if (perk) arena.want(&d_sellk, sellk.size());
         arena.want(&d_slice_off, soff.size());
@@ -497,6 +515,7 @@ struct Engine {
             CU(cudaMemcpy(d_tiles[b], tiles[b].data(), tiles[b].size() * sizeof(int4), cudaMemcpyHostToDevice));
             CU(cudaMemcpy(d_twin[b], twin[b].data(), twin[b].size() * sizeof(int2), cudaMemcpyHostToDevice));
         }
+        CU(cudaMemcpy(d_slices, slices.data(), slices.size() * sizeof(int4), cudaMemcpyHostToDevice));
         CU(cudaMemcpy(d_sell, sell.data(), sell.size() * sizeof(uint2), cudaMemcpyHostToDevice));
         if (perk) CU(cudaMemcpy(d_sellk, sellk.data(), sellk.size() * sizeof(float), cudaMemcpyHostToDevice));
         CU(cudaMemcpy(d_slice_off, soff.data(), soff.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -530,7 +549,7 @@ struct Engine {
     int variant(int blk) const {
         int v = variant();
         const int bi = block_index(blk);
-        if (stage && bi >= 0 && win_cap[bi] > 0) v |= SV_STAGED;
+        if (stage && bi >= 0 && slice_cap > 0) v |= SV_STAGED;
         else if ((v & SV_COLLIDE) && blk <= kHelpBlockMax && helped())
             v |= SV_HELP;
         // two chains of large kernels share the SMs: one chain's blocks that wait for their
@@ -606,6 +625,10 @@ struct Engine {
         a.wild = d_wild;
         a.twin = d_twin[bi] + t0;
         a.win_cap = win_cap[bi];
+        const int c0 = (two && grp == 1) ? ssplit : 0, c1 = (two && grp == 0) ? ssplit : n_slices;
+        a.slices = d_slices + c0;
+        a.n_slices = c1 - c0;
+        a.slice_cap = slice_cap;
         a.settled = settled ? 1 : 0;
         a.p = step_params();
         return a;
@@ -1161,7 +1184,7 @@ struct Engine {
         if (!finalized) return fail(VISG_ERR_STATE, "not finalized");
         const int bi = block_index(blk);
         if (bi < 0) return fail(VISG_ERR_INVALID_ARG, "block must be 128, 256, 512 or 1024");
-        if (ctas < 0 || (ctas > 0 && ctas > step_max_ctas_per_sm(variant(blk), blk, win_cap[bi])))
+        if (ctas < 0 || (ctas > 0 && ctas > step_max_ctas_per_sm(variant(blk), blk, slice_cap)))
             return fail(VISG_ERR_INVALID_ARG, "ctas_per_sm out of range for this block size");
         if (int r = sync()) return r;
         if (blk != block || ctas * sm_count != grid || reserve != 0) {
@@ -1232,11 +1255,11 @@ struct Engine {
             split = (sv / kNumBlocks) % n_split;
             const int bi = sv % kNumBlocks;
             const int blk = kBlocks[bi];
-            if (stage && win_cap[bi] == 0) continue;
+            if (stage && slice_cap == 0) continue;
             // few vertices: what a step takes then is the latency of its contacts, which the
             // state at hand may not show (a sheet still falling); only shapes with helper warps
             if (helped() && (stage || blk > kHelpBlockMax)) continue;
-            const int occ = step_max_ctas_per_sm(variant(blk), blk, win_cap[bi]);
+            const int occ = step_max_ctas_per_sm(variant(blk), blk, slice_cap);
             std::vector<int> ctas;
             for (int c = 1; c <= occ; c *= 2) ctas.push_back(c);
             if (occ > 0 && ctas.back() != occ) ctas.push_back(occ);
@@ -1290,7 +1313,7 @@ struct Engine {
         Shape best = shapes.empty() ? Shape{0.0f, block, grid, 0, split, stage} : shapes[0];
         if (e == cudaSuccess && groups() == 2 && p.use_graph && !shapes.empty()) {
             // two chains overlap only in the graphs, and how well depends on the shape: the best
-            // single chain of 30 garments is one CTA of 1,024 threads an SM, the best pair of
+            // single chain of 24 garments is one CTA of 1,024 threads an SM, the best pair of
             // chains 4 of 256 (six frames with their read-back 396 -> 380 us).  So the shapes
             // within a quarter of the best are timed again as they run (at most 10; 2 ms each)
             float best_ms = 1e30f;

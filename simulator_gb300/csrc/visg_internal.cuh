@@ -193,7 +193,10 @@ struct StepArgs {
     const uint2* vcount;      // per vertex: springs per list, 16 bits each (list 3: 15), bit 63 = pinned
     uint32_t* wild;           // sticky: some record had |x| >= 3e14 or |v| >= 1e15 (or NaN)
     const int2* twin;         // per tile sliced-ELL block, with SV_STAGED
-    int win_cap;              // entries per shared-memory stage buffer
+    int win_cap;              // entries of the longest tile block that helper launches stage
+    const int4* slices;       // {garment, first vertex, first entry, vertices | row length << 6} per slice
+    int n_slices;
+    int slice_cap;            // entries a warp's stage buffer holds
     int settled;              // the bodies' trees were complete before the launch before this one began
     StepParams p;
 };
@@ -210,12 +213,12 @@ enum StepVariant : int {
     SV_OVERLAP = 256, // a launch may begin while the one before it runs (fused collision)
 };
 constexpr int kHelpBlockMax = 256;  // tile sizes up to which there are kernels with helper warps
-// dynamic shared memory of a launch: two stage buffers of win_cap entries + barriers
-int step_smem_bytes(int variant, int win_cap);
+// dynamic shared memory of a staged launch: a buffer of slice_cap entries and a barrier per warp
+int step_smem_bytes(int variant, int block, int slice_cap);
 cudaError_t launch_step(const StepArgs& a, int variant, int block, int grid, cudaStream_t s);
 // record `before` / `after` around every step-kernel launch this thread issues (null: stop)
 void set_step_timing(cudaEvent_t before, cudaEvent_t after);
-int step_max_ctas_per_sm(int variant, int block, int win_cap);
+int step_max_ctas_per_sm(int variant, int block, int slice_cap);
 
 // self-tests of the bounded waits: each must give up and set ERR_TIMEOUT in *err
 cudaError_t launch_selftest_mbar_wait(int* err, cudaStream_t s);

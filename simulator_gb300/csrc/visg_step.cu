@@ -288,7 +288,7 @@ __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const floa
 // F + the spring forces of one vertex, list by list as the reference does
 // (force += list sum, verlet.cu:148-149); cnt holds the row's per-list counts.
 // UNROLL pairs are in flight: 1 where many warps hide the gathers (more registers would
-// cost warps), 2 where there are few.
+// cost warps) or the registers are few (damped), 2 beside helper warps.
 template <SumMode MODE, int UNROLL, bool PERK, class Rec, class Ent>
 __device__ __forceinline__ f3 row_lists(const Rec& rec, const Ent& ep, const float* __restrict__ kp, uint2 cnt, f3 x,
                                         f3 vel, f3 F, const StepParams& P, f3 eps3, PairRange& rg) {
@@ -399,23 +399,28 @@ __device__ __forceinline__ void helper_query(const StepArgs& a, const int4 td, c
     pair_arrive(j >> 5);
 }
 
-// One thread's vertex of tile td = {garment, first vertex, end vertex, first slice}.
+struct NoHook {
+    __device__ __forceinline__ void operator()() const {}
+};
+
+// One thread's vertex i (`active`: it has one; else ii stands in for loads) of garment
+// `garment` (a tile's or slice's flags word), whose row's sliced-ELL entry 0 is sb.
+// after_sum() is called by the whole warp once its rows are summed.
 // State record of vertex i in buffer b: [x.xyz, v.x] [v.y, v.z, flags, 0] with
 // v = (x - x_old) / dt.  x_old is x itself when FLAG_XO_IS_X is set (after a
 // contact, a pin or update_vertex) and otherwise the previous step's x, which is
 // still in the other buffer: the step reads it there before overwriting it.
-template <bool COLL, bool KD0, bool SPLIT, bool SMEM_ENT, bool HELP>
-__device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, const uint2* ebase, const uint32_t e0,
+template <bool COLL, bool KD0, bool SPLIT, bool SMEM_ENT, bool HELP, class Hook>
+__device__ __forceinline__ void vertex_step(const StepArgs& a, const int garment, const int i, const bool active,
+                                            const int ii, const uint32_t sb, const uint2* ebase, const uint32_t e0,
                                             const int refv, const int check, const int perk, const bool wild,
-                                            const HelperAnswers& help, float& my_disp, uint32_t& my_bad) {
-    constexpr int kPairs = HELP ? 2 : 1;
+                                            const HelperAnswers& help, float& my_disp, uint32_t& my_bad,
+                                            const Hook& after_sum) {
+    constexpr int kPairs = HELP && KD0 ? 2 : 1;
     const GlobalRecords rec{a.state_in};
     const StepParams& P = a.p;
     const f3 grav = mk3(P.gx, P.gy, P.gz);
     const f3 eps3 = mk3(kFltEpsilon, kFltEpsilon, kFltEpsilon);
-    const int i = td.y + (int)threadIdx.x;
-    const bool active = i < td.z;
-    const int ii = active ? i : td.y;
     const float4 s0 = rec.r0(ii);
     const f3 x = mk3(s0.x, s0.y, s0.z);
     const uint2 cnt = __ldg(&a.vcount[ii]);
@@ -424,7 +429,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         // the record's flags word (the sector s0 came in): start the loads that a cached
         // contact answer and a stored normal need after the spring sum
         const uint32_t fl0 = __float_as_uint(reinterpret_cast<const float*>(a.state_in + 2 * ii + 1)[2]);
-        const BvhRoot* const rt = a.roots + (td.x & TILE_GARMENT);
+        const BvhRoot* const rt = a.roots + (garment & TILE_GARMENT);
         if (fl0 & FLAG_LEAF_CACHED) prefetch_contact(rt->leaves + 2 * (fl0 >> LEAF_SHIFT));
         if (fl0 & FLAG_HAS_NORMAL) prefetch_contact(a.normal + ii);
     }
@@ -432,26 +437,30 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
     bool has_n = false;
     uint32_t flags = 0u;
     float margin = 0.0f;
-    if (active && !pinned) {
-        const int lane = (int)(threadIdx.x & 31u);
-        const uint32_t sb = __ldg(&a.slice_off[td.w + (int)(threadIdx.x >> 5)]) + (uint32_t)lane;  // row entry 0
+    const bool moves = active && !pinned;
+    f3 F = mk3(0.0f, 0.0f, 0.0f);
+    bool redo = wild;
+    // gravity and force damping.  With drec and force damping exactly +0 the term v * +0 is a
+    // signed zero for every tame v, and g m + (+-0) only differs in the sign of a zero
+    // component, which the first list's sum (never -0) erases.
+    const bool damped = !P.drec || __float_as_uint(P.damp) != 0u || wild;
+    const auto outer_force = [&](f3 vel) {
+        const f3 f = mul(grav, P.mass);
+        return damped ? add(f, mul(vel, P.damp)) : f;
+    };
+    if (moves) {
         // The zero-damping sum needs only positions: there the rest of the record
         // (v or D, flags, the query cache's margin) is read after the sum, not held in
-        // registers across it.  With drec and force damping exactly +0 the term v * +0
-        // is a signed zero for every tame v, and g m + (+-0) only differs in the sign
-        // of a zero component, which the first list's sum (never -0) erases.
-        const bool pos_only = KD0 && P.drec && __float_as_uint(P.damp) == 0u && !wild;
+        // registers across it.
+        const float* kp = perk ? a.sellk + sb : nullptr;
         f3 vel = mk3(0.0f, 0.0f, 0.0f);
-        f3 F0 = mul(grav, P.mass);
-        if (!pos_only) {
+        if (!KD0 || damped) {
             const float4 s1 = rec.r1(ii);
             const f3 rv = mk3(s0.w, s1.x, s1.y);  // v, or D = x - x_old with drec
             vel = P.drec ? divs(rv, P.dt) : rv;
-            if (!P.drec || __float_as_uint(P.damp) != 0u || wild) F0 = add(F0, mul(vel, P.damp));
         }
+        const f3 F0 = outer_force(vel);
         const Entries<SMEM_ENT> ep{ebase + (sb - e0)};
-        const float* kp = perk ? a.sellk + sb : nullptr;
-        f3 F;
         PairRange rg;
         if (KD0) {
             // Spring damping is +0: the reference adds +0 * RN(dv.d / |d|) to every c.
@@ -464,16 +473,24 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
         } else {
             F = row_forces<SUM_DAMPED, kPairs>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3, rg);
         }
+        redo = redo || !rg.exact();
+    }
+    if constexpr (!HELP) after_sum();
+    if (moves) {
         // the record again (a second read of a line this thread has just read)
         const f4x2 own = ld8(a.state_in + 2 * ii);
         const float4 r0 = own.a, r1 = own.b;
         const f3 rv = mk3(r0.w, r1.x, r1.y);  // v, or D = x - x_old with drec
         flags = __float_as_uint(r1.z);
         margin = r1.w;
-        // what the packed evaluation does not answer for, spring by spring
-        if (wild || !rg.exact() || !(isfinite(F.x) && isfinite(F.y) && isfinite(F.z))) {
-            vel = P.drec ? divs(rv, P.dt) : rv;
-            F = row_forces<SUM_SCALAR, 1>(rec, ep, kp, cnt, x, vel, F0, P, perk != 0, eps3, rg);
+        // what the packed evaluation does not answer for, spring by spring (a staged row may
+        // be gone by now: from global memory)
+        if (redo || !(isfinite(F.x) && isfinite(F.y) && isfinite(F.z))) {
+            const f3 vel = P.drec ? divs(rv, P.dt) : rv;
+            const Entries<false> ep{a.sell + sb};
+            PairRange rg;
+            F = row_forces<SUM_SCALAR, 1>(rec, ep, perk ? a.sellk + sb : nullptr, __ldg(&a.vcount[ii]), x, vel,
+                                          outer_force(vel), P, perk != 0, eps3, rg);
         }
         // x - x_old: from the record (drec), else from x_old in the other buffer
         f3 xo = x, d = rv;
@@ -497,8 +514,8 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
     float skin = 0.0f;
     uint32_t leaf_bits = 0u;  // the cached leaf, in the flags word's place (0: no leaf cached)
     if (COLL) {
-        const int g = td.x & TILE_GARMENT;
-        const bool body = (td.x & TILE_BODY) != 0;  // the garment has a body (its tree has leaves)
+        const int g = garment & TILE_GARMENT;
+        const bool body = (garment & TILE_BODY) != 0;  // the garment has a body (its tree has leaves)
         bool query = false;
         int leaf = -1;
         if (HELP) {
@@ -584,7 +601,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int4 td, co
 }
 
 // ---- TMA bulk copies into shared memory, completed on an mbarrier ----------------------
-constexpr int kBarBytes = 128;                 // two 8-byte mbarriers, padded
+constexpr int kBarBytes = 256;                 // an 8-byte mbarrier per warp
 constexpr uint64_t kWaitNs = 1000000000ull;    // a stage that has not landed after 1 s is an error
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -631,37 +648,49 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return true;
 }
 
-// the stager: stage the sliced-ELL block of `tile` at shared address dst, completing
-// the buffer's `full` phase when it lands; a tile without a staged block completes
-// the phase at once (every tile takes one phase, so no warp runs ahead of the ring)
-__device__ __forceinline__ void stage_entries(const StepArgs& a, int tile, uint32_t dst, uint32_t full) {
-    const int2 tw = __ldg(&a.twin[tile]);
-    if (tw.y > 0) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the readers' loads come first
-        bulk_stage(dst, a.sell + (uint32_t)tw.x, (uint32_t)tw.y * 8u, full);
-    } else {
-        mbar_arrive(full);
-    }
+// whether slice sl is staged: it has entries, and they fit a warp's buffer
+__device__ __forceinline__ bool slice_staged(const StepArgs& a, const int4 sl) {
+    const uint32_t rows = (uint32_t)sl.w >> 6;
+    return rows != 0u && 32u * rows <= (uint32_t)a.slice_cap;
 }
 
-// The fused step: persistent CTAs walk the tile table.  With STAGED, one thread (the
-// stager) copies the next tile's block of sliced-ELL entries (the tile's slices are
-// contiguous: one TMA bulk copy) into the other shared-memory buffer while the warps
-// compute the current tile, so each spring's chain starts with a shared-memory load;
-// tiles whose block exceeds the buffer read their entries from global memory.  No CTA
-// barrier per tile: warps report a finished buffer on its `empty` mbarrier and only
-// the stager waits for it before refilling.  The stager of iteration `it` is lane 0 of
-// warp it % (BLOCK / 32), so the wait for the slowest warp and the copy's issue
-// latency fall on each warp once per BLOCK / 32 tiles.  With thread 0 as the only
-// stager they fell on warp 0 every tile, and warp 0 paced the CTA: the other warps
-// ran up to a tile ahead and then waited on `full`.  Waits are bounded: one that
-// gives up after kWaitNs sets ERR_TIMEOUT, the iteration's stager waits (again
-// bounded) for the copies in flight, and the warp exits; warps left waiting on a
-// copy that is never issued give up the same way.
+// One tile's vertices (a thread each), entries read where ebase points.
+template <bool COLL, bool KD0, bool SPLIT, bool SMEM_ENT, bool HELP>
+__device__ __forceinline__ void tile_step(const StepArgs& a, const int4 td, const uint2* ebase, const uint32_t e0,
+                                          const int refv, const int check, const int perk, const bool wild,
+                                          const HelperAnswers& help, float& my_disp, uint32_t& my_bad) {
+    const int i = td.y + (int)threadIdx.x;
+    const bool active = i < td.z;
+    const uint32_t sb =
+        active ? __ldg(&a.slice_off[td.w + (int)(threadIdx.x >> 5)]) + (uint32_t)(threadIdx.x & 31u) : e0;
+    vertex_step<COLL, KD0, SPLIT, SMEM_ENT, HELP>(a, td.x, i, active, active ? i : td.y, sb, ebase, e0, refv, check,
+                                                  perk, wild, help, my_disp, my_bad, NoHook());
+}
+
+// The fused step.  With STAGED, persistent warps walk the slices (32 vertices of a garment
+// and their contiguous sliced-ELL entries): each has a shared-memory buffer for one slice,
+// which a TMA bulk copy fills, so every spring's chain starts with a shared-memory load.
+// Once a warp has summed its rows nothing reads the buffer any more (rows that must be
+// summed again read global memory), so it starts the copy of its next slice and answers
+// the queries, stores the records and loads the next vertices while that lands.  A warp
+// waits for no other, and half the shared memory of a ring of two buffers leaves the L1,
+// which serves the neighbours' records, the rest: 44 garments (two chains) 68.0 -> 61.8 us a
+// step against a ring of two tiles a CTA of 128 (9 CTAs an SM in both).  Slices longer than
+// the buffer are read from global memory.  Waits are bounded: one that gives up after kWaitNs sets ERR_TIMEOUT,
+// waits (again bounded) for the copy in flight, and the warp exits.
 //
 // HELP: BLOCK more threads are helper warps (above); one tile per CTA.
+// Threads per SM that the registers of the staged kernels allow (CTAs of less than 1,024):
+// 56 registers.  44 garments, us a step with as many CTAs as fit: 1,024 threads 68.5, 1,152
+// 61.8 (13 registers' worth of values that the springs do not use are spilled), 1,280 67.0,
+// 1,536 65.1.  Two pairs of springs in flight (UNROLL) 68, the next slice's records
+// prefetched 62.7.
+constexpr int kStagedThreads = 1152;
+// With helper warps 64 registers, so that launches that overlap find room (72: 20 steps of a
+// 131 x 127 mesh 245 us, 64: 233).
 template <int BLOCK, bool COLL, bool KD0, bool SPLIT, bool STAGED, bool HELP>
-__global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK)
+__global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK,
+                                  STAGED && BLOCK < 1024 ? kStagedThreads / BLOCK : HELP ? 512 / BLOCK : 0)
     k_step(const StepArgs a, const int refv, const int check, const int perk) {
     extern __shared__ __align__(128) unsigned char dyn_smem[];
     __shared__ int s_leaf[HELP ? BLOCK : 1];
@@ -689,11 +718,11 @@ __global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK)
         const bool wild = *reinterpret_cast<const volatile uint32_t*>(a.wild) != 0u;
         const bool landed = __all_sync(0xffffffffu, staged && mbar_wait(full, 0u));
         if (landed) {
-            vertex_step<COLL, KD0, SPLIT, true, HELP>(a, td, reinterpret_cast<const uint2*>(dyn_smem + kBarBytes),
+            tile_step<COLL, KD0, SPLIT, true, HELP>(a, td, reinterpret_cast<const uint2*>(dyn_smem + kBarBytes),
                                                       (uint32_t)tw.x, refv, check, perk, wild, help, my_disp, my_bad);
         } else {
             if (staged && (threadIdx.x & 31u) == 0u) atomicOr(a.err, ERR_TIMEOUT);
-            vertex_step<COLL, KD0, SPLIT, false, HELP>(a, td, a.sell, 0u, refv, check, perk, wild, help, my_disp,
+            tile_step<COLL, KD0, SPLIT, false, HELP>(a, td, a.sell, 0u, refv, check, perk, wild, help, my_disp,
                                                        my_bad);
             if (staged && threadIdx.x == 0u) mbar_wait(full, 0u);  // the copy in flight, again bounded
         }
@@ -701,59 +730,59 @@ __global__ void __launch_bounds__(HELP ? 2 * BLOCK : BLOCK)
         wait_for_earlier_launches();
         const bool wild = *reinterpret_cast<const volatile uint32_t*>(a.wild) != 0u;
         for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x)
-            vertex_step<COLL, KD0, SPLIT, false, false>(a, __ldg(&a.tiles[tile]), a.sell, 0u, refv, check, perk, wild,
-                                                        help, my_disp, my_bad);
+            tile_step<COLL, KD0, SPLIT, false, false>(a, __ldg(&a.tiles[tile]), a.sell, 0u, refv, check, perk, wild,
+                                                      help, my_disp, my_bad);
     } else {
-        // two-buffer ring: full[b] completes when buffer b holds its tile's block,
-        // empty[b] when every warp is done reading it
-        const uint32_t full = smem_addr(dyn_smem), empty = full + 16u;
-        const uint32_t buf0 = full + kBarBytes;
-        const uint2* sbuf = reinterpret_cast<const uint2*>(dyn_smem + kBarBytes);
-        const uint32_t bbytes = (uint32_t)a.win_cap * 8u;
-        const int lane = (int)(threadIdx.x & 31u);
-        if (threadIdx.x == 0) {
-            mbar_init(full, 1u);
-            mbar_init(full + 8u, 1u);
-            mbar_init(empty, BLOCK / 32);
-            mbar_init(empty + 8u, BLOCK / 32);
+        const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u);
+        const uint32_t bar = smem_addr(dyn_smem) + 8u * (uint32_t)warp;
+        const uint32_t buf = smem_addr(dyn_smem) + kBarBytes + (uint32_t)(warp * a.slice_cap) * 8u;
+        const uint2* const entries = reinterpret_cast<const uint2*>(dyn_smem + kBarBytes) + warp * a.slice_cap;
+        const int stride = (int)gridDim.x * (BLOCK / 32);
+        int s = (int)blockIdx.x * (BLOCK / 32) + warp;
+        int4 sl = make_int4(0, 0, 0, 0);
+        if (s < a.n_slices) sl = __ldg(&a.slices[s]);
+        if (lane == 0) {
+            mbar_init(bar, 1u);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            if (slice_staged(a, sl)) bulk_stage(buf, a.sell + (uint32_t)sl.z, ((uint32_t)sl.w >> 6) * 256u, bar);
         }
-        __syncthreads();
-        if (threadIdx.x == 0 && (int)blockIdx.x < a.n_tiles) stage_entries(a, blockIdx.x, buf0, full);
+        __syncwarp();
         wait_for_earlier_launches();  // the springs do not change, so the first are on their way
         const bool wild = *reinterpret_cast<const volatile uint32_t*>(a.wild) != 0u;
-        int it = 0;
-        for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++it) {
-            const int b = it & 1;
-            const uint32_t par = (uint32_t)(it >> 1) & 1u;  // phase parity of this iteration's buffer
-            const int nxt = tile + (int)gridDim.x;
-            const uint32_t stager = (uint32_t)(it % (BLOCK / 32)) * 32u;
-            bool pok = true;
-            if (threadIdx.x == stager && nxt < a.n_tiles) {
-                // the other buffer was read in iteration it - 1: wait for every warp to finish it
-                if (it >= 1) pok = mbar_wait(empty + 8u * (b ^ 1), (uint32_t)((it - 1) >> 1) & 1u);
-                if (pok) stage_entries(a, nxt, buf0 + (uint32_t)(b ^ 1) * bbytes, full + 8u * (b ^ 1));
-            }
-            const bool landed = mbar_wait(full + 8u * b, par);
-            if (!__all_sync(0xffffffffu, landed && pok)) {
-                // a wait gave up: record it; the stager lets the copies in flight land
-                if (lane == 0) atomicOr(a.err, ERR_TIMEOUT);
-                if (threadIdx.x == stager) {
-                    mbar_wait(full + 8u * b, par);
-                    if (pok && nxt < a.n_tiles) mbar_wait(full + 8u * (b ^ 1), (uint32_t)((it + 1) >> 1) & 1u);
+        uint32_t parity = 0u;
+        for (; s < a.n_slices; s += stride) {
+            const bool staged = slice_staged(a, sl);
+            const int i = sl.y + lane;
+            const bool active = lane < (sl.w & 63);
+            int4 next = make_int4(0, 0, 0, 0);
+            if (staged) {
+                if (!__all_sync(0xffffffffu, mbar_wait(bar, parity))) {
+                    if (lane == 0) {
+                        atomicOr(a.err, ERR_TIMEOUT);
+                        mbar_wait(bar, parity);
+                    }
+                    return;
                 }
-                return;
+                parity ^= 1u;
             }
-            const int4 td = __ldg(&a.tiles[tile]);
-            const int2 tw = __ldg(&a.twin[tile]);
-            if (tw.y > 0)
-                vertex_step<COLL, KD0, SPLIT, true, false>(a, td, sbuf + (size_t)b * a.win_cap, (uint32_t)tw.x, refv,
-                                                           check, perk, wild, help, my_disp, my_bad);
+            const auto fetch_next = [&]() {
+                __syncwarp();
+                if (s + stride < a.n_slices) next = __ldg(&a.slices[s + stride]);
+                if (lane == 0 && slice_staged(a, next)) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the rows' loads come first
+                    bulk_stage(buf, a.sell + (uint32_t)next.z, ((uint32_t)next.w >> 6) * 256u, bar);
+                }
+                __syncwarp();
+            };
+            const uint32_t e0 = (uint32_t)sl.z, sb = e0 + (uint32_t)lane;
+            const int ii = active ? i : sl.y;
+            if (staged)
+                vertex_step<COLL, KD0, SPLIT, true, false>(a, sl.x, i, active, ii, sb, entries, e0, refv, check, perk,
+                                                           wild, help, my_disp, my_bad, fetch_next);
             else
-                vertex_step<COLL, KD0, SPLIT, false, false>(a, td, a.sell, 0u, refv, check, perk, wild, help, my_disp,
-                                                            my_bad);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty + 8u * b);
+                vertex_step<COLL, KD0, SPLIT, false, false>(a, sl.x, i, active, ii, sb, a.sell, 0u, refv, check, perk,
+                                                            wild, help, my_disp, my_bad, fetch_next);
+            sl = next;
         }
     }
     if (check) {
@@ -890,7 +919,7 @@ cudaError_t launch_block(const StepArgs& a, int variant, int grid, cudaStream_t 
     const bool help = BLOCK <= kHelpBlockMax && (variant & SV_HELP) && !(variant & SV_STAGED) && grid == a.n_tiles;
     const StepKernel fn = step_kernel<BLOCK>(help ? variant : variant & ~SV_HELP);
     const bool split = (variant & SV_COLLIDE) && (variant & SV_SPLIT);
-    const int smem = help ? kBarBytes + 8 * a.win_cap : step_smem_bytes(variant, a.win_cap);
+    const int smem = help ? kBarBytes + 8 * a.win_cap : step_smem_bytes(variant, BLOCK, a.slice_cap);
     cudaError_t e = allow_smem((const void*)fn, smem);
     if (e != cudaSuccess) return e;
     if (split) {
@@ -920,9 +949,9 @@ cudaError_t launch_block(const StepArgs& a, int variant, int grid, cudaStream_t 
 }
 
 template <int BLOCK>
-int occupancy_block(int variant, int win_cap) {
+int occupancy_block(int variant, int slice_cap) {
     const StepKernel fn = step_kernel<BLOCK>(variant & ~SV_HELP);
-    const int smem = step_smem_bytes(variant, win_cap);
+    const int smem = step_smem_bytes(variant, BLOCK, slice_cap);
     if (allow_smem((const void*)fn, smem) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, BLOCK, smem) != cudaSuccess) return 0;
@@ -1119,16 +1148,16 @@ cudaError_t launch_step(const StepArgs& a, int variant, int block, int grid, cud
     }
 }
 
-int step_smem_bytes(int variant, int win_cap) {
-    return (variant & SV_STAGED) ? kBarBytes + 2 * 8 * win_cap : 0;
+int step_smem_bytes(int variant, int block, int slice_cap) {
+    return (variant & SV_STAGED) ? kBarBytes + block / 32 * 8 * slice_cap : 0;
 }
 
-int step_max_ctas_per_sm(int variant, int block, int win_cap) {
+int step_max_ctas_per_sm(int variant, int block, int slice_cap) {
     switch (block) {
-        case 128: return occupancy_block<128>(variant, win_cap);
-        case 256: return occupancy_block<256>(variant, win_cap);
-        case 512: return occupancy_block<512>(variant, win_cap);
-        case 1024: return occupancy_block<1024>(variant, win_cap);
+        case 128: return occupancy_block<128>(variant, slice_cap);
+        case 256: return occupancy_block<256>(variant, slice_cap);
+        case 512: return occupancy_block<512>(variant, slice_cap);
+        case 1024: return occupancy_block<1024>(variant, slice_cap);
         default: return 0;
     }
 }
