@@ -106,14 +106,14 @@ int Engine::forward(int nsteps, int ckpt) {
         return adj.tmp + (size_t)(t & 1) * st;
     };
     double* first = place(0);
-    CU(launch_unpack_state(d_state[cur], d_state[cur ^ 1], d_normal, N, d_stage, d_stage + n3, d_stage + 2 * n3,
+    CU(launch_unpack_state(d_state[cur], d_state[cur ^ 1], d_normal, 0, N, d_stage, d_stage + n3, d_stage + 2 * n3,
                            stream));
     CU(launch_widen(d_stage, first, (int64_t)st, stream));
     CU(launch_vel_f64(first, first + n3, damped_springs() ? adj.vel : nullptr, p.dt, adj.wild, (int64_t)n3, stream));
     for (int s = 0; s < nsteps; ++s) CU(step64(place(s), place(s + 1), s, adj.contacts + s));
     // the simulator continues from the FP64 final state, rounded to float
     CU(launch_narrow(place(nsteps), d_stage, (int64_t)st, stream));
-    CU(launch_pack_state(d_state[cur], d_state[cur ^ 1], d_normal, N, d_stage, d_stage + n3, d_stage + 2 * n3, p.dt,
+    CU(launch_pack_state(d_state[cur], d_state[cur ^ 1], d_normal, 0, N, d_stage, d_stage + n3, d_stage + 2 * n3, p.dt,
                          step_params().drec, step_params().dmax, d_wild, stream));
     if (int r = sync()) return r;
     adj.rec_seg = last;

@@ -415,7 +415,8 @@ struct Engine {
                     return fail(VISG_ERR_UNSUPPORTED, "more than 65535 springs of one list at one vertex");
                 h_vcount[v] = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16) | (h_rowp[v] & PIN_BIT));
                 for (uint32_t k = 0; k < n; ++k) {
-                    sell[soff[s] + 32 * (int64_t)k + lane] = make_uint2(ent[rp + k].x & END_MASK, ent[rp + k].y);
+                    const int64_t end = ent[rp + k].x & END_MASK;
+                    sell[soff[s] + 32 * (int64_t)k + lane] = make_uint2((uint32_t)rec_at(end), ent[rp + k].y);
                     if (perk) sellk[soff[s] + 32 * (int64_t)k + lane] = kk[rp + k];
                 }
             }
@@ -463,8 +464,8 @@ struct Engine {
             }
         }
         // plan the allocation
-        arena.want(&d_state[0], 2 * (size_t)N + 2);
-        arena.want(&d_state[1], 2 * (size_t)N + 2);
+        arena.want(&d_state[0], records(N));
+        arena.want(&d_state[1], records(N));
         arena.want(&d_normal, (size_t)N + 1);
         arena.want(&d_rowp, (size_t)N + 2);
         arena.want(&d_ent, (size_t)E + 1);
@@ -496,16 +497,16 @@ struct Engine {
         CU(arena.commit());
         for (int g = 0; g < G; ++g) bvh[g].root = d_roots + g;
         // upload
-        std::vector<float4> st(2 * (size_t)N);
+        std::vector<float4> st(records(N), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
         float xo_is_x_bits;
         const uint32_t fl0 = FLAG_XO_IS_X;
         std::memcpy(&xo_is_x_bits, &fl0, 4);
         for (int g = 0; g < G; ++g)
             for (int i = 0; i < gin[g].N; ++i) {
                 const float* q = &gin[g].xyz[3 * (size_t)i];
-                int64_t v = voff[g] + i;
-                st[2 * v] = make_float4(q[0], q[1], q[2], 0.0f);  // x = x_old: v = 0 (simulation.cu:84-85)
-                st[2 * v + 1] = make_float4(0.0f, 0.0f, xo_is_x_bits, 0.0f);
+                const int64_t v = rec_at(voff[g] + i);
+                st[v] = make_float4(q[0], q[1], q[2], 0.0f);  // x = x_old: v = 0 (simulation.cu:84-85)
+                st[v + 32] = make_float4(0.0f, 0.0f, xo_is_x_bits, 0.0f);
             }
         CU(cudaMemcpy(d_state[0], st.data(), st.size() * sizeof(float4), cudaMemcpyHostToDevice));
         CU(cudaMemcpy(d_rowp, h_rowp.data(), h_rowp.size() * 4, cudaMemcpyHostToDevice));
@@ -889,7 +890,7 @@ struct Engine {
         }
         const int k = rb.next;
         if (rb.used[k]) CU(cudaStreamWaitEvent(stream, rb.copied[k], 0));  // slot's last copy has left
-        CU(launch_unpack_positions(d_state[cur], N, rb.d_pos[k], stream));
+        CU(launch_unpack_positions(d_state[cur], 0, N, rb.d_pos[k], stream));
         CU(cudaMemcpyAsync(rb.h_err + k, d_err, 4, cudaMemcpyDeviceToHost, stream));
         CU(cudaEventRecord(rb.unpacked[k], stream));
         CU(cudaStreamWaitEvent(rb.copy, rb.unpacked[k], 0));
@@ -993,10 +994,10 @@ struct Engine {
             n = voff[g + 1] - voff[g];
         }
         if (on_device) {
-            CU(launch_unpack_positions(d_state[cur] + 2 * v0, n, out, stream));
+            CU(launch_unpack_positions(d_state[cur], v0, n, out, stream));
             return VISG_OK;
         }
-        CU(launch_unpack_positions(d_state[cur] + 2 * v0, n, d_stage, stream));
+        CU(launch_unpack_positions(d_state[cur], v0, n, d_stage, stream));
         CU(cudaMemcpyAsync(out, d_stage, (size_t)n * 12, cudaMemcpyDeviceToHost, stream));
         return sync();
     }
@@ -1032,7 +1033,7 @@ struct Engine {
         float* sx = d_stage;
         float* sxo = d_stage + 3 * n;
         float* sn = d_stage + 6 * n;
-        CU(launch_unpack_state(d_state[cur] + 2 * v0, d_state[cur ^ 1] + 2 * v0, d_normal + v0, n, sx, sxo, sn,
+        CU(launch_unpack_state(d_state[cur], d_state[cur ^ 1], d_normal, v0, n, sx, sxo, sn,
                                stream));
         if (x) CU(cudaMemcpyAsync(x, sx, (size_t)n * 12, cudaMemcpyDeviceToHost, stream));
         if (xo) CU(cudaMemcpyAsync(xo, sxo, (size_t)n * 12, cudaMemcpyDeviceToHost, stream));
@@ -1051,7 +1052,7 @@ struct Engine {
         if (xo) CU(cudaMemcpyAsync(sxo, xo, (size_t)n * 12, cudaMemcpyHostToDevice, stream));
         if (nrm) CU(cudaMemcpyAsync(sn, nrm, (size_t)n * 12, cudaMemcpyHostToDevice, stream));
         prev_ok = false;
-        CU(launch_pack_state(d_state[cur] + 2 * v0, d_state[cur ^ 1] + 2 * v0, d_normal + v0, n, x ? sx : nullptr,
+        CU(launch_pack_state(d_state[cur], d_state[cur ^ 1], d_normal, v0, n, x ? sx : nullptr,
                              xo ? sxo : nullptr, nrm ? sn : nullptr, p.dt, step_params().drec,
                              step_params().dmax, d_wild, stream));
         CU(cudaStreamSynchronize(stream));
@@ -1212,7 +1213,7 @@ struct Engine {
         if (!finalized) return fail(VISG_ERR_STATE, "not finalized");
         if (int r = sync()) return r;
         float4 *bs = nullptr, *bn = nullptr;
-        CU(cudaMalloc((void**)&bs, 4 * (size_t)N * sizeof(float4)));
+        CU(cudaMalloc((void**)&bs, 2 * records(N) * sizeof(float4)));
         cudaError_t e = cudaMalloc((void**)&bn, (size_t)N * sizeof(float4));
         if (e != cudaSuccess) {
             cudaFree(bs);
@@ -1221,19 +1222,19 @@ struct Engine {
         const int cur0 = cur;
         const bool prev_ok0 = prev_ok;
         const int64_t since_check0 = steps_since_check;
-        e = cudaMemcpyAsync(bs, d_state[cur], 2 * (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice, stream);
+        e = cudaMemcpyAsync(bs, d_state[cur], records(N) * sizeof(float4), cudaMemcpyDeviceToDevice, stream);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(bs + 2 * N, d_state[cur ^ 1], 2 * (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice,
+            e = cudaMemcpyAsync(bs + records(N), d_state[cur ^ 1], records(N) * sizeof(float4), cudaMemcpyDeviceToDevice,
                                 stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(bn, d_normal, (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice, stream);
         // every candidate starts from the same state, so all are timed on the same contacts
         auto restore = [&]() {
             cur = cur0;
             if (e == cudaSuccess)
-                e = cudaMemcpyAsync(d_state[cur], bs, 2 * (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice,
+                e = cudaMemcpyAsync(d_state[cur], bs, records(N) * sizeof(float4), cudaMemcpyDeviceToDevice,
                                     stream);
             if (e == cudaSuccess)
-                e = cudaMemcpyAsync(d_state[cur ^ 1], bs + 2 * N, 2 * (size_t)N * sizeof(float4),
+                e = cudaMemcpyAsync(d_state[cur ^ 1], bs + records(N), records(N) * sizeof(float4),
                                     cudaMemcpyDeviceToDevice, stream);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(d_normal, bn, (size_t)N * sizeof(float4), cudaMemcpyDeviceToDevice, stream);

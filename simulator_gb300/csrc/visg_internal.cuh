@@ -2,7 +2,11 @@
 //
 // HBM layout (all arrays 16-byte aligned, one allocation per engine):
 //   cloth state, double-buffered: 2 float4 per vertex
-//        [x.x x.y x.z v.x] [v.y v.z flags margin]        32 B, one sector per gather
+//        [x.x x.y x.z v.x] [v.y v.z flags margin]
+//        in blocks of 32 vertices, first halves before second halves (rec_at): the springs
+//        of a warp read neighbours' positions, mostly consecutive, from 512 dense bytes (4
+//        L1 wavefronts a gather; 8 with whole records side by side, half of each line
+//        unread), and a block's halves share their lines with no other block
 //        v = (x - x_old) / dt, computed once per step by the vertex's own thread;
 //        with StepParams::drec the record carries D = x - x_old in its place (then
 //        no spring reads a neighbour's velocity and the step needs only x - x_old);
@@ -16,7 +20,7 @@
 //   rowp:   u32 per vertex + 1, merged CSR row offsets; bit 31 = vertex pinned
 //   ent:    uint2 per directed spring {end | list << 30, rest}         8 B
 //   kent:   f32 per directed spring, only with per-spring stiffness
-//   sell:   the same springs {end, rest} in sliced-ELL order for the step kernel: a slice is 32
+//   sell:   the same springs {rec_at(end), rest} in sliced-ELL order for the step kernel: a slice is 32
 //           consecutive vertices of one garment, padded to its longest row; entry k of
 //           lane l of slice s sits at slice_off[s] + 32 k + l, so the k-th springs of a
 //           warp are one contiguous 256-byte run (sellk: stiffness, same layout)
@@ -45,6 +49,10 @@ void set_last_error(const char* msg);  // what visg_last_error returns next
 
 constexpr uint32_t PIN_BIT = 0x80000000u;
 constexpr uint32_t ROW_MASK = 0x7fffffffu;
+// the first half of vertex i's record, in float4; the second half is 32 further on
+__host__ __device__ __forceinline__ int64_t rec_at(int64_t i) { return 2 * (i & ~(int64_t)31) + (i & 31); }
+__host__ __device__ __forceinline__ uint32_t rec_at(int i) { return (uint32_t)i + ((uint32_t)i & ~31u); }
+inline size_t records(int64_t n) { return 2 * (size_t)((n + 31) & ~(int64_t)31) + 2; }  // float4 for n vertices
 constexpr uint32_t END_MASK = 0x3fffffffu;
 constexpr int LIST_SHIFT = 30;
 constexpr uint32_t FLAG_HAS_NORMAL = 1u;  // the previous contact normal is stored (non-zero)
@@ -232,11 +240,11 @@ cudaError_t launch_query(BvhView v, const float* pts, int n, int* leaf, int* ins
                          float* normal, int* err, cudaStream_t s);
 
 // unpack positions of vertices [0, n) into packed xyz
-cudaError_t launch_unpack_positions(const float4* state, int64_t n, float* out, cudaStream_t s);
-cudaError_t launch_unpack_state(const float4* state, const float4* other, const float4* normal, int64_t n, float* x,
+cudaError_t launch_unpack_positions(const float4* state, int64_t v0, int64_t n, float* out, cudaStream_t s);
+cudaError_t launch_unpack_state(const float4* state, const float4* other, const float4* normal, int64_t v0, int64_t n, float* x,
                                 float* xo, float* nrm, cudaStream_t s);
 // x/xo/nrm may be NULL (kept); dt recomputes v = (x - x_old) / dt
-cudaError_t launch_pack_state(float4* state, float4* other, float4* normal, int64_t n, const float* x,
+cudaError_t launch_pack_state(float4* state, float4* other, float4* normal, int64_t v0, int64_t n, const float* x,
                               const float* xo, const float* nrm, float dt, int drec, float dmax, uint32_t* wild,
                               cudaStream_t s);
 

@@ -338,7 +338,7 @@ __device__ void phase_verts(const RebuildArgs& A) {
     }
     if (A.margin_state)
         for (int64_t i = A.m0 + (int64_t)blockIdx.x * RB + threadIdx.x; i < A.m1; i += (int64_t)gridDim.x * RB)
-            reinterpret_cast<float*>(A.margin_state + 2 * i + 1)[3] = 0.0f;
+            reinterpret_cast<float*>(A.margin_state + rec_at(i) + 32)[3] = 0.0f;
 }
 
 constexpr int BOX_BATCH = 3;  // triangles a thread loads before it computes any

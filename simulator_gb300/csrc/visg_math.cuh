@@ -70,6 +70,11 @@ VISG_LD8(ld8, "ld.global", volatile)
 VISG_LD8(ld8_once, "ld.global.nc", volatile) // the same, not merged with an earlier load of the address
 VISG_LD8(ld8_cg, "ld.global.cg", volatile)   // through L2: data another CTA wrote earlier in the launch
 #undef VISG_LD8
+__device__ __forceinline__ float4 ld4(const float4* p) {  // 16 bytes, not merged with an earlier load
+    float4 r;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
 __device__ __forceinline__ void st8(float4* p, float4 a, float4 b) {
     asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
                  "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(p)

@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(RENDER_THREADS) k_render_pos(const float4* __r
                                                                float4* __restrict__ pos4) {
     const int64_t i = (int64_t)blockIdx.x * RENDER_THREADS + threadIdx.x;
     if (i >= n) return;
-    const float4 s = __ldg(st + 2 * i);
+    const float4 s = __ldg(st + rec_at(i));
     pos4[i] = make_float4(s.x, s.y, s.z, 1.0f);
 }
 
@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(RENDER_THREADS) k_face_normals(const float4* _
     const int64_t f = (int64_t)blockIdx.x * RENDER_THREADS + threadIdx.x;
     if (f >= nf) return;
     const uint32_t a = __ldg(faces + 3 * f), b = __ldg(faces + 3 * f + 1), c = __ldg(faces + 3 * f + 2);
-    const f3 p0 = xyz(__ldg(st + 2 * (int64_t)a));
-    const f3 p1 = xyz(__ldg(st + 2 * (int64_t)b));
-    const f3 p2 = xyz(__ldg(st + 2 * (int64_t)c));
+    const f3 p0 = xyz(__ldg(st + rec_at((int64_t)a)));
+    const f3 p1 = xyz(__ldg(st + rec_at((int64_t)b)));
+    const f3 p2 = xyz(__ldg(st + rec_at((int64_t)c)));
     const f3 nrm = normalize(cross(sub(p1, p0), sub(p2, p0)));
     fn[3 * f] = nrm.x;
     fn[3 * f + 1] = nrm.y;

@@ -217,12 +217,21 @@ __device__ __forceinline__ void wait_for_earlier_launches() {
 
 // Vertex records (about half the neighbour reads hit L1: rows of a grid share most
 // neighbours).
-struct GlobalRecords {
+struct GlobalRecords {  // by record index (rec_at)
     const float4* p;
-    __device__ __forceinline__ float4 r0(int j) const { return p[2 * j]; }
-    __device__ __forceinline__ float4 r1(int j) const { return p[2 * j + 1]; }
-    __device__ __forceinline__ f4x2 both(int j) const { return ld8(p + 2 * j); }
+    __device__ __forceinline__ float4 r0(uint32_t r) const { return p[r]; }
+    __device__ __forceinline__ float4 r1(uint32_t r) const { return p[r + 32u]; }
 };
+// a record read anew (not merged with an earlier read of it)
+__device__ __forceinline__ f4x2 ld_record(const float4* st, int i) {
+    const float4* const p = st + rec_at(i);
+    return f4x2{ld4(p), ld4(p + 32)};
+}
+__device__ __forceinline__ void st_record(float4* st, int i, float4 s0, float4 s1) {
+    float4* const p = st + rec_at(i);
+    p[0] = s0;
+    p[32] = s1;
+}
 
 // A row's sliced-ELL entries (entry e at p[32 e]): in global memory, or in the tile's
 // block that a TMA bulk copy staged in shared memory.
@@ -251,13 +260,13 @@ __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const floa
             const uint2 ea = ep[ea_at], eb = ep[eb_at];
             f4x2 ra, rb;
             if (FAST) {
-                ra.a = rec.r0((int)ea.x);
-                rb.a = rec.r0((int)eb.x);
+                ra.a = rec.r0(ea.x);
+                rb.a = rec.r0(eb.x);
                 ra.b = ra.a;
                 rb.b = rb.a;
             } else {
-                ra = rec.both((int)ea.x);
-                rb = rec.both((int)eb.x);
+                ra = f4x2{rec.r0(ea.x), rec.r1(ea.x)};
+                rb = f4x2{rec.r0(eb.x), rec.r1(eb.x)};
             }
             const fp2 kk = PERK ? pk2(__ldg(kp + 32 * ea_at), __ldg(kp + 32 * eb_at)) : k2;
             spring_pair<FAST>(x, vel, ra.a, ra.b, rb.a, rb.b, kk, __uint_as_float(ea.y), __uint_as_float(eb.y), kd2,
@@ -278,9 +287,8 @@ __device__ __forceinline__ f3 list_sum(const Rec& rec, const Ent& ep, const floa
     }
     for (; e < end; ++e) {
         const uint2 ea = ep[e];
-        const int ja = (int)ea.x;
         const float nk = PERK ? -__ldg(kp + 32 * e) : -k;
-        acc = add(acc, spring_force(x, vel, rec.r0(ja), rec.r1(ja), nk, __uint_as_float(ea.y), kd, eps3, drec, dt));
+        acc = add(acc, spring_force(x, vel, rec.r0(ea.x), rec.r1(ea.x), nk, __uint_as_float(ea.y), kd, eps3, drec, dt));
     }
     return acc;
 }
@@ -366,7 +374,7 @@ __device__ __forceinline__ void helper_query(const StepArgs& a, const int4 td, c
     float m = 0.0f, reach;
     f3 p = mk3(0.0f, 0.0f, 0.0f);
     if (mine && a.settled) {
-        const f4x2 rec = ld8(a.state_out + 2 * i);
+        const f4x2 rec = ld_record(a.state_out, i);
         const f3 q = step_ahead(a.p, rec, 2.0f, reach);
         if (!(rec.b.w > 4.0f * reach)) {
             p = q;
@@ -377,7 +385,7 @@ __device__ __forceinline__ void helper_query(const StepArgs& a, const int4 td, c
     __syncwarp();
     wait_for_earlier_launches();
     if (mine) {
-        const f4x2 rec = ld8(a.state_in + 2 * i);
+        const f4x2 rec = ld_record(a.state_in, i);
         const f3 q = step_ahead(a.p, rec, 1.0f, reach);
         if (rec.b.w > 2.0f * reach) {
             m = 0.0f;  // the cached answer will do
@@ -421,14 +429,15 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int garment
     const StepParams& P = a.p;
     const f3 grav = mk3(P.gx, P.gy, P.gz);
     const f3 eps3 = mk3(kFltEpsilon, kFltEpsilon, kFltEpsilon);
-    const float4 s0 = rec.r0(ii);
+    const uint32_t ri = rec_at(ii);
+    const float4 s0 = rec.r0(ri);
     const f3 x = mk3(s0.x, s0.y, s0.z);
     const uint2 cnt = __ldg(&a.vcount[ii]);
     const bool pinned = (cnt.y & PIN_BIT) != 0u;
     if (COLL && kPrefetchContact) {
-        // the record's flags word (the sector s0 came in): start the loads that a cached
+        // the record's flags word: start the loads that a cached
         // contact answer and a stored normal need after the spring sum
-        const uint32_t fl0 = __float_as_uint(reinterpret_cast<const float*>(a.state_in + 2 * ii + 1)[2]);
+        const uint32_t fl0 = __float_as_uint(reinterpret_cast<const float*>(a.state_in + ri + 32)[2]);
         const BvhRoot* const rt = a.roots + (garment & TILE_GARMENT);
         if (fl0 & FLAG_LEAF_CACHED) prefetch_contact(rt->leaves + 2 * (fl0 >> LEAF_SHIFT));
         if (fl0 & FLAG_HAS_NORMAL) prefetch_contact(a.normal + ii);
@@ -455,7 +464,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int garment
         const float* kp = perk ? a.sellk + sb : nullptr;
         f3 vel = mk3(0.0f, 0.0f, 0.0f);
         if (!KD0 || damped) {
-            const float4 s1 = rec.r1(ii);
+            const float4 s1 = rec.r1(ri);
             const f3 rv = mk3(s0.w, s1.x, s1.y);  // v, or D = x - x_old with drec
             vel = P.drec ? divs(rv, P.dt) : rv;
         }
@@ -478,7 +487,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int garment
     if constexpr (!HELP) after_sum();
     if (moves) {
         // the record again (a second read of a line this thread has just read)
-        const f4x2 own = ld8(a.state_in + 2 * ii);
+        const f4x2 own = ld_record(a.state_in, ii);
         const float4 r0 = own.a, r1 = own.b;
         const f3 rv = mk3(r0.w, r1.x, r1.y);  // v, or D = x - x_old with drec
         flags = __float_as_uint(r1.z);
@@ -495,7 +504,7 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int garment
         // x - x_old: from the record (drec), else from x_old in the other buffer
         f3 xo = x, d = rv;
         if (!P.drec) {
-            if (!(flags & FLAG_XO_IS_X)) xo = xyz(a.state_out[2 * ii]);
+            if (!(flags & FLAG_XO_IS_X)) xo = xyz(a.state_out[rec_at(ii)]);
             d = sub(x, xo);
         }
         f3 np = mk3(0.0f, 0.0f, 0.0f);
@@ -583,8 +592,8 @@ __device__ __forceinline__ void vertex_step(const StepArgs& a, const int garment
         untamed = P.drec ? !tame_d(xn, dn, P.dmax) : !tame(xn, vn);
         const uint32_t fl = (has_n ? FLAG_HAS_NORMAL : 0u) | (xo_is_x ? FLAG_XO_IS_X : 0u) |
                             (skin > 0.0f ? leaf_bits : 0u);
-        st8(a.state_out + 2 * i, make_float4(xn.x, xn.y, xn.z, vn.x),
-            make_float4(vn.y, vn.z, __uint_as_float(fl), skin > 0.0f ? skin : 0.0f));
+        st_record(a.state_out, i, make_float4(xn.x, xn.y, xn.z, vn.x),
+                  make_float4(vn.y, vn.z, __uint_as_float(fl), skin > 0.0f ? skin : 0.0f));
         if (has_n) a.normal[i] = make_float4(nn.x, nn.y, nn.z, 0.0f);
         if (check) {
             const float dd = fmaxf(fabsf(__fsub_rn(xn.x, x.x)),
@@ -810,7 +819,7 @@ __global__ void __launch_bounds__(COLLIDE_BLOCK) k_collide(const StepArgs a) {
     for (uint32_t k = blockIdx.x * COLLIDE_BLOCK + threadIdx.x; k < n; k += gridDim.x * COLLIDE_BLOCK) {
         const int2 c = a.cand[k];
         const BvhRoot* const rt = a.roots + c.y;
-        const f4x2 rec = ld8(a.state_out + 2 * c.x);
+        const f4x2 rec = ld_record(a.state_out, c.x);
         float4 s0 = rec.a, s1 = rec.b;
         f3 xn = mk3(s0.x, s0.y, s0.z);
         float m = __int_as_float(0x7f800000);  // +inf
@@ -840,7 +849,7 @@ __global__ void __launch_bounds__(COLLIDE_BLOCK) k_collide(const StepArgs a) {
             skin = 0.0f;
             fl &= 7u & ~FLAG_LEAF_CACHED;
         }
-        st8(a.state_out + 2 * c.x, s0, make_float4(s1.x, s1.y, __uint_as_float(fl), skin));
+        st_record(a.state_out, c.x, s0, make_float4(s1.x, s1.y, __uint_as_float(fl), skin));
     }
 }
 
@@ -984,74 +993,77 @@ __global__ void k_query(BvhView bv, const float* __restrict__ pts, int n, int* l
     }
 }
 
-__global__ void k_unpack_positions(const float4* st, int64_t n, float* out) {
+__global__ void k_unpack_positions(const float4* st, int64_t v0, int64_t n, float* out) {
     wait_for_earlier_launches();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 s0 = st[2 * i];
+    const float4 s0 = st[rec_at(v0 + i)];
     out[3 * i] = s0.x;
     out[3 * i + 1] = s0.y;
     out[3 * i + 2] = s0.z;
 }
 
 __global__ void k_unpack_state(const float4* __restrict__ st, const float4* __restrict__ other,
-                               const float4* __restrict__ nr, int64_t n, float* x, float* xo, float* nrm) {
+                               const float4* __restrict__ nr, int64_t v0, int64_t n, float* x, float* xo, float* nrm) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 s0 = st[2 * i], s1 = st[2 * i + 1];
+    const int64_t r = rec_at(v0 + i);
+    const float4 s0 = st[r], s1 = st[r + 32];
     const uint32_t fl = __float_as_uint(s1.z);
     if (x) { x[3 * i] = s0.x; x[3 * i + 1] = s0.y; x[3 * i + 2] = s0.z; }
     if (xo) {
-        const float4 o = (fl & FLAG_XO_IS_X) ? s0 : other[2 * i];
+        const float4 o = (fl & FLAG_XO_IS_X) ? s0 : other[r];
         xo[3 * i] = o.x; xo[3 * i + 1] = o.y; xo[3 * i + 2] = o.z;
     }
     if (nrm) {
-        const float4 v = (fl & FLAG_HAS_NORMAL) ? nr[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 v = (fl & FLAG_HAS_NORMAL) ? nr[v0 + i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         nrm[3 * i] = v.x; nrm[3 * i + 1] = v.y; nrm[3 * i + 2] = v.z;
     }
 }
 
 // x == nullptr keeps x, etc.  x_old is written into the other buffer and v is
 // recomputed as (x - x_old) / dt; a vertex has a stored normal iff it is non-zero.
-__global__ void k_pack_state(float4* st, float4* other, float4* nr, int64_t n, const float* x, const float* xo,
-                             const float* nrm, float dt, int drec, float dmax, uint32_t* wild) {
+__global__ void k_pack_state(float4* st, float4* other, float4* nr, int64_t v0, int64_t n, const float* x,
+                             const float* xo, const float* nrm, float dt, int drec, float dmax, uint32_t* wild) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float4 s0 = st[2 * i], s1 = st[2 * i + 1];
+    const int64_t r = rec_at(v0 + i);
+    float4 s0 = st[r], s1 = st[r + 32];
     uint32_t fl = __float_as_uint(s1.z) & (FLAG_HAS_NORMAL | FLAG_XO_IS_X);  // no cached answer
     const f3 x0 = mk3(s0.x, s0.y, s0.z);
-    const f3 xo0 = (fl & FLAG_XO_IS_X) ? x0 : xyz(other[2 * i]);
+    const f3 xo0 = (fl & FLAG_XO_IS_X) ? x0 : xyz(other[r]);
     const f3 xv = x ? mk3(x[3 * i], x[3 * i + 1], x[3 * i + 2]) : x0;
     const f3 xov = xo ? mk3(xo[3 * i], xo[3 * i + 1], xo[3 * i + 2]) : xo0;
     const f3 v = drec ? sub(xv, xov) : divs(sub(xv, xov), dt);  // what the record carries
     if (nrm) {
         const float a = nrm[3 * i], b = nrm[3 * i + 1], c = nrm[3 * i + 2];
         const bool h = a != 0.0f || b != 0.0f || c != 0.0f;
-        nr[i] = make_float4(a, b, c, 0.0f);
+        nr[v0 + i] = make_float4(a, b, c, 0.0f);
         fl = (fl & ~FLAG_HAS_NORMAL) | (h ? FLAG_HAS_NORMAL : 0u);
     }
     fl &= ~FLAG_XO_IS_X;
-    other[2 * i] = make_float4(xov.x, xov.y, xov.z, 0.0f);
-    st[2 * i] = make_float4(xv.x, xv.y, xv.z, v.x);
-    st[2 * i + 1] = make_float4(v.y, v.z, __uint_as_float(fl), 0.0f);
+    other[r] = make_float4(xov.x, xov.y, xov.z, 0.0f);
+    st[r] = make_float4(xv.x, xv.y, xv.z, v.x);
+    st[r + 32] = make_float4(v.y, v.z, __uint_as_float(fl), 0.0f);
     if (drec ? !tame_d(xv, v, dmax) : !tame(xv, v)) atomicOr(wild, 1u);
 }
 
 __global__ void k_check_tame(const float4* __restrict__ st, int64_t n, uint32_t* wild) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 s0 = st[2 * i], s1 = st[2 * i + 1];
+    const int64_t r = rec_at(i);
+    const float4 s0 = st[r], s1 = st[r + 32];
     if (!tame(mk3(s0.x, s0.y, s0.z), mk3(s0.w, s1.x, s1.y))) atomicOr(wild, 1u);
 }
 
 __global__ void k_clear_margin(float4* st, int64_t v0, int64_t v1) {
     const int64_t i = v0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < v1) reinterpret_cast<float*>(st + 2 * i + 1)[3] = 0.0f;
+    if (i < v1) reinterpret_cast<float*>(st + rec_at(i) + 32)[3] = 0.0f;
 }
 
 __global__ void k_count_contacts(const float4* __restrict__ st, int64_t n, unsigned long long* count) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool c = i < n && (__float_as_uint(st[2 * i + 1].z) & FLAG_HAS_NORMAL);
+    const bool c = i < n && (__float_as_uint(st[rec_at(i) + 32].z) & FLAG_HAS_NORMAL);
     const unsigned m = __ballot_sync(0xffffffffu, c);
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, (unsigned long long)__popc(m));
 }
@@ -1062,12 +1074,12 @@ __global__ void k_set_vertices(float4* st, const uint32_t* __restrict__ idx, con
                                float dt, uint32_t* wild) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const int64_t v = idx[k];
+    const int64_t v = rec_at((int64_t)idx[k]);
     const f3 p = mk3(xyz3[3 * k], xyz3[3 * k + 1], xyz3[3 * k + 2]);
     const f3 vel = divs(sub(p, p), dt);
-    const uint32_t fl = (__float_as_uint(st[2 * v + 1].z) & FLAG_HAS_NORMAL) | FLAG_XO_IS_X;
-    st[2 * v] = make_float4(p.x, p.y, p.z, vel.x);
-    st[2 * v + 1] = make_float4(vel.y, vel.z, __uint_as_float(fl), 0.0f);
+    const uint32_t fl = (__float_as_uint(st[v + 32].z) & FLAG_HAS_NORMAL) | FLAG_XO_IS_X;
+    st[v] = make_float4(p.x, p.y, p.z, vel.x);
+    st[v + 32] = make_float4(vel.y, vel.z, __uint_as_float(fl), 0.0f);
     if (!tame(p, vel)) atomicOr(wild, 1u);
 }
 
@@ -1169,15 +1181,15 @@ cudaError_t launch_query(BvhView v, const float* pts, int n, int* leaf, int* ins
     return cudaGetLastError();
 }
 
-cudaError_t launch_unpack_positions(const float4* state, int64_t n, float* out, cudaStream_t s) {
+cudaError_t launch_unpack_positions(const float4* state, int64_t v0, int64_t n, float* out, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    return launch_after(k_unpack_positions, (int)grid_for(n, 256), 256, 0, s, true, state, n, out);
+    return launch_after(k_unpack_positions, (int)grid_for(n, 256), 256, 0, s, true, state, v0, n, out);
 }
 
-cudaError_t launch_unpack_state(const float4* state, const float4* other, const float4* normal, int64_t n, float* x,
-                                float* xo, float* nrm, cudaStream_t s) {
+cudaError_t launch_unpack_state(const float4* state, const float4* other, const float4* normal, int64_t v0, int64_t n,
+                                float* x, float* xo, float* nrm, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_unpack_state<<<grid_for(n, 256), 256, 0, s>>>(state, other, normal, n, x, xo, nrm);
+    k_unpack_state<<<grid_for(n, 256), 256, 0, s>>>(state, other, normal, v0, n, x, xo, nrm);
     return cudaGetLastError();
 }
 
@@ -1206,10 +1218,12 @@ cudaError_t launch_set_vertices(float4* state, const uint32_t* idx, const float*
     return cudaGetLastError();
 }
 
-cudaError_t launch_pack_state(float4* state, float4* other, float4* normal, int64_t n, const float* x, const float* xo,
+cudaError_t launch_pack_state(float4* state, float4* other, float4* normal, int64_t v0, int64_t n, const float* x,
+                              const float* xo,
                               const float* nrm, float dt, int drec, float dmax, uint32_t* wild, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_pack_state<<<grid_for(n, 256), 256, 0, s>>>(state, other, normal, n, x, xo, nrm, dt, drec, dmax, wild);
+    k_pack_state<<<grid_for(n, 256), 256, 0, s>>>(state, other, normal, v0, n, x, xo, nrm, dt, drec,
+                                                 dmax, wild);
     return cudaGetLastError();
 }
 
