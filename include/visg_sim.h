@@ -68,7 +68,7 @@ typedef struct VisgParams {
                                 garment of at most 512 vertices per SM is always stepped fused
                                 (collision_margin on): helper warps of the same kernel answer
                                 its queries beside the spring sums.                           */
-    int32_t stage_neighbours; /* 1: each tile's block of spring entries is staged in shared
+    int32_t stage_neighbours; /* 1: each slice's spring entries are staged in shared
                                 memory by TMA bulk copies, 0: read through the L1 (default);
                                 same results.  visg_autotune / visg_batch_autotune may change it. */
     int32_t collision_margin; /* 1: each vertex caches its last first-hit query's answer with
@@ -423,7 +423,7 @@ int visg_mesh_rotate(float* xyz, int32_t n, float angle_degrees, int32_t axis);
 #define VISG_NOALLOC_SCRATCH_BYTES (9u * 1024u * 1024u)
 /* Self-test of the device-side failure detection: runs, on the current device, one
  * kernel that waits on an mbarrier phase nothing completes (the wait of the step's
- * shared-memory staging ring), one that looks back at a radix-sort status word
+ * shared-memory stage), one that looks back at a radix-sort status word
  * nothing publishes (the wait of the LBVH's radix passes), and one that waits at a
  * grid barrier for CTAs that never arrive (the wait between the LBVH build's
  * phases).  Each wait is bounded and must give up, record the timeout and return;

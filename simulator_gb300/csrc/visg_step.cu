@@ -3,11 +3,11 @@
 // k_step is the reference's `verlet` kernel (src/verlet.cu:129-161) rebuilt for
 // GB300: one thread per vertex, persistent CTAs walking a tile table (a tile is
 // BLOCK consecutive vertices of one garment, so one launch covers any number of
-// garments of uneven size), 32-byte interleaved state records (one float4 load per
-// spring neighbour when spring damping is zero, two otherwise), springs of all
-// lists merged into one sliced-ELL table of 8-byte entries (optionally staged per
-// tile in shared memory by TMA bulk copies while the previous tile is computed)
-// summed list by list with the list's stiffness uniform across the loop, the previous
+// garments of uneven size) or persistent warps walking slices of 32 vertices, state
+// records in two 16-byte halves (one float4 load per spring neighbour when spring damping
+// is zero, two otherwise), springs of all lists merged into one sliced-ELL table of 8-byte
+// entries (optionally staged per slice in shared memory by TMA bulk copies while the warp
+// finishes the slice before) summed list by list with the list's stiffness uniform across the loop, the previous
 // contact normal read only for vertices that had a contact, and the collision
 // (collision_response_projection, verlet.cu:24-50) fused behind a warp vote on the
 // body's root box.  Arithmetic follows the reference operation by operation with
@@ -1057,7 +1057,7 @@ inline unsigned grid_for(int64_t n, int b) { return (unsigned)((n + b - 1) / b);
 }  // namespace
 
 namespace {
-// Self-test of the staging ring's bounded wait: thread 0 waits on the phase of an
+// Self-test of the staged copies' bounded wait: thread 0 waits on the phase of an
 // mbarrier that nothing arrives on; the wait gives up after kWaitNs and the kernel
 // records ERR_TIMEOUT and returns (no copy is in flight).
 __global__ void k_selftest_mbar_wait(int* err) {
