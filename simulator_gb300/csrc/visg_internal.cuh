@@ -134,7 +134,7 @@ struct BvhBuffers {
     Node* nodes = nullptr;       // nt-1
     float4* leaves = nullptr;    // 2*nt
     int2* range = nullptr;       // nt-1 leaf range of each internal node
-    // Summaries of the chunks (512 sorted positions each) for the nodes whose leaf range spans chunks
+    // Summaries of the chunks (up to 512 sorted positions each) for the nodes whose leaf range spans chunks
     int* cmin = nullptr;         // min delta over the boundaries that end the chunk's unjoined subtrees
     float4* cbox = nullptr;      // 2 per chunk: union of its leaf boxes
     int2* srec = nullptr;        // 32 per chunk: suffix-minimum boundaries {position, delta}, right to left
@@ -143,7 +143,7 @@ struct BvhBuffers {
     float4* pbox = nullptr;      // 2 per record: union of the chunk's leaves up to the boundary
     uint32_t* rcnt = nullptr;    // 2 per chunk: prefix record count | nodes in `top` << 16; suffix record count
     int2* top = nullptr;         // 64 per chunk: {boundary, delta} of the nodes that span chunks
-    int chunks = 0;
+    int chunks = 0, chunk_len = 0;
     BvhRoot* root = nullptr;
     uint32_t* scratch = nullptr; // radix histograms, look-back status words, tile counters (the build clears them)
     size_t scratch_words = 0;

@@ -65,7 +65,7 @@ namespace visg {
 
 namespace {
 
-constexpr int RB = 512;        // threads per CTA: one chunk of leaves, one leaf per thread
+constexpr int RB = 512;        // threads per CTA: one chunk of leaves at most, one leaf per thread
 constexpr int RW = RB / 32;    // warps per CTA
 constexpr int SORT_ITEMS = 4;
 constexpr int SORT_TILE = RB * SORT_ITEMS;  // 2048 keys per radix tile
@@ -206,7 +206,7 @@ struct RebuildArgs {
     uint32_t* ucnt;    // per chunk: its leaves, with CNT_READY once known
     uint32_t* chg;     // [0] changed codes, then {triangle, new code, old code} x CHG_CAP
     uint32_t* sync;    // [0] barrier arrivals, [1] CTAs finished (both 0 between launches)
-    int chunks;
+    int chunks, chunk_len;
     int* err;
     float4* margin_state;  // cloth records whose query-cache margins the moved body voids
     int64_t m0, m1;        // (vertices [m0, m1): their margin words are cleared)
@@ -909,7 +909,7 @@ __device__ __forceinline__ int far_leaf(int w) { return w & 0xffff; }
 __device__ __forceinline__ int far_delta(int w) { return (w >> 16) - 1; }
 
 // De-duplication, bottom-up build of the chunk-local nodes, and the chunk summary.  A
-// chunk is RB positions [p0, p0 + m) of the sorted list; its leaves are the positions
+// chunk is at most RB positions [p0, p0 + m) of the sorted list (chunk_length); its leaves are the positions
 // whose code differs from the one before (remove_redundant, Utilities.h:35-55: the first
 // triangle of every code).  The chunk works in its own leaf numbers; where its leaves
 // begin in the whole is the sum of the counts that the chunks before it publish, read
@@ -934,7 +934,7 @@ __device__ __forceinline__ int far_delta(int w) { return (w >> 16) - 1; }
 __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, const uint32_t* V, BuildSmem& S) {
     const ChunkView& cv = A.cv;
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nt = A.nt, p0 = chunk * RB, m = min(RB, nt - p0), p = p0 + tid;
+    const int nt = A.nt, p0 = chunk * A.chunk_len, m = min(A.chunk_len, nt - p0), p = p0 + tid;
     const bool in = tid < m;
     uint32_t k = 0u, t = 0u;
     float4 lo = ident_lo(), hi = ident_hi();
@@ -1485,6 +1485,20 @@ int resident_ctas() {
     return cached[dev];
 }
 
+// Positions per chunk of the build.  Two CTAs an SM take the chunks in turn, so the chunks of
+// the rounds that RB positions would need are made equal: 327,680 triangles are 640 chunks
+// of 512, two rounds and 32 chunks more, or 854 of 384 (rebuild 75.7 -> 72.2 us; of 256, 88.5:
+// four rounds).  A small body's are no shorter than 256 (19,584 triangles: 512 22.2 us, 256
+// 20.9, 128 22.7, its spanning nodes take what the build gains), and a body whose summaries
+// would no longer fit the spanning-node phase's shared memory for it keeps them there.
+int chunk_length(int nt) {
+    constexpr int kResident = 2 * SPREAD_CTAS, kLeast = 256;
+    const int rounds = cdiv(cdiv(nt, RB), kResident);
+    int len = std::max(cdiv(nt, rounds * kResident), kLeast);
+    if (nt <= TOP_STAGED * RB) len = std::max(len, cdiv(nt, TOP_STAGED));
+    return std::min(RB, (len + 31) / 32 * 32);
+}
+
 }  // namespace
 
 void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool own_root) {
@@ -1492,7 +1506,8 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool own_root) {
     nt = nt_;
     has_normals = normals;
     tiles_sort = nt > 0 ? cdiv(nt, SORT_TILE) : 0;
-    chunks = cdiv(std::max(nt, 1), RB);
+    chunk_len = chunk_length(std::max(nt, 1));
+    chunks = cdiv(std::max(nt, 1), chunk_len);
     // a chunk per CTA at most, but for a small body enough CTAs that the phases before
     // the build spread over the SMs
     max_ctas = std::max(chunks, std::min(SPREAD_CTAS, cdiv(std::max(nt, 1), RB / 4)));
@@ -1578,6 +1593,7 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.bcnt = b.bcnt;
     A.bkey = b.bkey;
     A.chunks = b.chunks;
+    A.chunk_len = b.chunk_len;
     A.err = d_err;
     const int grid = std::min(res, b.max_ctas);
     void* args[] = {&A};
