@@ -242,7 +242,6 @@ struct Engine {
         free_faces();
         if (rb.h_err) cudaFreeHost(rb.h_err);
         destroy_graphs();
-        if (d_sv_idx) cudaFree(d_sv_idx);
         if (h_sv) cudaFreeHost(h_sv);
         if (sv_done) cudaEventDestroy(sv_done);
         free_adjoint();
@@ -822,10 +821,8 @@ struct Engine {
         return VISG_OK;
     }
 
-    // many vertices at once: host arrays staged into a pinned buffer, one H2D, one scatter
-    uint32_t* d_sv_idx = nullptr;
-    float* d_sv_xyz = nullptr;
-    char* h_sv = nullptr;
+    // many vertices at once: host arrays packed into a page-locked buffer that the kernel reads
+    float4* h_sv = nullptr;  // {vertex, position}, which the kernel reads
     int sv_cap = 0;
     cudaEvent_t sv_done = nullptr;
     int set_vertices(const uint32_t* idx, const float* xyz, int n) {
@@ -836,24 +833,22 @@ struct Engine {
         if (n == 0) return VISG_OK;
         if (n > sv_cap) {
             if (sv_done) CU(cudaEventSynchronize(sv_done));
-            cudaFree(d_sv_idx);
             cudaFreeHost(h_sv);
-            d_sv_idx = nullptr;
             h_sv = nullptr;
-            int cap = std::max(n, 1024);
-            CU(cudaMalloc((void**)&d_sv_idx, (size_t)cap * 16));
-            d_sv_xyz = (float*)(d_sv_idx + cap);
-            CU(cudaHostAlloc((void**)&h_sv, (size_t)cap * 16, cudaHostAllocDefault));
+            sv_cap = 0;
+            const int cap = std::max(n, 1024);
+            CU(cudaHostAlloc((void**)&h_sv, (size_t)cap * sizeof(float4), cudaHostAllocMapped));
             if (!sv_done) CU(cudaEventCreateWithFlags(&sv_done, cudaEventDisableTiming));
             sv_cap = cap;
         }
-        CU(cudaEventSynchronize(sv_done));  // the previous upload has left the staging buffer
-        std::memcpy(h_sv, idx, (size_t)n * 4);
-        std::memcpy(h_sv + (size_t)sv_cap * 4, xyz, (size_t)n * 12);
-        CU(cudaMemcpyAsync(d_sv_idx, h_sv, (size_t)n * 4, cudaMemcpyHostToDevice, stream));
-        CU(cudaMemcpyAsync(d_sv_xyz, h_sv + (size_t)sv_cap * 4, (size_t)n * 12, cudaMemcpyHostToDevice, stream));
+        CU(cudaEventSynchronize(sv_done));  // the kernel of the previous call has read the staging buffer
+        for (int k = 0; k < n; ++k) {
+            float v;
+            std::memcpy(&v, &idx[k], 4);
+            h_sv[k] = make_float4(v, xyz[3 * (size_t)k], xyz[3 * (size_t)k + 1], xyz[3 * (size_t)k + 2]);
+        }
+        CU(launch_set_vertices(d_state[cur], h_sv, n, p.dt, d_wild, stream));
         CU(cudaEventRecord(sv_done, stream));
-        CU(launch_set_vertices(d_state[cur], d_sv_idx, d_sv_xyz, n, p.dt, d_wild, stream));
         return VISG_OK;
     }
 

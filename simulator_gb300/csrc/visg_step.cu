@@ -1038,13 +1038,17 @@ __global__ void k_count_contacts(const float4* __restrict__ st, int64_t n, unsig
 }
 
 // update_vertex (simulation.cu:253-257): x = x_old = p, so v = (p - p) / dt; the
-// stored contact normal is kept
-__global__ void k_set_vertices(float4* st, const uint32_t* __restrict__ idx, const float* __restrict__ xyz3, int n,
-                               float dt, uint32_t* wild) {
+// stored contact normal is kept.  moves: {vertex, p} in page-locked host memory, read from
+// there, before the wait for earlier launches: two copies in the stream before it took longer
+// than the kernel (dragged 64 x 64 sheet 33 -> 28 us a frame, six frames
+// of 24 garments with their read-back, whose copies shared the engines, 371 -> 285).
+__global__ void k_set_vertices(float4* st, const float4* moves, int n, float dt, uint32_t* wild) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const float4 m = k < n ? __ldcv(moves + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    wait_for_earlier_launches();
     if (k >= n) return;
-    const int64_t v = rec_at((int64_t)idx[k]);
-    const f3 p = mk3(xyz3[3 * k], xyz3[3 * k + 1], xyz3[3 * k + 2]);
+    const int64_t v = rec_at((int64_t)__float_as_uint(m.x));
+    const f3 p = mk3(m.y, m.z, m.w);
     const f3 vel = divs(sub(p, p), dt);
     const uint32_t fl = (__float_as_uint(st[v + 32].z) & FLAG_HAS_NORMAL) | FLAG_XO_IS_X;
     st[v] = make_float4(p.x, p.y, p.z, vel.x);
@@ -1180,11 +1184,9 @@ cudaError_t launch_count_contacts(const float4* state, int64_t n, unsigned long 
     return cudaGetLastError();
 }
 
-cudaError_t launch_set_vertices(float4* state, const uint32_t* idx, const float* xyz, int n, float dt, uint32_t* wild,
-                                cudaStream_t s) {
+cudaError_t launch_set_vertices(float4* state, const float4* moves, int n, float dt, uint32_t* wild, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_set_vertices<<<grid_for(n, 256), 256, 0, s>>>(state, idx, xyz, n, dt, wild);
-    return cudaGetLastError();
+    return launch_after(k_set_vertices, (int)grid_for(n, 256), 256, 0, s, true, state, moves, n, dt, wild);
 }
 
 cudaError_t launch_pack_state(float4* state, float4* other, float4* normal, int64_t v0, int64_t n, const float* x,
