@@ -142,7 +142,7 @@ int visg_update_body_device(VisgSim* sim, const float* d_body_xyz, const float* 
 int visg_set_vertex(VisgSim* sim, uint32_t idx, const float xyz[3]);
 
 /* update_vertex for many vertices in one call: idx[k] gets x = x_old = xyz[3k..3k+2].
- * One host-to-device copy and one scatter kernel, asynchronous on the stream (the
+ * One scatter kernel that reads a page-locked copy of the arrays, asynchronous on the stream (the
  * host arrays are staged before the call returns).  Duplicate indices: the last wins. */
 int visg_set_vertices(VisgSim* sim, const uint32_t* idx, const float* xyz, int32_t n);
 
