@@ -116,12 +116,13 @@ __device__ __forceinline__ int first_hit(const Node* nodes, int node, int budget
     return ~node;
 }
 
-// The whole first-hit query of one body (root box, single leaf, walk) with its margin.
+// The whole first-hit query of one body (root box, single leaf, walk) with its margin.  A NaN
+// is in no box, but its answer holds for no other point: margin 0.
 __device__ __forceinline__ int query_margin(const BvhRoot* rt, f3 p, int* err, float& m) {
     const f4x2 box = ld8(&rt->top_lo);
     const float4 lo = box.a, hi = box.b;
     if (!in_box(p, lo, hi)) {  // also a NaN
-        m = fminf(m, box_gap(p, lo, hi));
+        m = isnan(p.x) || isnan(p.y) || isnan(p.z) ? 0.0f : fminf(m, box_gap(p, lo, hi));
         return -1;
     }
     const int nl = rt->n_leaves;
@@ -349,7 +350,7 @@ __device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0,
 // With `settled` (no tree has been rebuilt since the launch before) the walk begins already
 // while that launch runs, before the wait: from the records it reads, which nobody writes
 // until this launch does, two steps ahead.  Whatever those records are, an answer is only
-// taken over within its margin.
+// taken over within its margin (none if they lead to a NaN).
 __device__ __forceinline__ f3 step_ahead(const StepParams& P, const f4x2& rec, float steps, float& reach) {
     f3 d = mk3(rec.a.w, rec.b.x, rec.b.y);  // D, or v
     if (!P.drec) d = mul(d, P.dt);

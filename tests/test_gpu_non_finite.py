@@ -1,0 +1,45 @@
+"""Simulations that hold NaNs for a while, against the float oracle bit for bit: vertices
+that had gone to NaN are put back and meet their body as if they had never left."""
+import numpy as np
+import pytest
+
+import simulator_gb300 as vs
+from oracle.ffi import OracleSim
+from simulator_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def scene(physics, side=64):
+    cloth = scenes.grid_cloth(side, 1.0, 0.0, pin_top_corners=False)
+    body = scenes.icosphere(3, 0.3, (0.0, -0.3003, 0.0))
+    if physics == "workload":
+        p = scenes.physics_params(4)
+    else:
+        p = vs.reference_params(3)
+        p.gravity[1] = -0.05
+        p.list_k[:] = (100.0, 60.0, 2.0, 0.0)
+    return cloth, body, p
+
+
+def assert_equal(gpu, oracle):
+    for a, b in zip(gpu.state(), oracle.state()):
+        assert np.array_equal(a, b.astype(np.float32), equal_nan=True)
+
+
+@pytest.mark.parametrize("calls", [[1] * 96, [16] * 6, [1, 95]])  # single steps, graphs, both
+@pytest.mark.parametrize("physics", ["workload", "reference"])
+def test_vertices_put_back(physics, calls):
+    cloth, body, p = scene(physics)
+    g = vs.Simulator(cloth.xyz, cloth.lists, body.xyz, body.tris, None, params=p)
+    o = OracleSim(p, cloth.xyz, cloth.lists, body.xyz, body.tris, None, prec=4)
+    everything = np.arange(len(cloth.xyz), dtype=np.uint32)
+    g.update_vertices(everything, np.full_like(cloth.xyz, np.nan))
+    g.simulate(3)  # both halves of the double-buffered state are NaN
+    assert np.isnan(g.positions()).all()
+    g.update_vertices(everything, cloth.xyz)
+    for n in calls:
+        g.simulate(n)
+        o.step(n)
+        assert_equal(g, o)
+    assert g.count_contacts() > 0
