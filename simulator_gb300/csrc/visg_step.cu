@@ -40,12 +40,20 @@ __device__ __forceinline__ bool in_box(f3 p, float4 lo, float4 hi) {  // BBox::i
     return (p.x >= lo.x && p.x <= hi.x) && (p.y >= lo.y && p.y <= hi.y) && (p.z >= lo.z && p.z <= hi.z);
 }
 
-// Upper bound of max_axis |a - b| (each difference rounded up).
+// the larger of two floats, NaN if either is (fmaxf drops a NaN)
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// Upper bound of max_axis |a - b| (each difference rounded up); NaN, which no margin covers,
+// if a coordinate is.
 __device__ __forceinline__ float disp_bound(f3 a, f3 b) {
-    const float dx = __fsub_ru(fmaxf(a.x, b.x), fminf(a.x, b.x));
-    const float dy = __fsub_ru(fmaxf(a.y, b.y), fminf(a.y, b.y));
-    const float dz = __fsub_ru(fmaxf(a.z, b.z), fminf(a.z, b.z));
-    return fmaxf(dx, fmaxf(dy, dz));
+    const float dx = max_nan(__fsub_ru(a.x, b.x), __fsub_ru(b.x, a.x));
+    const float dy = max_nan(__fsub_ru(a.y, b.y), __fsub_ru(b.y, a.y));
+    const float dz = max_nan(__fsub_ru(a.z, b.z), __fsub_ru(b.z, a.z));
+    return max_nan(dx, max_nan(dy, dz));
 }
 
 // Lower bounds (differences rounded down) of the L-infinity distance p can move

@@ -1,5 +1,6 @@
 """Simulations that hold NaNs for a while, against the float oracle bit for bit: vertices
-that had gone to NaN are put back and meet their body as if they had never left."""
+that had gone to NaN are put back and meet their body as if they had never left, and
+vertices that are going to NaN meet nothing."""
 import numpy as np
 import pytest
 
@@ -43,3 +44,23 @@ def test_vertices_put_back(physics, calls):
         o.step(n)
         assert_equal(g, o)
     assert g.count_contacts() > 0
+
+
+@pytest.mark.parametrize("bad", [(np.nan, np.nan, np.nan), (np.nan, 0.0, 0.0), (np.inf, 0.0, 0.0)])
+@pytest.mark.parametrize("physics", ["workload", "reference"])
+def test_vertices_going_to_nan(physics, bad):
+    cloth, body, p = scene(physics, 48)
+    g = vs.Simulator(cloth.xyz, cloth.lists, body.xyz, body.tris, None, params=p)
+    o = OracleSim(p, cloth.xyz, cloth.lists, body.xyz, body.tris, None, prec=4)
+    g.simulate(160)
+    o.step(160)
+    assert_equal(g, o)
+    touching = np.flatnonzero(np.abs(g.state()[2]).sum(1))
+    assert len(touching) > 4
+    v = int(touching[len(touching) // 2])
+    g.update_vertices([v], [bad])
+    o.set_vertex(v, np.array(bad, np.float32))
+    for _ in range(4):
+        g.simulate(1)
+        o.step(1)
+        assert_equal(g, o)
