@@ -1074,6 +1074,12 @@ struct Engine {
         auto put = [](float* dst, float4 lo, float4 hi) {
             dst[0] = lo.x; dst[1] = lo.y; dst[2] = lo.z; dst[3] = hi.x; dst[4] = hi.y; dst[5] = hi.z;
         };
+        // a leaf's empty axis is a NaN box's (the build leaves no NaN in the tree)
+        auto put_leaf = [&](float* dst, float4 lo, float4 hi) {
+            put(dst, lo, hi);
+            for (int k = 0; k < 3; ++k)
+                if (dst[k] > dst[k + 3]) dst[k] = dst[k + 3] = std::nanf("");
+        };
         for (int t = 0; t < T; ++t) {
             if (tri_codes) tri_codes[t] = codes[t];
             if (tri_boxes) put(tri_boxes + 6 * t, tb[2 * t], tb[2 * t + 1]);
@@ -1085,7 +1091,7 @@ struct Engine {
         if (root_box) put(root_box, rt.frame_lo, rt.frame_hi);
         if (Tp == 1) {
             if (parent_leaf) parent_leaf[0] = 0;
-            if (leaf_boxes) put(leaf_boxes, rt.top_lo, rt.top_hi);
+            if (leaf_boxes) put_leaf(leaf_boxes, rt.top_lo, rt.top_hi);
             return VISG_OK;
         }
         const int ni = Tp - 1;
@@ -1118,7 +1124,7 @@ struct Engine {
             if (la < 0) {
                 ca[k] = -(~la) - 1;
                 pl[~la] = k + 1;
-                put(&lb6[6 * (size_t)(~la)], nd[gg].a_lo, nd[gg].a_hi);
+                put_leaf(&lb6[6 * (size_t)(~la)], nd[gg].a_lo, nd[gg].a_hi);
             } else {
                 ca[k] = kidx[la] + 1;
                 pi[kidx[la]] = k + 1;
@@ -1127,7 +1133,7 @@ struct Engine {
             if (lbk < 0) {
                 cb[k] = -(~lbk) - 1;
                 pl[~lbk] = k + 1;
-                put(&lb6[6 * (size_t)(~lbk)], nd[gg].b_lo, nd[gg].b_hi);
+                put_leaf(&lb6[6 * (size_t)(~lbk)], nd[gg].b_lo, nd[gg].b_hi);
             } else {
                 cb[k] = kidx[lbk] + 1;
                 pi[kidx[lbk]] = k + 1;

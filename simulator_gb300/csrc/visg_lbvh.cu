@@ -932,6 +932,7 @@ __device__ __forceinline__ int far_delta(int w) { return (w >> 16) - 1; }
 //   * the chunk's min delta and leaf box union.
 // Two warps make the summary of at most 63 pieces, two per lane, from either end.
 __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, const uint32_t* V, BuildSmem& S) {
+    const float inf = __int_as_float(0x7f800000);
     const ChunkView& cv = A.cv;
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nt = A.nt, p0 = chunk * A.chunk_len, m = min(A.chunk_len, nt - p0), p = p0 + tid;
@@ -941,9 +942,12 @@ __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, 
     if (in) {
         k = __ldcg(K + p);
         t = min(__ldcg(V + p), (uint32_t)(nt - 1));
+        // A triangle whose corners are all NaN on an axis has a NaN box, which holds no point.
+        // As a leaf it is empty on that axis, so that the walks test boxes by their gaps;
+        // a union takes neither a NaN nor an empty axis in.
         const f4x2 b = ld8_cg(A.tri_box + 2 * t);
-        lo = b.a;
-        hi = b.b;
+        lo = make_float4(fminf(b.a.x, inf), fminf(b.a.y, inf), fminf(b.a.z, inf), 0.0f);
+        hi = make_float4(fmaxf(b.b.x, -inf), fmaxf(b.b.y, -inf), fmaxf(b.b.z, -inf), 0.0f);
     }
     // the counts of the chunks before (most are there by the time they are needed)
     uint32_t cw = tid < chunk ? ld_volatile(A.ucnt + tid) : CNT_READY;

@@ -59,6 +59,9 @@ __device__ __forceinline__ float disp_bound(f3 a, f3 b) {
 // Lower bounds (differences rounded down) of the L-infinity distance p can move
 // before the closed-box test (BBox::intersect) changes its answer: outside the box,
 // the largest per-axis gap; inside, the distance to the nearest face.
+// A rounded-down difference has the sign of the exact one (a difference of two floats is zero
+// only if they are equal), so a point is in the closed box exactly when its gap is not
+// positive, if neither has a NaN.  A tree's boxes have none (build_chunk).
 __device__ __forceinline__ float box_gap(f3 p, float4 lo, float4 hi) {
     return fmaxf(fmaxf(fmaxf(__fsub_rd(lo.x, p.x), __fsub_rd(p.x, hi.x)), fmaxf(__fsub_rd(lo.y, p.y), __fsub_rd(p.y, hi.y))),
                  fmaxf(__fsub_rd(lo.z, p.z), __fsub_rd(p.z, hi.z)));
@@ -67,12 +70,6 @@ __device__ __forceinline__ float box_inner(f3 p, float4 lo, float4 hi) {
     return fminf(fminf(fminf(__fsub_rd(p.x, lo.x), __fsub_rd(hi.x, p.x)), fminf(__fsub_rd(p.y, lo.y), __fsub_rd(hi.y, p.y))),
                  fminf(__fsub_rd(p.z, lo.z), __fsub_rd(hi.z, p.z)));
 }
-
-// The box test as one number: the largest signed gap, rounded down.  A rounded-down
-// difference has the sign of the exact one (a difference of two floats is zero only if they
-// are equal), so a point without NaN is in the closed box exactly when this is not positive;
-// outside it is box_gap.
-__device__ __forceinline__ float box_side(f3 p, float4 lo, float4 hi) { return box_gap(p, lo, hi); }
 
 // D_BVH::intersect semantics: children tested pairwise; an overlapping leaf child is
 // returned before any descent (A before B); both internal -> descend A, push B.
@@ -104,7 +101,7 @@ __device__ __forceinline__ int first_hit(const Node* nodes, int node, int budget
         stack[sp] = top;
         const int below = stack[max(sp - 1, 0)];
         const int la = __float_as_int(a.a.w), lb = __float_as_int(b.a.w);
-        const float ga = box_side(p, a.a, a.b), gb = box_side(p, b.a, b.b);
+        const float ga = box_gap(p, a.a, a.b), gb = box_gap(p, b.a, b.b);
         const bool in_a = !(ga > 0.0f), in_b = !(gb > 0.0f);
         hit_a = in_a && la < 0;
         const bool hit_b = in_b && lb < 0 && !hit_a;

@@ -1,6 +1,6 @@
-"""Simulations that hold NaNs for a while, against the float oracle bit for bit: vertices
-that had gone to NaN are put back and meet their body as if they had never left, and
-vertices that are going to NaN meet nothing."""
+"""Simulations that hold NaNs, against the float oracle bit for bit: vertices that had gone
+to NaN are put back and meet their body as if they had never left, vertices that are going
+to NaN meet nothing, and triangles whose corners are NaN are met by nothing."""
 import numpy as np
 import pytest
 
@@ -64,3 +64,61 @@ def test_vertices_going_to_nan(physics, bad):
         g.simulate(1)
         o.step(1)
         assert_equal(g, o)
+
+
+def broken_body(seed, inf=False, partly=False):
+    """A sphere of separate triangles; of 40 % of them all corners are NaN on one axis or on
+    all (with `inf`, infinite instead), with `partly` also a single one."""
+    b = scenes.icosphere(4, 0.3, (0.0, -0.3003, 0.0))
+    rng = np.random.default_rng(seed)
+    v = b.xyz[b.tris].copy()
+    for t in np.flatnonzero(rng.random(len(v)) < 0.4):
+        bad = rng.choice([np.inf, -np.inf]) if inf else np.nan
+        axes = slice(None) if rng.random() < 0.3 else rng.integers(3)
+        if not partly or rng.random() < 0.8:
+            v[t, :, axes] = bad
+        else:
+            v[t, rng.integers(3), axes] = bad
+    return v.reshape(-1, 3), np.arange(3 * len(v), dtype=np.uint32).reshape(-1, 3)
+
+
+@pytest.mark.parametrize("inf", [False, True])
+def test_queries_of_a_broken_body(inf):
+    cloth, _, p = scene("workload", 8)
+    xyz, tris = broken_body(1, inf, True)
+    g = vs.Simulator(cloth.xyz, cloth.lists, xyz, tris, None, params=p)
+    o = OracleSim(p, cloth.xyz, cloth.lists, xyz, tris, None, prec=4)
+    tree, ref = g.export_lbvh(), o.export_lbvh()
+    for k in tree:
+        assert np.array_equal(tree[k], ref[k], equal_nan=True), k
+    rng = np.random.default_rng(2)
+    d = rng.normal(0, 1, (40000, 3))
+    pts = (d / np.linalg.norm(d, axis=1, keepdims=True) * rng.uniform(0.28, 0.31, (len(d), 1)) + [0, -0.3003, 0])
+    pts = pts.astype(np.float32)
+    pts[:300, rng.integers(0, 3, 300)] = np.inf
+    pts[300:600] *= np.where(rng.random((300, 3)) < 0.5, np.inf, 1.0).astype(np.float32)
+    pts[600:700, 1] = np.nan
+    a, b = g.query(pts), o.query(pts)
+    assert (a[0] >= 0).sum() > (0 if inf else 4000)  # an infinite body has few distinct codes
+    for x, y in zip(a, b):
+        assert np.array_equal(x, np.asarray(y, x.dtype), equal_nan=x.dtype.kind == "f")
+
+
+@pytest.mark.parametrize("margin", [1, 0])
+@pytest.mark.parametrize("physics", ["workload", "reference"])
+def test_steps_onto_a_broken_body(physics, margin):
+    cloth, body, p = scene(physics)
+    p.collision_margin = margin
+    xyz, tris = broken_body(3)
+    b = scenes.icosphere(4, 0.3, (0.0, -0.3003, 0.0))
+    whole = b.xyz[b.tris].reshape(-1, 3)
+    g = vs.Simulator(cloth.xyz, cloth.lists, whole, tris, None, params=p)
+    o = OracleSim(p, cloth.xyz, cloth.lists, whole, tris, None, prec=4)
+    for s in (g, o):
+        s.update_body(xyz, None)
+    for n in [1] * 8 + [16] * 9:
+        g.simulate(n)
+        o.step(n)
+        assert_equal(g, o)
+    assert g.count_contacts() > 0
+    assert not np.isnan(g.positions()).any()
