@@ -490,7 +490,7 @@ struct Engine {
         bvh.resize(G);
         for (int g = 0; g < G; ++g)
             if (gin[g].nt > 0) {
-                bvh[g].plan(arena, gin[g].nv, gin[g].nt, !gin[g].bnrm.empty(), false);
+                bvh[g].plan(arena, gin[g].nv, gin[g].nt, !gin[g].bnrm.empty(), true);
                 bvh[g].coherent = true;  // rebuilt in place: the last build's order is at hand
             }
         CU(arena.commit());

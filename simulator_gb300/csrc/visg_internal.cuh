@@ -150,13 +150,16 @@ struct BvhBuffers {
     int max_ctas = 0;            // CTAs a build launches at most
     uint32_t* bcnt = nullptr;    // bucket counts of the bucket sort
     unsigned long long* bkey = nullptr;  // its sampled keys
+    unsigned long long* bslot = nullptr;  // its buckets' slots (null: in the node array)
+    int buckets = 0;
     float* part = nullptr;       // 8 per CTA: the CTA's box union
     uint32_t* ucnt = nullptr;    // per chunk: its leaves
     uint32_t* chg = nullptr;     // count + the triangles whose code changed since the last build
     uint32_t* sync = nullptr;    // grid-barrier counters, zero between builds
 
-    // everything but the root record when `own_root` is false (the caller provides `root`)
-    void plan(Arena& a, int nv_, int nt_, bool normals, bool own_root);
+    // walked: steps and queries walk the tree (the caller provides `root`, one of an array);
+    // else the tree is only read out
+    void plan(Arena& a, int nv_, int nt_, bool normals, bool walked);
     BvhView view() const { return BvhView{nodes, leaves, root}; }
 };
 

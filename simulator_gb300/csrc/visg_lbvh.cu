@@ -202,6 +202,8 @@ struct RebuildArgs {
     uint32_t* scount;  // PASSES tile counters
     uint32_t* bcnt;    // BK_MAX bucket counts
     unsigned long long* bkey;  // SAMPLES sampled keys in order
+    unsigned long long* bslot;  // BK_CAP keys per bucket
+    int buckets;               // 0: too many triangles for the bucket sort
     float* part;       // 8 per CTA: its box union (min xyz, max xyz)
     uint32_t* ucnt;    // per chunk: its leaves, with CNT_READY once known
     uint32_t* chg;     // [0] changed codes, then {triangle, new code, old code} x CHG_CAP
@@ -605,8 +607,9 @@ __device__ void phase_merge(const RebuildArgs& A, int nc, const uint32_t* ko, co
 // bucket is sorted by one CTA in shared memory (phase_bucket_sort).  The splitters are
 // nb - 1 entries at equal distances of the last build's list, whose codes have moved only
 // a little; without one, of a sample.  The keys are distinct, so equal codes do not fill a
-// bucket.  Small buckets, so that a small body's sort takes all SMs.  The slots lie in the
-// node array, which the build writes only later.
+// bucket.  Small buckets, so that a small body's sort takes all SMs.  The slots are an array
+// of their own: a build that gives up after phase_scatter leaves whatever it wrote, and
+// the steps behind it in the stream still walk the nodes, whose links must be in range.
 //
 // The i-th of ns sampled triangles: one from each of ns equal parts of the list, at a
 // scrambled place in its part (a mesh's rows repeat: at equal distances the sample of the
@@ -644,7 +647,7 @@ __device__ void phase_scatter(const RebuildArgs& A, int nb, const uint32_t* ko, 
             S.key[i] = __ldcg(A.bkey + (i + 1) * OVERSAMPLE);
         }
     }
-    unsigned long long* slots = reinterpret_cast<unsigned long long*>(A.nodes);
+    unsigned long long* const slots = A.bslot;
     const int per = (nt + gridDim.x - 1) / gridDim.x;
     const int a = blockIdx.x * per, b = min(nt, a + per);
     constexpr int ITEMS = 4;
@@ -704,7 +707,7 @@ __device__ bool buckets_fit(const RebuildArgs& A, int nb, BucketSmem& S, uint32_
 }
 
 __device__ void phase_bucket_sort(const RebuildArgs& A, int nb, uint32_t* kn, uint32_t* vn, BucketSmem& S) {
-    const unsigned long long* slots = reinterpret_cast<const unsigned long long*>(A.nodes);
+    const unsigned long long* const slots = A.bslot;
     const int i = (int)threadIdx.x;
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
         const int n = (int)S.cnt[b];
@@ -1407,9 +1410,9 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
         }
     } else {
         bool sorted = false;
-        if (coherent ? nt <= BK_MAX * (BK_CAP / 2) : nt <= SAMPLED_MAX) {
+        if (coherent ? A.buckets > 0 : nt <= SAMPLED_MAX) {
             BucketSmem& S = *reinterpret_cast<BucketSmem*>(rb_smem);
-            const int nb = min((nt + BK_TARGET - 1) / BK_TARGET, BK_MAX);
+            const int nb = A.buckets;
             after = cur ^ 1;
             if (!coherent && nb > 1) {
                 if (ok) phase_sample(A, nb * OVERSAMPLE, S);
@@ -1505,7 +1508,7 @@ int chunk_length(int nt) {
 
 }  // namespace
 
-void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool own_root) {
+void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool walked) {
     nv = nv_;
     nt = nt_;
     has_normals = normals;
@@ -1540,13 +1543,15 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool own_root) {
     a.want(&pbox, 64 * (size_t)chunks);
     a.want(&rcnt, 2 * (size_t)chunks);
     a.want(&top, (size_t)MAX_PIECES * chunks);
-    if (own_root) a.want(&root, 1);
+    if (!walked) a.want(&root, 1);
     // histograms | sort status (PASSES x tiles x RADIX) | sort counters (the launch
     // clears them) | bucket counts | CTA box unions | chunk leaf counts | change list | barrier counters
     scratch_words = (size_t)PASSES * RADIX + (size_t)PASSES * tiles_sort * RADIX + PASSES;
     a.want(&scratch, scratch_words);
     a.want(&bcnt, (size_t)BK_MAX);
     a.want(&bkey, (size_t)SAMPLES);
+    buckets = nt <= BK_MAX * (BK_CAP / 2) ? std::min(cdiv(std::max(nt, 1), BK_TARGET), BK_MAX) : 0;
+    if (walked) a.want(&bslot, (size_t)buckets * BK_CAP);
     a.want(&part, 8 * (size_t)max_ctas);
     a.want(&ucnt, (size_t)chunks);
     a.want(&chg, 1 + 3 * (size_t)CHG_CAP);
@@ -1596,6 +1601,9 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.sync = b.sync;
     A.bcnt = b.bcnt;
     A.bkey = b.bkey;
+    // a tree that nobody walks keeps the slots in its node array, which the build writes later
+    A.bslot = b.bslot ? b.bslot : reinterpret_cast<unsigned long long*>(b.nodes);
+    A.buckets = b.buckets;
     A.chunks = b.chunks;
     A.chunk_len = b.chunk_len;
     A.err = d_err;

@@ -115,7 +115,7 @@ extern "C" int visg_lbvh_build_noalloc(const float* d_xyz, const float* d_normal
     // allocating path uses), then point inputs and outputs at the caller's arrays
     BvhBuffers b;
     Arena plan;
-    b.plan(plan, n_vertices, n_tris, d_normals != nullptr, true);
+    b.plan(plan, n_vertices, n_tris, d_normals != nullptr, false);
     int* d_err = nullptr;
     plan.want(&d_err, 4);
     size_t used = 0;
