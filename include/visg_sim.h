@@ -143,7 +143,8 @@ int visg_set_vertex(VisgSim* sim, uint32_t idx, const float xyz[3]);
 
 /* update_vertex for many vertices in one call: idx[k] gets x = x_old = xyz[3k..3k+2].
  * One scatter kernel that reads a page-locked copy of the arrays, asynchronous on the stream (the
- * host arrays are staged before the call returns).  Duplicate indices: the last wins. */
+ * host arrays are staged before the call returns).  Duplicate indices: the last wins (more
+ * than 256 indices that do not ascend take a second kernel for it). */
 int visg_set_vertices(VisgSim* sim, const uint32_t* idx, const float* xyz, int32_t n);
 
 /* Pinned vertices keep x and get x_old = x every step (the reference's drag via

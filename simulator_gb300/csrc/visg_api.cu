@@ -159,6 +159,7 @@ struct Engine {
     uint2* d_vcount = nullptr;                      // springs per list | pin bit, per vertex
     std::vector<uint2> h_vcount;
     uint32_t* d_wild = nullptr;                      // sticky: a record was not tame
+    uint32_t* d_claim = nullptr;                     // per vertex: number of the last move that named it
     int stage = 0;                                   // stage sliced-ELL blocks (autotuned)
     BvhView* d_views = nullptr;
     BvhRoot* d_roots = nullptr;                      // per garment (unset without a body)
@@ -480,6 +481,7 @@ struct Engine {
         arena.want(&d_slice_off, soff.size());
         arena.want(&d_vcount, h_vcount.size());
         arena.want(&d_wild, 4);
+        arena.want(&d_claim, (size_t)N);
         arena.want(&d_views, (size_t)G);
         arena.want(&d_roots, (size_t)G);
         arena.want(&d_err, 4);
@@ -824,6 +826,7 @@ struct Engine {
     // many vertices at once: host arrays packed into a page-locked buffer that the kernel reads
     float4* h_sv = nullptr;  // {vertex, position}, which the kernel reads
     int sv_cap = 0;
+    uint32_t sv_moves = 0;   // moves numbered so far
     cudaEvent_t sv_done = nullptr;
     int set_vertices(const uint32_t* idx, const float* xyz, int n) {
         if (!finalized) return fail(VISG_ERR_STATE, "not finalized");
@@ -842,12 +845,21 @@ struct Engine {
             sv_cap = cap;
         }
         CU(cudaEventSynchronize(sv_done));  // the kernel of the previous call has read the staging buffer
+        bool ascending = true;  // then no vertex is named twice
+        uint32_t before = idx[0];
         for (int k = 0; k < n; ++k) {
+            ascending &= k == 0 || idx[k] > before;
+            before = idx[k];
             float v;
-            std::memcpy(&v, &idx[k], 4);
+            std::memcpy(&v, &before, 4);
             h_sv[k] = make_float4(v, xyz[3 * (size_t)k], xyz[3 * (size_t)k + 1], xyz[3 * (size_t)k + 2]);
         }
-        CU(launch_set_vertices(d_state[cur], h_sv, n, p.dt, d_wild, stream));
+        if (!ascending && sv_moves > UINT32_MAX - (uint32_t)n) {
+            CU(cudaMemsetAsync(d_claim, 0, (size_t)N * sizeof(uint32_t), stream));
+            sv_moves = 0;
+        }
+        CU(launch_set_vertices(d_state[cur], h_sv, n, p.dt, d_wild, ascending ? nullptr : d_claim, sv_moves + 1u, stream));
+        if (!ascending) sv_moves += (uint32_t)n;
         CU(cudaEventRecord(sv_done, stream));
         return VISG_OK;
     }

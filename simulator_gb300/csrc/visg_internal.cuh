@@ -265,8 +265,10 @@ cudaError_t launch_clear_margin(float4* state, int64_t v0, int64_t v1, cudaStrea
 cudaError_t launch_count_contacts(const float4* state, int64_t n, unsigned long long* count, cudaStream_t s);
 
 // scatter moves[k] = {vertex, p} (x = x_old = p) into the state, keeping the contact flag; moves
-// is page-locked host memory that stays as it is until the kernel has run
-cudaError_t launch_set_vertices(float4* state, const float4* moves, int n, float dt, uint32_t* wild, cudaStream_t s);
+// is page-locked host memory that stays as it is until the kernel has run.  With `claim` (one
+// word per vertex, below `number` so far) a vertex named several times gets the last position.
+cudaError_t launch_set_vertices(float4* state, const float4* moves, int n, float dt, uint32_t* wild, uint32_t* claim,
+                                uint32_t number, cudaStream_t s);
 
 // set *wild when some record of [0, n) has a component of |x| >= 3e14 or |v| >= 1e15 (or NaN)
 cudaError_t launch_check_tame(const float4* state, int64_t n, uint32_t* wild, cudaStream_t s);

@@ -1048,10 +1048,32 @@ __global__ void k_count_contacts(const float4* __restrict__ st, int64_t n, unsig
 // there, before the wait for earlier launches: two copies in the stream before it took longer
 // than the kernel (dragged 64 x 64 sheet 33 -> 28 us a frame, six frames
 // of 24 garments with their read-back, whose copies shared the engines, 371 -> 285).
-__global__ void k_set_vertices(float4* st, const float4* moves, int n, float dt, uint32_t* wild) {
+// The threads run in no order, so where a vertex may be named twice (`claim`) the moves are
+// numbered, each claims its vertex for its number, and only the highest writes: within the
+// block where one holds all the moves (`alone`), else in a kernel of their own before.
+// Unordered moves and a synchronisation, racing -> claimed: 256 24 -> 24 us, 1,000 25 -> 27,
+// 262,144 368 -> 400 (929 with the duplicates found on the host; 1,000 in one block of 1,024
+// 33).  Ascending indices, noticed while they are packed, name no vertex twice.
+constexpr int SET_BLOCK = 256;
+__global__ void k_claim_vertices(const float4* moves, int n, uint32_t* claim, uint32_t number) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t v = k < n ? __float_as_uint(__ldcv(&moves[k].x)) : 0u;
+    wait_for_earlier_launches();
+    if (k < n) atomicMax(claim + v, number + (uint32_t)k);
+}
+__global__ void k_set_vertices(float4* st, const float4* moves, int n, float dt, uint32_t* wild, uint32_t* claim,
+                               uint32_t number, bool alone) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const float4 m = k < n ? __ldcv(moves + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     wait_for_earlier_launches();
+    if (claim) {
+        uint32_t* const c = claim + __float_as_uint(m.x);
+        if (alone) {
+            if (k < n) atomicMax(c, number + (uint32_t)k);
+            __syncthreads();
+        }
+        if (k < n && __ldcg(c) != number + (uint32_t)k) return;
+    }
     if (k >= n) return;
     const int64_t v = rec_at((int64_t)__float_as_uint(m.x));
     const f3 p = mk3(m.y, m.z, m.w);
@@ -1190,9 +1212,15 @@ cudaError_t launch_count_contacts(const float4* state, int64_t n, unsigned long 
     return cudaGetLastError();
 }
 
-cudaError_t launch_set_vertices(float4* state, const float4* moves, int n, float dt, uint32_t* wild, cudaStream_t s) {
+cudaError_t launch_set_vertices(float4* state, const float4* moves, int n, float dt, uint32_t* wild, uint32_t* claim,
+                                uint32_t number, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    return launch_after(k_set_vertices, (int)grid_for(n, 256), 256, 0, s, true, state, moves, n, dt, wild);
+    const int grid = (int)grid_for(n, SET_BLOCK);
+    if (claim && grid > 1) {
+        const cudaError_t e = launch_after(k_claim_vertices, grid, SET_BLOCK, 0, s, true, moves, n, claim, number);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_after(k_set_vertices, grid, SET_BLOCK, 0, s, true, state, moves, n, dt, wild, claim, number, grid == 1);
 }
 
 cudaError_t launch_pack_state(float4* state, float4* other, float4* normal, int64_t v0, int64_t n, const float* x,
