@@ -859,8 +859,9 @@ using StepKernel = void (*)(const StepArgs, const int, const int, const int);
 
 template <int BLOCK, bool KD0, bool STAGED, bool HELP>
 StepKernel step_kernel(bool coll, bool split) {
-    if (coll && split) return k_step<BLOCK, true, KD0, true, STAGED, HELP>;
-    if (coll || HELP) return k_step<BLOCK, true, KD0, false, STAGED, HELP>;
+    if constexpr (HELP) return k_step<BLOCK, true, KD0, false, STAGED, true>;
+    if (coll && split) return k_step<BLOCK, true, KD0, true, STAGED, false>;
+    if (coll) return k_step<BLOCK, true, KD0, false, STAGED, false>;
     return k_step<BLOCK, false, KD0, false, STAGED, false>;
 }
 
@@ -899,10 +900,10 @@ thread_local cudaEvent_t t_before_step = nullptr, t_after_step = nullptr;
 
 template <int BLOCK>
 cudaError_t launch_block(const StepArgs& a, int variant, int grid, cudaStream_t s) {
-    // helper warps need one tile per CTA and the entries read from global memory
-    const bool help = BLOCK <= kHelpBlockMax && (variant & SV_HELP) && !(variant & SV_STAGED) && grid == a.n_tiles;
-    const StepKernel fn = step_kernel<BLOCK>(help ? variant : variant & ~SV_HELP);
     const bool split = (variant & SV_COLLIDE) && (variant & SV_SPLIT);
+    // helper warps need a fused step of one tile per CTA, which they stage as a whole
+    const bool help = BLOCK <= kHelpBlockMax && (variant & SV_HELP) && !split && !(variant & SV_STAGED) && grid == a.n_tiles;
+    const StepKernel fn = step_kernel<BLOCK>(help ? variant : variant & ~SV_HELP);
     const int smem = help ? kBarBytes + 8 * a.win_cap : step_smem_bytes(variant, BLOCK, a.slice_cap);
     cudaError_t e = allow_smem((const void*)fn, smem);
     if (e != cudaSuccess) return e;
