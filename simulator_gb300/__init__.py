@@ -514,8 +514,8 @@ def selftest_bounded_waits() -> int:
 
 
 def selftest_exact_math() -> tuple[int, int]:
-    """Run visg_selftest_exact_math: the step's packed square root and reciprocal on
-    every float of their range against the CUDA intrinsics; (checked, mismatches)."""
+    """Run visg_selftest_exact_math: the step's packed square root, reciprocal and division
+    on every float of their range against the CUDA intrinsics; (checked, mismatches)."""
     n, bad = C.c_uint64(0), C.c_uint64(0)
     _check(lib().visg_selftest_exact_math(C.byref(n), C.byref(bad)))
     return int(n.value), int(bad.value)

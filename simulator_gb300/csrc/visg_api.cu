@@ -1775,17 +1775,17 @@ int visg_selftest_exact_math(uint64_t* checked, uint64_t* mismatches) {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return fail(VISG_ERR_NO_DEVICE, "no CUDA device");
     unsigned long long* d = nullptr;
-    cudaError_t e = cudaMalloc((void**)&d, 3 * sizeof(unsigned long long));
+    cudaError_t e = cudaMalloc((void**)&d, 4 * sizeof(unsigned long long));
     if (e != cudaSuccess) return cuda_fail(e, "self-test buffer");
-    unsigned long long h[3] = {0, 0, 0};
+    unsigned long long h[4] = {0, 0, 0, 0};
     e = cudaMemset(d, 0, sizeof h);
     if (e == cudaSuccess) e = launch_selftest_exact_math(d, nullptr);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof h, cudaMemcpyDeviceToHost);
     cudaFree(d);
-    if (e != cudaSuccess) return cuda_fail(e, "self-test of the packed square root and reciprocal");
+    if (e != cudaSuccess) return cuda_fail(e, "self-test of the packed square root, reciprocal and division");
     *checked = h[0];
-    *mismatches = h[1] + h[2];
+    *mismatches = h[1] + h[2] + h[3];
     return VISG_OK;
 }
 

@@ -137,7 +137,7 @@ __device__ __forceinline__ fp2 splat2(float v) { return pk2(v, v); }
 //   z ~ 1/q (rcp.approx);  e = 1 - q z (one FMA);  r = z + z e.
 // The reciprocal comes negated because rcp.approx takes -q at no cost and the packed FMA,
 // which has no negated operands, then needs no extra product for the residuals.
-// The caller sees to the range (spring_sum_exact): below 2^-100 the remainder s - g^2 can
+// The caller sees to the range (PairRange): below 2^-100 the remainder s - g^2 can
 // fall among the subnormals and lose the bits the last correction needs.
 constexpr uint32_t kExactLo = 27u << 23;                     // 2^-100
 constexpr uint32_t kExactSpan = (227u << 23) - (27u << 23);  // up to 2^100
@@ -168,7 +168,7 @@ __device__ __forceinline__ void sqrt_rcp_pair(fp2 s, fp2& q, fp2& nr) {
 // sqrt_rcp_pair returns them: two corrections of g r by an FMA's exact residual (the same
 // sources).  The first brings the quotient within one unit in the last place of g / q,
 // from where, with r correctly rounded, the second is correctly rounded (Markstein's
-// theorem; 6.9e10 pairs, over every significand of q, showed no other result).  The caller
+// theorem; visg_selftest_exact_math runs 1.3e10 pairs, over every significand of q).  The caller
 // sees to it that |g| >= 2^-60 or g = 0, so that no residual underflows, and that the
 // quotient does not overflow.  A zero numerator gives a zero, of either sign.
 __device__ __forceinline__ fp2 div_pair(fp2 g, fp2 q, fp2 nr) {

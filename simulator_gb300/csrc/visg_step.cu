@@ -1108,10 +1108,22 @@ namespace {
 // Every float s of [2^-100, 2^100) (the range where the step takes the packed square
 // root and reciprocal) through sqrt_rcp_pair, against __fsqrt_rn(s) and
 // __frcp_rn(__fsqrt_rn(s)).  The other lane of each pair carries a different float of
-// the range (s with its low mantissa bits reversed), checked too.  cnt[0] = floats
-// checked, cnt[1] = mismatches of the root, cnt[2] = of the reciprocal.
+// the range (s with its low mantissa bits reversed), checked too.  With each root q, div_pair
+// against __fdiv_rn on four numerators in its range [2^-60, 2^52 q): any significand and
+// exponent, one just below a power of two, the least, and zero (whose quotient may have
+// either sign); so every significand of q meets some 800.  cnt[0] = floats checked, cnt[1] =
+// mismatches of the root, cnt[2] = of the reciprocal, cnt[3] = of the quotients.
+__device__ __forceinline__ float numerator(uint32_t b, float q, int kind) {
+    const uint32_t h = b * 2654435761u, lo = kDivLo >> 23, hi = (__float_as_uint(q) >> 23) + 51u;
+    const uint32_t e = lo + (h >> 8) % (hi - lo + 1u), sign = h << 31;
+    const uint32_t mantissa = kind == 0 ? (h ^ (b * 40503u)) & 0x7fffffu : 0x7fffffu;
+    return kind == 3 ? 0.0f : __uint_as_float(sign | (kind == 2 ? kDivLo : e << 23 | mantissa));
+}
+__device__ __forceinline__ bool same_quotient(float neg, float g, float q) {  // neg = -g / q
+    return g == 0.0f ? neg == 0.0f : __float_as_uint(-neg) == __float_as_uint(__fdiv_rn(g, q));
+}
 __global__ void k_selftest_exact_math(unsigned long long* cnt) {
-    unsigned long long n = 0, bad_q = 0, bad_r = 0;
+    unsigned long long n = 0, bad_q = 0, bad_r = 0, bad_d = 0;
     const uint64_t lo = kExactLo, hi = (uint64_t)kExactLo + kExactSpan;
     for (uint64_t u = lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < hi;
          u += (uint64_t)gridDim.x * blockDim.x) {
@@ -1125,10 +1137,17 @@ __global__ void k_selftest_exact_math(unsigned long long* cnt) {
         bad_r += (__float_as_uint(-lo2(nr)) != __float_as_uint(__frcp_rn(qa))) +
                  (__float_as_uint(-hi2(nr)) != __float_as_uint(__frcp_rn(qb)));
         n += 2;
+#pragma unroll 1
+        for (int kind = 0; kind < 4; ++kind) {
+            const float ga = numerator(b, qa, kind), gb = numerator(b2, qb, kind);
+            const fp2 d = div_pair(pk2(ga, gb), q, nr);
+            bad_d += !same_quotient(lo2(d), ga, qa) + !same_quotient(hi2(d), gb, qb);
+        }
     }
     atomicAdd(&cnt[0], n);
     if (bad_q) atomicAdd(&cnt[1], bad_q);
     if (bad_r) atomicAdd(&cnt[2], bad_r);
+    if (bad_d) atomicAdd(&cnt[3], bad_d);
 }
 }  // namespace
 
