@@ -52,9 +52,11 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 constexpr int kNumBlocks = 4;
 constexpr int kBlocks[kNumBlocks] = {128, 256, 512, 1024};
-// largest sliced-ELL block (entries) of a tile that a launch with helper warps stages in
-// shared memory: 16 entries per vertex
-constexpr int kStageCap[kNumBlocks] = {2048, 4096, 8192, 14336};
+// the block sizes that have helper warps, and the largest sliced-ELL block (entries) of a tile
+// that such a launch stages in shared memory: 16 entries per vertex
+constexpr int kHelpBlocks = 2;
+static_assert(kBlocks[kHelpBlocks - 1] == kHelpBlockMax && kBlocks[kHelpBlocks] > kHelpBlockMax, "the first ones");
+constexpr int kStagedPerVertex = 16;
 // longest slice that a warp's stage buffer may hold: rows of 24, so that the 32 buffers of a
 // 1,024-thread CTA (192 KB) fit an SM; the buffers are as long as the longest such slice
 constexpr int kSliceCap = 32 * 24;
@@ -149,8 +151,8 @@ struct Engine {
     float* d_k = nullptr;
     int4* d_tiles[kNumBlocks] = {nullptr, nullptr, nullptr, nullptr};
     int n_tiles[kNumBlocks] = {0, 0, 0, 0};
-    int2* d_twin[kNumBlocks] = {nullptr, nullptr, nullptr, nullptr};  // per tile sliced-ELL block {first entry, count}
-    int win_cap[kNumBlocks] = {0, 0, 0, 0};                           // entries of the longest block
+    int2* d_twin[kHelpBlocks] = {nullptr, nullptr};  // per tile sliced-ELL block {first entry, count}
+    int win_cap[kHelpBlocks] = {0, 0};               // entries of the longest block
     int4* d_slices = nullptr;                        // per slice, for the staged step
     int n_slices = 0, slice_cap = 0;                 // entries per warp's stage buffer, 0 = no slice staged
     uint2* d_sell = nullptr;                         // sliced-ELL springs
@@ -431,19 +433,19 @@ struct Engine {
                 if (cnt <= kSliceCap) slice_cap = std::max(slice_cap, (int)cnt);
             }
         n_slices = (int)S;
-        // tiles for each block size, with the sliced-ELL block of each one's slices
+        // tiles for each block size; for those with helper warps the sliced-ELL block of each
+        // tile's slices
         std::vector<std::vector<int4>> tiles(kNumBlocks);
-        std::vector<std::vector<int2>> twin(kNumBlocks);
+        std::vector<std::vector<int2>> twin(kHelpBlocks);
         for (int b = 0; b < kNumBlocks; ++b) {
-            const int cap = kStageCap[b];
-            win_cap[b] = 0;
             for (int g = 0; g < G; ++g)
                 for (int64_t v = voff[g]; v < voff[g + 1]; v += kBlocks[b]) {
                     const int64_t v1 = std::min<int64_t>(v + kBlocks[b], voff[g + 1]);
                     const int64_t s0 = slice0[g] + (v - voff[g]) / 32, s1 = s0 + (v1 - v + 31) / 32;
                     tiles[b].push_back(make_int4(g | (gin[g].nt > 0 ? TILE_BODY : 0), (int)v, (int)v1, (int)s0));
+                    if (b >= kHelpBlocks) continue;
                     const int64_t cnt = (int64_t)soff[s1] - soff[s0];
-                    if (cnt > 0 && cnt <= cap && soff[s1] <= 0x7fffffffu) {
+                    if (cnt > 0 && cnt <= kStagedPerVertex * kBlocks[b] && soff[s1] <= 0x7fffffffu) {
                         twin[b].push_back(make_int2((int)soff[s0], (int)cnt));
                         win_cap[b] = std::max(win_cap[b], (int)cnt);
                     } else {
@@ -473,7 +475,7 @@ struct Engine {
         for (int b = 0; b < kNumBlocks; ++b) {
             n_tiles[b] = (int)tiles[b].size();
             arena.want(&d_tiles[b], tiles[b].size() + 1);
-            arena.want(&d_twin[b], twin[b].size() + 1);
+            if (b < kHelpBlocks) arena.want(&d_twin[b], twin[b].size() + 1);
         }
         arena.want(&d_slices, slices.size());
         arena.want(&d_sell, sell.size());
@@ -515,7 +517,8 @@ struct Engine {
         if (perk && E > 0) CU(cudaMemcpy(d_k, kk.data(), E * sizeof(float), cudaMemcpyHostToDevice));
         for (int b = 0; b < kNumBlocks; ++b) {
             CU(cudaMemcpy(d_tiles[b], tiles[b].data(), tiles[b].size() * sizeof(int4), cudaMemcpyHostToDevice));
-            CU(cudaMemcpy(d_twin[b], twin[b].data(), twin[b].size() * sizeof(int2), cudaMemcpyHostToDevice));
+            if (b < kHelpBlocks)
+                CU(cudaMemcpy(d_twin[b], twin[b].data(), twin[b].size() * sizeof(int2), cudaMemcpyHostToDevice));
         }
         CU(cudaMemcpy(d_slices, slices.data(), slices.size() * sizeof(int4), cudaMemcpyHostToDevice));
         CU(cudaMemcpy(d_sell, sell.data(), sell.size() * sizeof(uint2), cudaMemcpyHostToDevice));
@@ -613,9 +616,6 @@ struct Engine {
         a.state_in = d_state[from];
         a.state_out = d_state[from ^ 1];
         a.normal = d_normal;
-        a.rowp = d_rowp;
-        a.ent = d_ent;
-        a.kent = d_k;
         int bi = block_index(blk);
         const int two = groups() == 2;
         const int t0 = (two && grp == 1) ? tsplit[bi] : 0, t1 = (two && grp == 0) ? tsplit[bi] : n_tiles[bi];
@@ -631,8 +631,8 @@ struct Engine {
         a.slice_off = d_slice_off;
         a.vcount = d_vcount;
         a.wild = d_wild;
-        a.twin = d_twin[bi] + t0;
-        a.win_cap = win_cap[bi];
+        a.twin = bi < kHelpBlocks ? d_twin[bi] + t0 : nullptr;
+        a.win_cap = bi < kHelpBlocks ? win_cap[bi] : 0;
         const int c0 = (two && grp == 1) ? ssplit : 0, c1 = (two && grp == 0) ? ssplit : n_slices;
         a.slices = d_slices + c0;
         a.n_slices = c1 - c0;

@@ -188,9 +188,6 @@ struct StepArgs {
     const float4* state_in;
     float4* state_out;
     float4* normal;  // in place
-    const uint32_t* rowp;
-    const uint2* ent;
-    const float* kent;
     const int4* tiles;
     int n_tiles;
     const BvhRoot* roots;  // per garment
@@ -203,7 +200,7 @@ struct StepArgs {
     const uint32_t* slice_off;
     const uint2* vcount;      // per vertex: springs per list, 16 bits each (list 3: 15), bit 63 = pinned
     uint32_t* wild;           // sticky: some record had |x| >= 3e14 or |v| >= 1e15 (or NaN)
-    const int2* twin;         // per tile sliced-ELL block, with SV_STAGED
+    const int2* twin;         // per tile sliced-ELL block, with SV_HELP
     int win_cap;              // entries of the longest tile block that helper launches stage
     const int4* slices;       // {garment, first vertex, first entry, vertices | row length << 6} per slice
     int n_slices;

@@ -67,7 +67,6 @@ struct f4x2 {
     }
 VISG_LD8(ld8_nc, "ld.global.nc", )           // data no one writes during the launch
 VISG_LD8(ld8, "ld.global", volatile)
-VISG_LD8(ld8_once, "ld.global.nc", volatile) // the same, not merged with an earlier load of the address
 VISG_LD8(ld8_cg, "ld.global.cg", volatile)   // through L2: data another CTA wrote earlier in the launch
 #undef VISG_LD8
 __device__ __forceinline__ float4 ld4(const float4* p) {  // 16 bytes, not merged with an earlier load
