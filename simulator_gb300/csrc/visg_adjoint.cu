@@ -48,8 +48,7 @@ namespace visg {
 namespace {
 
 // The reverse sweep runs in double: per-spring contributions of both signs cancel
-// over hundreds of steps, and float accumulation loses several digits there (the
-// forward trajectory it differentiates is the float one, bit for bit).
+// over hundreds of steps, and float accumulation loses several digits there.
 struct V {
     double x, y, z;
 };
@@ -348,6 +347,9 @@ __global__ void k_adj_result(const double* __restrict__ dk, const uint32_t* __re
 // FULL: the springs are damped, or some state was not tame (then the damping terms' NaNs
 // must come out as written); two bodies, so that the undamped one issues none of the rest.
 constexpr int ADJ_THREADS = 128;
+__device__ __forceinline__ bool adj_full(const AdjArgs& a) {
+    return a.gxo != nullptr && (__float_as_uint(a.p.kd) != 0u || *a.wild != 0u);
+}
 template <bool FULL>
 __device__ __forceinline__ void adj_entry(const AdjArgs& a, const uint32_t e) {
     const uint32_t i = __ldg(a.src + e), r = __ldg(a.rev + e);
@@ -388,7 +390,7 @@ __device__ __forceinline__ void adj_entry(const AdjArgs& a, const uint32_t e) {
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_entry(const AdjArgs a) {
     const int64_t e = (int64_t)blockIdx.x * ADJ_THREADS + threadIdx.x;
     if (e >= a.E) return;
-    if (__float_as_uint(a.p.kd) != 0u || *a.wild != 0u)
+    if (adj_full(a))
         adj_entry<true>(a, (uint32_t)e);
     else
         adj_entry<false>(a, (uint32_t)e);
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(3 * ADJ_VERTS * ADJ_PARTS) k_adj_vertex(const 
     __shared__ double s_lx[3 * ADJ_VERTS], s_lxo[3 * ADJ_VERTS];
     const StepParams& P = a.p;
     const int tid = (int)threadIdx.x;
-    const bool full = __float_as_uint(P.kd) != 0u || *a.wild != 0u;
+    const bool full = adj_full(a);
     const int64_t i0 = (int64_t)blockIdx.x * ADJ_VERTS;
     {
         const int q = tid % ADJ_PARTS, t = tid / ADJ_PARTS, vi = t / 3, c = t - 3 * vi;

@@ -184,7 +184,7 @@ struct Engine {
     bool prev_ok = false;  // the other buffer holds the positions the last step started from
     int split = 1;                     // collision in its own kernel (autotuned)
     float* d_stage = nullptr;  // 10*N floats
-    uint32_t* h_status = nullptr;  // pinned: err, check0, check1
+    uint32_t* h_status = nullptr;  // pinned: err, check0, check1, adj.wild
     int cur = 0;
     int block = 256, grid = 0;
     // SMs the persistent step kernel leaves free when two garment groups step as
@@ -206,7 +206,8 @@ struct Engine {
         double* vel = nullptr;       // 6N: velocities of a step's input and output state
         double* lam = nullptr;       // 2 x 3N: adjoints of x, x_old
         double* G = nullptr;         // 3N
-        double* g = nullptr;         // 12 per merged entry: its and its reverse entry's contributions to x, x_old
+        double* gx = nullptr;        // 6 per merged entry: its and its reverse entry's contributions to x
+        double* gxo = nullptr;       // the same for x_old, where a sweep needs it (backward)
         double* dk = nullptr;        // per merged entry dL/dk, its part of dL/dkd; per component of dL/dgamma, dL/dc
         float* out = nullptr;        // per merged entry: the gradient in the caller's order
         double* dsc = nullptr;       // 3, then the count of gradients that are not finite
@@ -218,6 +219,8 @@ struct Engine {
         unsigned* contacts = nullptr;  // vertices projected in each forward step
         int contacts_cap = 0;
         bool ready = false;
+        bool was_wild = false;  // some state of the last forward set `wild`
+        bool changed = false;   // the body or the pins changed since, so a replay may reach other states
     } adj;
 
     // asynchronous position read-back: two device staging slots copied to host memory
@@ -268,7 +271,7 @@ struct Engine {
     void free_adjoint() {
         for (auto* q : adj.ck) cudaFree(q);
         adj.ck.clear();
-        void* ps[] = {adj.tmp, adj.rec, adj.vel, adj.lam, adj.G,   adj.g,   adj.dk,
+        void* ps[] = {adj.tmp, adj.rec, adj.vel, adj.lam, adj.G,   adj.gx,  adj.gxo, adj.dk,
                       adj.out, adj.dsc, adj.wild, adj.rev, adj.src, adj.pos, adj.rest64, adj.contacts};
         for (void* q : ps)
             if (q) cudaFree(q);
@@ -800,6 +803,7 @@ struct Engine {
         // staged first.  The build also voids the garment's query-cache margins (the
         // body moves)
         adj.rec_seg = -1;  // a backward pass replays every segment over the body as it is then
+        adj.changed = true;
         settled = false;
         const bool dev = kind == cudaMemcpyDeviceToDevice;
         if (!dev) {
@@ -876,6 +880,7 @@ struct Engine {
         for (int k = 0; k < n; ++k)
             if (idx[k] >= (uint32_t)N) return fail(VISG_ERR_INVALID_ARG, "pinned index out of range");
         adj.rec_seg = -1;  // a backward pass replays every segment with the pins as they are then
+        adj.changed = true;
         for (int64_t i = 0; i < N; ++i) h_rowp[i] &= ROW_MASK;
         for (int k = 0; k < n; ++k) h_rowp[idx[k]] |= PIN_BIT;
         for (int64_t i = 0; i < N; ++i) h_vcount[i].y = (h_vcount[i].y & ROW_MASK) | (h_rowp[i] & PIN_BIT);

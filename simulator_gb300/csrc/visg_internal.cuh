@@ -320,7 +320,7 @@ struct AdjArgs {
     double* G;             // adjoint of the force on each vertex
     double* v;             // (x - xo) / dt
     double* gx;            // per entry two double3: its contribution to x of its vertex, and its reverse entry's;
-    double* gxo;           // the same for x_old (only with spring damping)
+    double* gxo;           // the same for x_old; NULL: springs undamped and every state tame
     double* dk;            // per entry, accumulated over steps
     double* dkd;           // per entry: its part of dL/d spring damping, accumulated
     double* dgc;           // per vertex component: its parts of dL/d gamma and force damping, accumulated
