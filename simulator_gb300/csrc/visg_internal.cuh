@@ -143,6 +143,8 @@ struct BvhBuffers {
     float4* pbox = nullptr;      // 2 per record: union of the chunk's leaves up to the boundary
     uint32_t* rcnt = nullptr;    // 2 per chunk: prefix record count | nodes in `top` << 16; suffix record count
     int2* top = nullptr;         // 64 per chunk: {boundary, delta} of the nodes that span chunks
+    int* gmin = nullptr;         // for bodies of more than 1,024 chunks, per 32 of them: min of cmin
+    float4* gbox = nullptr;      // and union of cbox (2)
     int chunks = 0, chunk_len = 0;
     BvhRoot* root = nullptr;
     uint32_t* scratch = nullptr; // radix histograms, look-back status words, tile counters (the build clears them)

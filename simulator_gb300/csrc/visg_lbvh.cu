@@ -27,8 +27,9 @@
 //           single CTAs sort in shared memory (phase_scatter, phase_bucket_sort).
 //           Otherwise, or if a bucket overflows: four stable LSD radix passes over 8-bit
 //           digits, tiles claimed in order, decoupled look-back.
-//   build   per chunk of 512 sorted positions: de-duplication (keep the first triangle
-//           of every distinct code, remove_redundant, Utilities.h:35-55) and a bottom-up
+//   build   per chunk of up to 512 sorted positions: de-duplication (keep the first triangle
+//           of every distinct code, remove_redundant, Utilities.h:35-55; of more than 524,288
+//           triangles in a phase before) and a bottom-up
 //           radix-tree build fused with the refit: each leaf thread climbs with handshakes
 //           in shared memory while both children lie in the chunk; the parent of range
 //           [l, r] is the boundary with the longer common prefix (delta(l-1,l)
@@ -173,6 +174,8 @@ struct ChunkView {  // summaries of the chunks (build_chunk)
     float4* pbox;
     uint32_t* rcnt;  // 2 per chunk
     int2* top;
+    int* gmin;       // per 32 chunks, for bodies of more than TOP_STAGED chunks: min delta
+    float4* gbox;    // and box union (2)
 };
 
 struct RebuildArgs {
@@ -864,6 +867,79 @@ __device__ void phase_sort_pass(const RebuildArgs& A, int p, SortSmem& S, uint32
     }
 }
 
+// ---- unique (bodies of more than TOP_STAGED chunks) ------------------------------------------------
+// De-duplication before the build.  A large body's codes are crowded (10 bits an axis), so many
+// triangles share one, and chunks of sorted positions would be chunks of few leaves: 5.1 M
+// triangles with 2.4 M codes take 641 us a rebuild with the de-duplication in the build, 362
+// with it before; 21.8 M with 4.7 M 2,371 and 966.  CTA c takes the positions [c per, (c + 1) per) of the sorted list.
+constexpr int UNIQ_ITEMS = 4;
+__device__ __forceinline__ int unique_slice(const RebuildArgs& A, int& b) {
+    const int per = (A.nt + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int a = (int)min((int64_t)blockIdx.x * per, (int64_t)A.nt);
+    b = min(A.nt, a + per);
+    return a;
+}
+// bit j: position p + j step is a leaf (position 0, or its code differs from the one before's)
+__device__ __forceinline__ uint32_t leaf_bits(const uint32_t* K, int p, int step, int b, uint32_t (&k)[UNIQ_ITEMS]) {
+    uint32_t before[UNIQ_ITEMS], f = 0;
+#pragma unroll
+    for (int j = 0; j < UNIQ_ITEMS; ++j) {
+        const int q = p + j * step;
+        k[j] = q < b ? __ldcg(K + q) : 0u;
+        before[j] = q < b && q > 0 ? __ldcg(K + q - 1) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < UNIQ_ITEMS; ++j)
+        if (p + j * step < b && (p + j * step == 0 || k[j] != before[j])) f |= 1u << j;
+    return f;
+}
+__device__ void phase_unique_count(const RebuildArgs& A, const uint32_t* K, uint32_t* s_scan) {
+    int b;
+    const int a = unique_slice(A, b);
+    uint32_t k[UNIQ_ITEMS], c = 0;
+    for (int p = a + (int)threadIdx.x; p < b; p += RB * UNIQ_ITEMS) c += __popc(leaf_bits(K, p, RB, b, k));
+    block_scan_incl(c, s_scan);
+    if (threadIdx.x == 0) A.ucnt[blockIdx.x] = s_scan[RW - 1];
+}
+// the leaves of this CTA's slice at its offset; returns the number of leaves in all
+__device__ int phase_unique_write(const RebuildArgs& A, const uint32_t* K, const uint32_t* V, uint32_t* s_scan) {
+    uint32_t before = 0, all = 0;
+    for (int c = threadIdx.x; c < (int)gridDim.x; c += RB) {
+        const uint32_t v = __ldcg(A.ucnt + c);
+        all += v;
+        if (c < (int)blockIdx.x) before += v;
+    }
+    block_scan_incl(before, s_scan);
+    uint32_t off = s_scan[RW - 1];
+    __syncthreads();
+    block_scan_incl(all, s_scan);
+    const int n = (int)min(s_scan[RW - 1], (uint32_t)A.nt);
+    __syncthreads();
+    int b;
+    const int a = unique_slice(A, b);
+    for (int base = a; base < b; base += RB * UNIQ_ITEMS) {
+        const int p = base + (int)threadIdx.x * UNIQ_ITEMS;
+        uint32_t k[UNIQ_ITEMS], t[UNIQ_ITEMS];
+#pragma unroll
+        for (int j = 0; j < UNIQ_ITEMS; ++j) t[j] = p + j < b ? __ldcg(V + p + j) : 0u;
+        const uint32_t f = leaf_bits(K, p, 1, b, k), cnt = (uint32_t)__popc(f);
+        uint32_t o = off + block_scan_incl(cnt, s_scan) - cnt;
+        off += s_scan[RW - 1];
+#pragma unroll
+        for (int j = 0; j < UNIQ_ITEMS; ++j)
+            if (f >> j & 1u) {
+                if (o < (uint32_t)A.nt) {
+                    A.ucode[o] = k[j];
+                    A.utri[o] = t[j];
+                }
+                ++o;
+            }
+        __syncthreads();  // s_scan is read above before the next scan overwrites it
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.root->n_leaves = n;
+    return n;
+}
+
 // ---- build ---------------------------------------------------------------------------------------
 // identity box (min +100, max -100) expanded by child A then child B
 __device__ __forceinline__ void merge_ab(float4 alo, float4 ahi, float4 blo, float4 bhi, float4& lo, float4& hi) {
@@ -934,17 +1010,21 @@ __device__ __forceinline__ int far_delta(int w) { return (w >> 16) - 1; }
 //     chunk's leaf boxes beyond / up to each of them;
 //   * the chunk's min delta and leaf box union.
 // Two warps make the summary of at most 63 pieces, two per lane, from either end.
-__device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, const uint32_t* V, BuildSmem& S) {
+// BIG: K and V are the np leaves themselves (phase_unique), so a chunk's positions are its
+// leaves and their numbers.
+template <bool BIG>
+__device__ void build_chunk(const RebuildArgs& A, int chunk, int np, const uint32_t* K, const uint32_t* V,
+                            BuildSmem& S) {
     const float inf = __int_as_float(0x7f800000);
     const ChunkView& cv = A.cv;
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nt = A.nt, p0 = chunk * A.chunk_len, m = min(A.chunk_len, nt - p0), p = p0 + tid;
+    const int p0 = chunk * A.chunk_len, m = min(A.chunk_len, np - p0), p = p0 + tid;
     const bool in = tid < m;
     uint32_t k = 0u, t = 0u;
     float4 lo = ident_lo(), hi = ident_hi();
     if (in) {
         k = __ldcg(K + p);
-        t = min(__ldcg(V + p), (uint32_t)(nt - 1));
+        t = min(__ldcg(V + p), (uint32_t)(A.nt - 1));
         // A triangle whose corners are all NaN on an axis has a NaN box, which holds no point.
         // As a leaf it is empty on that axis, so that the walks test boxes by their gaps;
         // a union takes neither a NaN nor an empty axis in.
@@ -953,24 +1033,27 @@ __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, 
         hi = make_float4(fmaxf(b.b.x, -inf), fmaxf(b.b.y, -inf), fmaxf(b.b.z, -inf), 0.0f);
     }
     // the counts of the chunks before (most are there by the time they are needed)
-    uint32_t cw = tid < chunk ? ld_volatile(A.ucnt + tid) : CNT_READY;
+    uint32_t cw = !BIG && tid < chunk ? ld_volatile(A.ucnt + tid) : CNT_READY;
     S.code[tid + 1] = k;
     if (tid == 0) S.code[0] = p0 > 0 ? __ldcg(K + p0 - 1) : 0u;
-    if (warp == 0) S.next[lane] = p0 + m + lane < nt ? __ldcg(K + p0 + m + lane) : 0xffffffffu;
+    if (warp == 0) S.next[lane] = p0 + m + lane < np ? __ldcg(K + p0 + m + lane) : 0xffffffffu;
     S.flag[tid] = 0u;
     if (lane == 0) S.pbits[warp] = 0u;
     __syncthreads();
-    const bool first = in && (p == 0 || k != S.code[tid]);
-    const unsigned fb = __ballot_sync(0xffffffffu, first);
-    if (lane == 0) S.wcnt[warp] = (uint32_t)__popc(fb);
-    __syncthreads();
-    const uint32_t wc = lane < RW ? S.wcnt[lane] : 0u;
-    const int cnt = (int)__reduce_add_sync(0xffffffffu, wc);
-    const int rank = (int)__reduce_add_sync(0xffffffffu, lane < warp ? wc : 0u) + __popc(fb & ((1u << lane) - 1u));
-    if (tid == 0) st_volatile(A.ucnt + chunk, CNT_READY | (uint32_t)cnt);
+    const bool first = in && (BIG || p == 0 || k != S.code[tid]);
+    int cnt = m, rank = tid;
+    if constexpr (!BIG) {
+        const unsigned fb = __ballot_sync(0xffffffffu, first);
+        if (lane == 0) S.wcnt[warp] = (uint32_t)__popc(fb);
+        __syncthreads();
+        const uint32_t wc = lane < RW ? S.wcnt[lane] : 0u;
+        cnt = (int)__reduce_add_sync(0xffffffffu, wc);
+        rank = (int)__reduce_add_sync(0xffffffffu, lane < warp ? wc : 0u) + __popc(fb & ((1u << lane) - 1u));
+        if (tid == 0) st_volatile(A.ucnt + chunk, CNT_READY | (uint32_t)cnt);
+    }
     if (first && rank == 0) S.delta[0] = p == 0 ? -1 : __clz((int)(k ^ S.code[tid]));
     const uint32_t* lc = S.code + 1;  // the leaves' codes
-    if (cnt != m) {                   // some position is not a leaf: close the ranks up
+    if (!BIG && cnt != m) {           // some position is not a leaf: close the ranks up
         lc = S.lcode;
         if (first) {
             S.lcode[rank] = k;
@@ -992,13 +1075,13 @@ __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, 
     if (warp == 0 && cnt > 0) {  // the boundary to the next leaf, wherever it is
         const uint32_t last = lc[cnt - 1];
         const int e = p0 + m;
-        const unsigned b = __ballot_sync(0xffffffffu, e + lane < nt && S.next[lane] != last);
+        const unsigned b = __ballot_sync(0xffffffffu, e + lane < np && S.next[lane] != last);
         if (lane == 0) {
             int d = -1;
             if (b) {
                 d = __clz((int)(last ^ S.next[__ffs(b) - 1]));
-            } else if (e + 32 < nt) {  // more than 32 copies of the code follow: the first larger one
-                int l = e + 32, len = nt - l;
+            } else if (!BIG && e + 32 < np) {  // more than 32 copies of the code follow: the first larger one
+                int l = e + 32, len = np - l;
                 while (len > 0) {
                     const int h = len >> 1;
                     if (__ldcg(K + l + h) <= last) {
@@ -1008,7 +1091,7 @@ __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, 
                         len = h;
                     }
                 }
-                if (l < nt) d = __clz((int)(last ^ __ldcg(K + l)));
+                if (l < np) d = __clz((int)(last ^ __ldcg(K + l)));
             }
             S.delta[cnt] = d;
         }
@@ -1057,30 +1140,34 @@ __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, 
         }
         link = g;
     }
-    // leaves before the chunk
-    uint32_t before = 0;
-    for (int c = tid; c < chunk; c += RB) {
-        int spins = 0;
-        if (c != tid) cw = ld_volatile(A.ucnt + c);
-        while (!(cw & CNT_READY)) {
-            if (++spins > SPIN_LIMIT) {
-                atomicOr(A.err, ERR_TIMEOUT);
-                break;
+    int base = p0;  // leaves before the chunk
+    if constexpr (!BIG) {
+        uint32_t before = 0;
+        for (int c = tid; c < chunk; c += RB) {
+            int spins = 0;
+            if (c != tid) cw = ld_volatile(A.ucnt + c);
+            while (!(cw & CNT_READY)) {
+                if (++spins > SPIN_LIMIT) {
+                    atomicOr(A.err, ERR_TIMEOUT);
+                    break;
+                }
+                __nanosleep(32);
+                cw = ld_volatile(A.ucnt + c);
             }
-            __nanosleep(32);
-            cw = ld_volatile(A.ucnt + c);
+            before += cw & ~CNT_READY;
         }
-        before += cw & ~CNT_READY;
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) S.wsum[warp] = before;
+        __syncthreads();
+        base = (int)__reduce_add_sync(0xffffffffu, lane < RW ? S.wsum[lane] : 0u);
+    } else {
+        __syncthreads();  // every climb is done
     }
-    before = __reduce_add_sync(0xffffffffu, before);
-    if (lane == 0) S.wsum[warp] = before;
-    __syncthreads();
-    const int base = (int)__reduce_add_sync(0xffffffffu, lane < RW ? S.wsum[lane] : 0u);
     const auto global_link = [&](float w) {
         const int v = __float_as_int(w);
         return __int_as_float(v >= 0 ? v + base : v - base);
     };
-    if (tid == 0 && chunk == A.chunks - 1) A.root->n_leaves = base + cnt;
+    if (!BIG && tid == 0 && chunk == A.chunks - 1) A.root->n_leaves = base + cnt;
     if (is_root) {  // the whole tree in one chunk; a single leaf has no root node
         A.root->root = l == r ? -1 : link + base;
         A.root->top_lo = make_float4(lo.x, lo.y, lo.z, 0.0f);
@@ -1175,8 +1262,10 @@ __device__ void build_chunk(const RebuildArgs& A, int chunk, const uint32_t* K, 
     // meanwhile the other warps write the leaves, and the nodes whose children both arrived here
     if (tid < cnt) {
         st8(A.leaves + 2 * (base + tid), leaf.a, leaf.b);
-        A.ucode[base + tid] = k;
-        A.utri[base + tid] = t;
+        if (!BIG) {
+            A.ucode[base + tid] = k;
+            A.utri[base + tid] = t;
+        }
     }
     if (tid < cnt - 1 && S.flag[tid] == 3u) {
         const int g = base + tid;
@@ -1204,7 +1293,10 @@ __device__ __forceinline__ int first_record(const int2* rec, int count, int g, i
 }
 
 // The chunk summaries as the spanning nodes read them: from shared memory (STAGED) or,
-// for bodies of more than TOP_STAGED chunks, where they are.
+// for bodies of more than TOP_STAGED chunks, where they are.  Those bodies have summaries of
+// 32 chunks too (phase_groups), or the node at the root alone would read every chunk's, one
+// round of 32 after another, and look at their slots 32 at a time (phase_top): 1.3 M triangles
+// with distinct codes 219 -> 208 us a rebuild.
 template <bool STAGED>
 struct Summaries {
     const ChunkView& cv;
@@ -1224,25 +1316,63 @@ struct Summaries {
             box_union(lo, hi, b.a, b.b);
         }
     }
-    // nearest chunk left of c (right of c) whose min delta is below d; -1: none
-    __device__ int nearest(int c, int F, int d, bool right, int lane) const {
-        constexpr int W = STAGED ? 1 : 4;  // groups of 32 in flight
-        for (int b = right ? c + 1 : c - 1; right ? b < F : b >= 0; b += right ? 32 * W : -32 * W) {
-            int v[W];
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-                const int i = right ? b + 32 * w + lane : b - 32 * w - lane;
-                v[w] = i >= 0 && i < F ? min_delta(i) : BIG_DELTA;
+    // the leaf boxes of chunks [a, b), over the lanes
+    __device__ __forceinline__ void add_boxes(int a, int b, int lane, float4& lo, float4& hi) const {
+        const int ga = (a + 31) >> 5, gb = b >> 5;  // whole groups
+        const bool grouped = !STAGED && ga < gb;
+        for (int e = a + lane; e < (grouped ? 32 * ga : b); e += 32) add_box(e, lo, hi);
+        if (grouped) {
+            for (int g = ga + lane; g < gb; g += 32) {
+                const f4x2 x = ld8_cg(cv.gbox + 2 * g);
+                box_union(lo, hi, x.a, x.b);
             }
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-                const unsigned h = __ballot_sync(0xffffffffu, v[w] < d);
-                if (h) return right ? b + 32 * w + __ffs(h) - 1 : b - 32 * w - (__ffs(h) - 1);
-            }
+            if (32 * gb + lane < b) add_box(32 * gb + lane, lo, hi);
+        }
+    }
+    // of the entries v(i), i from `from` in steps of +1 or -1 up to the bounds, the first below d
+    template <class Value>
+    __device__ __forceinline__ static int first_below(Value v, int from, int n, int d, bool right, int lane) {
+        for (int b = from; right ? b < n : b >= 0; b += right ? 32 : -32) {
+            const int i = right ? b + lane : b - lane;
+            const unsigned h = __ballot_sync(0xffffffffu, i >= 0 && i < n && v(i) < d);
+            if (h) return right ? b + __ffs(h) - 1 : b - (__ffs(h) - 1);
         }
         return -1;
     }
+    // nearest chunk left of c (right of c) whose min delta is below d; -1: none
+    __device__ int nearest(int c, int F, int d, bool right, int lane) const {
+        const auto chunk = [&](int i) { return min_delta(i); };
+        if (STAGED) return first_below(chunk, right ? c + 1 : c - 1, F, d, right, lane);
+        const int g = c >> 5, in = 32 * g + lane;  // the rest of the chunk's own group
+        const unsigned h = __ballot_sync(0xffffffffu, (right ? in > c : in < c) && in < F && min_delta(in) < d);
+        if (h) return right ? 32 * g + __ffs(h) - 1 : 32 * g + 31 - __clz(h);
+        const auto group = [&](int i) { return __ldcg(cv.gmin + i); };
+        const int f = first_below(group, right ? g + 1 : g - 1, (F + 31) >> 5, d, right, lane);
+        return f < 0 ? -1 : first_below(chunk, right ? 32 * f : min(32 * f + 31, F - 1), F, d, right, lane);
+    }
 };
+
+// min delta and leaf box union of every 32 chunks, a warp each
+__device__ void phase_groups(const RebuildArgs& A, int F) {
+    const ChunkView& cv = A.cv;
+    const int lane = (int)(threadIdx.x & 31u);
+    for (int g = blockIdx.x * RW + (int)(threadIdx.x >> 5); 32 * g < F; g += gridDim.x * RW) {
+        const int c = 32 * g + lane;
+        int d = BIG_DELTA;
+        float4 lo = ident_lo(), hi = ident_hi();
+        if (c < F) {
+            d = __ldcg(cv.cmin + c);
+            const f4x2 b = ld8_cg(cv.cbox + 2 * c);
+            box_union(lo, hi, b.a, b.b);
+        }
+        d = __reduce_min_sync(0xffffffffu, d);
+        warp_box_reduce(lo, hi);
+        if (lane == 0) {
+            cv.gmin[g] = d;
+            st8(cv.gbox + 2 * g, lo, hi);
+        }
+    }
+}
 
 // One node that spans chunks, by one warp: the range ends are the nearest boundaries
 // with a smaller delta on either side (the first suffix / prefix record past the node
@@ -1290,7 +1420,7 @@ __device__ void top_node(const RebuildArgs& A, const Summaries<STAGED>& sum, int
         cr = F;
     }
     float4 ul = ident_lo(), uh = ident_hi();
-    for (int e = cl + 1 + lane; e < cr; e += 32) sum.add_box(e, ul, uh);
+    sum.add_boxes(cl + 1, cr, lane, ul, uh);
     warp_box_reduce(ul, uh);
     box_union(lo, hi, ul, uh);
     if (lane == 0) {
@@ -1308,16 +1438,22 @@ __device__ void top_node(const RebuildArgs& A, const Summaries<STAGED>& sum, int
 // The nodes whose leaf range spans chunks, one warp each, independently.  Each CTA stages
 // the summaries it searches (28 bytes a chunk) and the running count of the chunks' nodes,
 // by which the warps share the nodes out.
-__device__ void phase_top(const RebuildArgs& A, TopSmem& S, uint32_t* s_scan) {
+template <bool BIG>
+__device__ void phase_top(const RebuildArgs& A, int F, TopSmem& S, uint32_t* s_scan) {
     const ChunkView& cv = A.cv;
-    const int lane = (int)(threadIdx.x & 31u), F = A.chunks;
+    const int lane = (int)(threadIdx.x & 31u);
     const int n = __ldcg(&A.root->n_leaves);
     const uint32_t w0 = blockIdx.x * RW + (threadIdx.x >> 5), nw = gridDim.x * RW;
-    if (F > TOP_STAGED) {  // slot s of every chunk before slot s + 1 of any: the low ones are occupied
+    if (BIG && F > TOP_STAGED) {  // slot s of every chunk before slot s + 1 of any: the low ones are occupied
         const Summaries<false> sum{cv, S};
-        for (uint64_t it = w0; it < (uint64_t)F * MAX_PIECES; it += nw) {
-            const int c = (int)(it % (uint32_t)F), sl = (int)(it / (uint32_t)F);
-            if (sl < sum.nodes(c)) top_node<false>(A, sum, c, sl, n, F, lane);
+        for (uint64_t it = w0; it < (uint64_t)F * MAX_PIECES; it += 32ull * nw) {  // a warp's next 32 slots
+            const uint64_t my = it + (uint64_t)lane * nw;
+            const int c = (int)(my % (uint32_t)F), sl = (int)(my / (uint32_t)F);
+            unsigned used = __ballot_sync(0xffffffffu, sl < MAX_PIECES && sl < sum.nodes(c));
+            for (; used; used &= used - 1u) {
+                const int from = __ffs(used) - 1;
+                top_node<false>(A, sum, __shfl_sync(0xffffffffu, c, from), __shfl_sync(0xffffffffu, sl, from), n, F, lane);
+            }
         }
         return;
     }
@@ -1352,6 +1488,9 @@ __device__ void phase_top(const RebuildArgs& A, TopSmem& S, uint32_t* s_scan) {
 }
 
 // ---- the launch -----------------------------------------------------------------------------------
+// BIG: more triangles than TOP_STAGED chunks hold.  An instance of its own, so that the
+// others' code stays as short as it is (with both in one, 327,680 triangles took 72 -> 78 us).
+template <bool BIG>
 __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
     extern __shared__ __align__(16) unsigned char rb_smem[];
     __shared__ uint32_t s_scan[32];
@@ -1388,7 +1527,7 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
         cen[q] = mk3(0.0f, 0.0f, 0.0f);
         old[q] = coherent && t < nt ? A.codes[t] : 0u;
     }
-    if (A.direct) {
+    if (!BIG && A.direct) {
         phase_boxes<true>(A, s_red, cen);
     } else {
         ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
@@ -1410,7 +1549,7 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
         }
     } else {
         bool sorted = false;
-        if (coherent ? A.buckets > 0 : nt <= SAMPLED_MAX) {
+        if (!BIG && (coherent ? A.buckets > 0 : nt <= SAMPLED_MAX)) {
             BucketSmem& S = *reinterpret_cast<BucketSmem*>(rb_smem);
             const int nb = A.buckets;
             after = cur ^ 1;
@@ -1442,11 +1581,26 @@ __global__ void __launch_bounds__(RB, 2) k_rebuild(const RebuildArgs A) {
         A.root->perm_valid = bad ? 0 : 1;
         A.root->sorted = after;
     }
+    const uint32_t *K = A.keys[after], *V = A.vals[after];
+    int np = nt, F = A.chunks;  // positions the build goes through, and their chunks
+    if constexpr (BIG) {
+        if (ok) phase_unique_count(A, K, s_scan);
+        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+        if (ok) np = phase_unique_write(A, K, V, s_scan);
+        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+        K = A.ucode;
+        V = A.utri;
+        F = (np + A.chunk_len - 1) / A.chunk_len;
+    }
     if (ok)
-        for (int c = blockIdx.x; c < A.chunks; c += gridDim.x)
-            build_chunk(A, c, A.keys[after], A.vals[after], *reinterpret_cast<BuildSmem*>(rb_smem));
+        for (int c = blockIdx.x; c < F; c += gridDim.x)
+            build_chunk<BIG>(A, c, np, K, V, *reinterpret_cast<BuildSmem*>(rb_smem));
     ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
-    if (ok) phase_top(A, *reinterpret_cast<TopSmem*>(rb_smem), s_scan);
+    if (BIG && F > TOP_STAGED) {
+        if (ok) phase_groups(A, F);
+        ok = grid_barrier(A.sync, target, ok, A.err, &s_ok);
+    }
+    if (ok) phase_top<BIG>(A, F, *reinterpret_cast<TopSmem*>(rb_smem), s_scan);
     // the last CTA out leaves both counters at zero for the next launch
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1477,6 +1631,7 @@ __global__ void k_selftest_look_back(const uint32_t* status, int* err) {
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 // CTAs of k_rebuild that fit on the device at once (cooperative launch limit)
+template <bool BIG>
 int resident_ctas() {
     static std::mutex mu;
     static int cached[64] = {};
@@ -1486,7 +1641,7 @@ int resident_ctas() {
     if (!cached[dev]) {
         int sms = 0, per = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rebuild, RB, kSmemBytes) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rebuild<BIG>, RB, kSmemBytes) != cudaSuccess) return 0;
         cached[dev] = sms * per;
     }
     return cached[dev];
@@ -1543,6 +1698,10 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool walked) {
     a.want(&pbox, 64 * (size_t)chunks);
     a.want(&rcnt, 2 * (size_t)chunks);
     a.want(&top, (size_t)MAX_PIECES * chunks);
+    if (chunks > TOP_STAGED) {
+        a.want(&gmin, (size_t)cdiv(chunks, 32));
+        a.want(&gbox, 2 * (size_t)cdiv(chunks, 32));
+    }
     if (!walked) a.want(&root, 1);
     // histograms | sort status (PASSES x tiles x RADIX) | sort counters (the launch
     // clears them) | bucket counts | CTA box unions | chunk leaf counts | change list | barrier counters
@@ -1561,7 +1720,8 @@ void BvhBuffers::plan(Arena& a, int nv_, int nt_, bool normals, bool walked) {
 cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_err, cudaStream_t s, const float* xyz,
                        const float* nrm, float4* margin_state, int64_t m0, int64_t m1) {
     if (b.nt == 0) return cudaSuccess;
-    const int res = resident_ctas();
+    const bool big = b.chunks > TOP_STAGED;
+    const int res = big ? resident_ctas<true>() : resident_ctas<false>();
     if (res <= 0) return cudaErrorLaunchOutOfResources;
     RebuildArgs A;
     A.xyz = xyz ? xyz : b.xyz_in;
@@ -1591,7 +1751,7 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.leaves = b.leaves;
     A.range = b.range;
     A.root = b.root;
-    A.cv = ChunkView{b.cmin, b.cbox, b.srec, b.sbox, b.prec, b.pbox, b.rcnt, b.top};
+    A.cv = ChunkView{b.cmin, b.cbox, b.srec, b.sbox, b.prec, b.pbox, b.rcnt, b.top, b.gmin, b.gbox};
     A.ghist = b.scratch;
     A.sstat = A.ghist + PASSES * RADIX;
     A.scount = A.sstat + (size_t)PASSES * b.tiles_sort * RADIX;
@@ -1609,7 +1769,8 @@ cudaError_t lbvh_build(BvhBuffers& b, float thickness, float box_depth, int* d_e
     A.err = d_err;
     const int grid = std::min(res, b.max_ctas);
     void* args[] = {&A};
-    return cudaLaunchCooperativeKernel((const void*)k_rebuild, dim3(grid), dim3(RB), args, kSmemBytes, s);
+    return cudaLaunchCooperativeKernel(big ? (const void*)k_rebuild<true> : (const void*)k_rebuild<false>, dim3(grid),
+                                       dim3(RB), args, kSmemBytes, s);
 }
 
 cudaError_t launch_selftest_look_back(const uint32_t* zero_status, int* err, cudaStream_t s) {
