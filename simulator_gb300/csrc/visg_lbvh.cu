@@ -45,8 +45,8 @@
 // between them (de-duplication in the build, centroids kept in registers from the boxes to
 // the codes, small bodies without the vertex phase), 32-byte records move as one access,
 // and the sorts spread over all CTAs.  Kernel time, before and now: 19,584 triangles with
-// few changed codes 32 -> 23 us, with most changed (radix passes before) 69 -> 31, without a
-// last order 68 -> 34; 327,680 triangles with few changed 107 -> 75.
+// few changed codes 32 -> 21 us, with most changed (radix passes before) 69 -> 29, without a
+// last order 68 -> 32; 327,680 triangles with few changed 107 -> 71.
 // Nodes are numbered by their split position; the tree is the same binary radix
 // tree processInternalNode (cudaBRT.cu:120-161) builds, and visg_export_lbvh
 // renumbers it into the reference's layout.  Data one CTA reads after another wrote

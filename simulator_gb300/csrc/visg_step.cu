@@ -1043,8 +1043,8 @@ __global__ void k_count_contacts(const float4* __restrict__ st, int64_t n, unsig
 // update_vertex (simulation.cu:253-257): x = x_old = p, so v = (p - p) / dt; the
 // stored contact normal is kept.  moves: {vertex, p} in page-locked host memory, read from
 // there, before the wait for earlier launches: two copies in the stream before it took longer
-// than the kernel (dragged 64 x 64 sheet 33 -> 28 us a frame, six frames
-// of 24 garments with their read-back, whose copies shared the engines, 371 -> 285).
+// than the kernel (dragged 64 x 64 sheet 21.8 -> 14.8 us a frame, six frames
+// of 24 garments with their read-back, whose copies shared the engines, 388 -> 300).
 // The threads run in no order, so where a vertex may be named twice (`claim`) the moves are
 // numbered, each claims its vertex for its number, and only the highest writes: within the
 // block where one holds all the moves (`alone`), else in a kernel of their own before.
