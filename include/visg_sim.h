@@ -67,8 +67,8 @@ typedef struct VisgParams {
                                 visg_autotune / visg_batch_autotune may change it.  A single
                                 garment of at most 512 vertices per SM is always stepped fused
                                 (collision_margin on), whatever its launch shape; in tiles of
-                                128 or 256, one per CTA and not staged, helper warps of the
-                                same kernel answer its queries beside the spring sums.        */
+                                128 or 256, one per CTA, with stage_neighbours 0, helper warps
+                                of the same kernel answer its queries beside the spring sums.  */
     int32_t stage_neighbours; /* 1: each slice's spring entries are staged in shared
                                 memory by TMA bulk copies, 0: read through the L1 (default);
                                 same results.  visg_autotune / visg_batch_autotune may change it. */
